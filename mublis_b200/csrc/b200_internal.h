@@ -204,6 +204,7 @@ int b200_copy_d2h(void *dst, long rs, long cs, const void *src, long ld, long ro
  * none is armed), cleared by the call: the next FP64 tensor-pipe GEMM launch
  * takes it and stalls. */
 unsigned long long b200_take_test_stall(void);
+int b200_test_stall_armed(void);
 
 /* noalloc.cu: resolves the allocation-free SGEMM's fixed scratch array on
  * the current device (run once by b200_init). */
@@ -214,6 +215,10 @@ void b200_noalloc_setup(void);
 int b200_take_device_error(void);
 
 /* l3.cu */
+/* Whether an m x n view and a rows x cols view (elements of elt bytes) may
+ * share memory (exact for blocks of one matrix). */
+int b200_views_overlap(const void *c, long rs_c, long cs_c, long m, long n, const void *x, long rs_x,
+                       long cs_x, long rows, long cols, long elt);
 int b200_l3_run(const b200_l3_desc_t *d);
 int b200_trsm_run(const b200_trsm_desc_t *d);
 int b200_scale_strided(int dtype, int m, int n, double beta, void *c, long rs, long cs,

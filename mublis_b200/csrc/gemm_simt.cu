@@ -596,3 +596,17 @@ int launch_scale(int m, int n, T beta, T *c, long rs, long cs, int ji, cudaStrea
 
 template int launch_scale<float>(int, int, float, float *, long, long, int, cudaStream_t);
 template int launch_scale<double>(int, int, double, double *, long, long, int, cudaStream_t);
+
+// Loads the kernels of the allocation-free SGEMM on the current device (the
+// driver loads a kernel's code, and takes memory for it, at its first use).
+int b200_simt_preload() {
+  using C = SimtConfig<float>;
+  cudaFuncAttributes fa;
+  SimtGemmArgs<float> none;
+  none.m = none.n = 0;
+  B200_TRY(launch_simt_gemm<float>(none, nullptr));  // no tiles: sets the kernel up only
+  B200_CUDA_TRY(cudaFuncGetAttributes(
+      &fa, simt_tile_kernel<float, C::BM, C::BN, C::BK, 4, 2, 2, 2, true>));
+  B200_CUDA_TRY(cudaFuncGetAttributes(&fa, scale_kernel<float>));
+  return B200_OK;
+}

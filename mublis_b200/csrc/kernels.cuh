@@ -263,5 +263,20 @@ void b200_tile_list(long m, long n, long k, int BM, int BN, int BK, b200_tile_do
 int b200_split_for(long m_full, long n_full, long k, int BM, int BN, int BK,
                    b200_tile_domain_t dom, long slots, double split_cost);
 
+// ---- small products in one launch (gemm_direct.cu)
+
+// How a product runs there: tile 64 or 32 (0: not there), and how many CTAs
+// share a tile's k range.
+struct b200_direct_choice_t {
+  int tile, splits;
+};
+b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d);
+// On the calling thread's stream; C must overlap no operand.
+int launch_direct_gemm(const b200_l3_desc_t *d, const b200_direct_choice_t &ch);
+
 template <typename T>
 int launch_scale(int m, int n, T beta, T *c, long rs, long cs, int ji, cudaStream_t s);
+
+// Load the kernels that the allocation-free SGEMM runs (noalloc.cu).
+int b200_simt_preload();
+int b200_pack_preload();

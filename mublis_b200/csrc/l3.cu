@@ -18,6 +18,35 @@
 #include "tc_common.cuh"
 #include "tc_gemm.cuh"
 
+// Whether an m x n view C and a rows x cols view X (elements of `elt` bytes)
+// may share memory.  Exact for two blocks of one matrix (the same leading
+// dimension and unit stride, as the blocks of a recursive solve have: their
+// byte intervals interleave although no element is shared); otherwise by
+// byte interval, and true for a negative stride.
+extern "C" int b200_views_overlap(const void *c, long rs_c, long cs_c, long m, long n, const void *x,
+                                  long rs_x, long cs_x, long rows, long cols, long elt) {
+  if (rs_c < 0 || cs_c < 0 || rs_x < 0 || cs_x < 0) return 1;
+  const intptr_t c0 = (intptr_t)c, x0 = (intptr_t)x;
+  const intptr_t c1 = c0 + elt * ((m - 1) * rs_c + (n - 1) * cs_c + 1);
+  const intptr_t x1 = x0 + elt * ((rows - 1) * rs_x + (cols - 1) * cs_x + 1);
+  if (c1 <= x0 || x1 <= c0) return 0;
+  // In one grid of lines of `ld` elements: C is cw x ch (along the unit
+  // stride x lines), X is xw x xh.
+  const bool c_row = rs_c == 1, x_row = rs_x == 1;
+  const long ld = c_row ? cs_c : rs_c, cw = c_row ? m : n, ch = c_row ? n : m;
+  const long xld = x_row ? cs_x : rs_x, xw = x_row ? rows : cols, xh = x_row ? cols : rows;
+  if ((!c_row && cs_c != 1) || (!x_row && cs_x != 1) || ld != xld || cw > ld || xw > ld ||
+      (x0 - c0) % elt != 0)
+    return 1;
+  const long off = (x0 - c0) / elt;
+  long line = off / ld, at = off % ld;
+  if (at < 0) at += ld, --line;  // X starts at (at, line) relative to C, 0 <= at < ld
+  const bool lines = line < ch && line + xh > 0;
+  if (lines && at < cw) return 1;
+  // The part of X that runs past the line's end is on the next line.
+  return at + xw > ld && line + 1 < ch && line + 1 + xh > 0;
+}
+
 namespace {
 
 // "auto" picks, per call, the fastest form whose error is no worse than the
@@ -82,6 +111,15 @@ bool use_dmma() {
   return on;
 }
 
+// MUBLIS_B200_DIRECT=0 keeps the pack pass for every call.
+bool direct_on() {
+  static const bool on = [] {
+    const char *e = getenv("MUBLIS_B200_DIRECT");
+    return !(e && !strcmp(e, "0"));
+  }();
+  return on;
+}
+
 // A strided FP64 view (rows x cols, element (i, j) at x + i rs + j cs) as a
 // TMA source: one stride must be 1 and the other a positive multiple of 2
 // elements (16 bytes) at least the unit-stride extent, the base 16-byte
@@ -99,11 +137,16 @@ bool tma_view_ok(const void *x, long rs, long cs, long rows, long cols, bool *ro
   return false;
 }
 
-// Byte interval [lo, hi] spanned by a view with non-negative strides.
-void view_span(const void *x, long rs, long cs, long rows, long cols, uintptr_t *lo,
-               uintptr_t *hi) {
-  *lo = (uintptr_t)x;
-  *hi = (uintptr_t)x + sizeof(double) * ((rows - 1) * rs + (cols - 1) * cs + 1) - 1;
+// Whether C shares memory with an operand of the product.
+bool overlaps_operand(const b200_l3_desc_t *d) {
+  const long elt = d->dtype == B200_F64 ? 8 : 4;
+  for (int t = 0; t < d->npairs; ++t)
+    if (b200_views_overlap(d->c, d->rs_c, d->cs_c, d->m, d->n, d->a[t], d->rs_a[t], d->cs_a[t], d->m,
+                      d->k, elt) ||
+        b200_views_overlap(d->c, d->rs_c, d->cs_c, d->m, d->n, d->b[t], d->rs_b[t], d->cs_b[t], d->k,
+                      d->n, elt))
+      return true;
+  return false;
 }
 
 // The FP64 tensor-pipe kernel can read op(A) and op(B) straight from the
@@ -112,20 +155,13 @@ void view_span(const void *x, long rs, long cs, long rows, long cols, uintptr_t 
 // with the same orientation, a SYR2K's pairs meeting on a k-block boundary,
 // and C overlapping no operand (an in-place product must read its operand
 // before it is overwritten, which only a copy guarantees).
-// MUBLIS_B200_DIRECT=0 keeps the pack pass for every call.
 bool dmma_direct(const b200_l3_desc_t *d, DmmaGemmArgs *g) {
-  static const bool on = [] {
-    const char *e = getenv("MUBLIS_B200_DIRECT");
-    return !(e && !strcmp(e, "0"));
-  }();
   const mublis_l3_product_t &pr = d->product;
-  if (!on || pr.a.struc != MUBLIS_STRUC_GENERAL || pr.b.struc != MUBLIS_STRUC_GENERAL ||
+  if (!direct_on() || pr.a.struc != MUBLIS_STRUC_GENERAL || pr.b.struc != MUBLIS_STRUC_GENERAL ||
       pr.domain.jp != MUBLIS_L3_ALL || pr.domain.pi != MUBLIS_L3_ALL)
     return false;
   if (d->npairs == 2 && d->k % B200_DMMA_BK != 0) return false;
-  if (d->rs_c < 0 || d->cs_c < 0) return false;
-  uintptr_t clo, chi;
-  view_span(d->c, d->rs_c, d->cs_c, d->m, d->n, &clo, &chi);
+  if (overlaps_operand(d)) return false;
   bool a_mc = false, b_kc = false;
   for (int t = 0; t < d->npairs; ++t) {
     bool ac, bc;
@@ -138,11 +174,6 @@ bool dmma_direct(const b200_l3_desc_t *d, DmmaGemmArgs *g) {
     } else if (ac != a_mc || bc != b_kc) {
       return false;
     }
-    uintptr_t lo, hi;
-    view_span(d->a[t], d->rs_a[t], d->cs_a[t], d->m, d->k, &lo, &hi);
-    if (lo <= chi && clo <= hi) return false;
-    view_span(d->b[t], d->rs_b[t], d->cs_b[t], d->k, d->n, &lo, &hi);
-    if (lo <= chi && clo <= hi) return false;
   }
   // Tensor maps: op(A) tile 128 (m) x 16 (k), op(B) tile 16 (k) x 128 (n);
   // k innermost tiles are 16 doubles = 128 bytes, 128-byte swizzled.
@@ -330,6 +361,50 @@ int run_plain(const b200_l3_desc_t *d) {
   return st;
 }
 
+// A small product in one launch (gemm_direct.cu), or 0 when the call is not
+// one.  An in-place product (TRMM, a solve's diagonal products: C is the
+// operand itself) reads a compact copy of that operand.
+int try_direct(const b200_l3_desc_t *d, int *status) {
+  // A stall armed by mublis_b200_test_stall_next waits for the FP64
+  // tensor-pipe kernel of the packed path.
+  if (!direct_on() || (d->dtype == B200_F64 && (!use_dmma() || b200_test_stall_armed()))) return 0;
+  const mublis_l3_product_t &pr = d->product;
+  if (d->npairs == 2 &&
+      (pr.a.struc != MUBLIS_STRUC_GENERAL || pr.b.struc != MUBLIS_STRUC_GENERAL ||
+       pr.domain.jp != MUBLIS_L3_ALL || pr.domain.pi != MUBLIS_L3_ALL))
+    return 0;
+  const b200_direct_choice_t ch = b200_direct_choice(d);
+  if (!ch.tile) return 0;
+  if (!overlaps_operand(d)) {
+    *status = launch_direct_gemm(d, ch);
+    return 1;
+  }
+  const bool is_b = d->b[0] == d->c && d->rs_b[0] == d->rs_c && d->cs_b[0] == d->cs_c && d->k == d->m;
+  const bool is_a = d->a[0] == d->c && d->rs_a[0] == d->rs_c && d->cs_a[0] == d->cs_c && d->k == d->n;
+  const bool rows = d->rs_c == 1 && d->cs_c >= d->m, cols = d->cs_c == 1 && d->rs_c >= d->n;
+  if (d->npairs != 1 || is_a == is_b || (!rows && !cols)) return 0;
+  const size_t elt = d->dtype == B200_F64 ? 8 : 4;
+  const long w = rows ? d->m : d->n, h = rows ? d->n : d->m;
+  const long ld = b200_round_up(w, (long)(16 / elt));
+  b200_l3_desc_t e = *d;
+  (is_b ? e.rs_b : e.rs_a)[0] = rows ? 1 : ld;
+  (is_b ? e.cs_b : e.cs_a)[0] = rows ? ld : 1;
+  if (b200_views_overlap(e.c, e.rs_c, e.cs_c, e.m, e.n, is_b ? e.a[0] : e.b[0], is_b ? e.rs_a[0] : e.rs_b[0],
+                    is_b ? e.cs_a[0] : e.cs_b[0], is_b ? e.m : e.k, is_b ? e.k : e.n, (long)elt))
+    return 0;
+  void *copy = nullptr;
+  *status = b200_alloc(&copy, elt * ld * h);
+  if (*status != B200_OK) return 1;
+  (is_b ? e.b : e.a)[0] = copy;
+  if (cudaMemcpy2DAsync(copy, ld * elt, d->c, (rows ? d->cs_c : d->rs_c) * elt, w * elt, h,
+                        cudaMemcpyDeviceToDevice, b200_cur_stream()) != cudaSuccess)
+    *status = b200_set_error(B200_ECUDA, "direct gemm: operand copy failed");
+  else
+    *status = launch_direct_gemm(&e, ch);
+  b200_free(copy);
+  return 1;
+}
+
 }  // namespace
 
 extern "C" int b200_scale_strided(int dtype, int m, int n, double beta, void *c, long rs, long cs,
@@ -365,6 +440,8 @@ extern "C" int b200_l3_run(const b200_l3_desc_t *d) {
       B200_TRY(b200_ozaki2_choice(&e, target, &e.slices, nullptr, 0));
     return tc_run_ozaki(&e);
   }
+  int st;
+  if (try_direct(d, &st)) return st;
   if (d->dtype == B200_F32) return run_plain<float>(d);
   return run_plain<double>(d);
 }

@@ -552,3 +552,13 @@ template int launch_absmax<float>(const PackView &, bool, long, long, unsigned l
                                   cudaStream_t);
 template int launch_absmax<double>(const PackView &, bool, long, long, unsigned long long *,
                                    cudaStream_t);
+
+// Loads the plain FP32 pack kernels on the current device (the driver loads a
+// kernel's code, and takes memory for it, at its first use).
+int b200_pack_preload() {
+  cudaFuncAttributes fa;
+  B200_CUDA_TRY(cudaFuncGetAttributes(&fa, pack_dense_kernel<float, true>));
+  B200_CUDA_TRY(cudaFuncGetAttributes(&fa, pack_dense_kernel<float, false>));
+  B200_CUDA_TRY(cudaFuncGetAttributes(&fa, pack_kernel<float>));
+  return B200_OK;
+}

@@ -217,6 +217,7 @@ int mublis_b200_test_stall_next(unsigned long long wait_limit_ns) {
 }
 
 unsigned long long b200_take_test_stall(void) { return g_test_stall.exchange(0); }
+int b200_test_stall_armed(void) { return g_test_stall.load() != 0; }
 
 int b200_set_error(int code, const char *where) {
   snprintf(t_error, sizeof t_error, "%s", where);
