@@ -1,4 +1,4 @@
-// gemm_simt.cu -- plain FP32 / FP64 GEMM on the FMA pipes: the device
+// gemm_simt.cu -- plain FP64 GEMM on the FMA pipe (MUBLIS_B200_DGEMM=simt): the device
 // form of the reference's five-loop driver (frame/l3/l3_driver.c:126-239)
 // plus its micro-kernel (include/mublis_instantiate.h:37-52).
 //
@@ -45,11 +45,7 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// One 16-byte shared-memory fragment: 4 floats or 2 doubles.
-__device__ __forceinline__ void lds16(float (&d)[4], const float *p) {
-  float4 v = *reinterpret_cast<const float4 *>(p);
-  d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-}
+// One 16-byte shared-memory fragment.
 __device__ __forceinline__ void lds16(double (&d)[2], const double *p) {
   double2 v = *reinterpret_cast<const double2 *>(p);
   d[0] = v.x; d[1] = v.y;
@@ -60,8 +56,7 @@ __device__ __forceinline__ void lds16(double (&d)[2], const double *p) {
 // every call that is not split along k: a persistent schedule of the same
 // tiles measured no faster (SGEMM 4096^3: 55.8 vs 55.6 TF/s), the tiles'
 // own efficiency, not the last wave, being the limit there.
-template <typename T, int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, int MINB,
-          bool PAIR = false>
+template <typename T, int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, int MINB>
 __global__ void __launch_bounds__(256, MINB) simt_tile_kernel(SimtGemmArgs<T> p) {
   constexpr int NT = 256;
   constexpr int WTM = BM / WARPS_M, WTN = BN / WARPS_N;
@@ -107,21 +102,11 @@ __global__ void __launch_bounds__(256, MINB) simt_tile_kernel(SimtGemmArgs<T> p)
   const int wm = warp % WARPS_M, wn = warp / WARPS_M;
   const int ty = lane >> 3, tx = lane & 7;
 
-  // PAIR (FP32 only): accumulators as column pairs updated with the packed
-  // sm_100 FMA (__ffma2_rn: two correctly rounded fmaf per instruction), so
-  // the FMA stream takes half the issue slots and the loads and address
-  // arithmetic fit beside it.  Each element's result is that of fmaf.
-  static_assert(!PAIR || (sizeof(T) == 4 && TN % 2 == 0), "pairs are FP32 column pairs");
-  constexpr int TNP = PAIR ? TN / 2 : TN;
-  using Acc = typename std::conditional<PAIR, float2, T>::type;
-  Acc acc[TM][TNP];
+  T acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TNP; ++j) {
-      if constexpr (PAIR) acc[i][j] = make_float2(0.f, 0.f);
-      else acc[i][j] = T(0);
-    }
+    for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
 
   auto load_stage = [&](int stage, int kt) {
     const T *ga = p.ap + (long)kt * BK * p.lda + m0;
@@ -176,13 +161,7 @@ __global__ void __launch_bounds__(256, MINB) simt_tile_kernel(SimtGemmArgs<T> p)
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TNP; ++j) {
-          if constexpr (PAIR)
-            acc[i][j] = __ffma2_rn(make_float2(af[i], af[i]), make_float2(bf[2 * j], bf[2 * j + 1]),
-                                   acc[i][j]);
-          else
-            acc[i][j] = fma(af[i], bf[j], acc[i][j]);
-        }
+        for (int j = 0; j < TN; ++j) acc[i][j] = fma(af[i], bf[j], acc[i][j]);
     }
   }
   cp_async_wait<0>();
@@ -205,9 +184,7 @@ __global__ void __launch_bounds__(256, MINB) simt_tile_kernel(SimtGemmArgs<T> p)
     for (int j = 0; j < TN; ++j) {
       const long gj = n0 + wn * WTN + (j / CW) * NSP + tx * CW + (j % CW);
       if (gj >= p.n || !b200_rel(p.ji, gj, gi)) continue;
-      T v;
-      if constexpr (PAIR) v = alpha * ((j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x);
-      else v = alpha * acc[i][j];
+      T v = alpha * acc[i][j];
       if (beta != T(0)) v = fma(beta, cv[j], v);
       p.c[gi * p.rs_c + gj * p.cs_c] = v;
     }
@@ -218,7 +195,7 @@ __global__ void __launch_bounds__(256, MINB) simt_tile_kernel(SimtGemmArgs<T> p)
 // Persistent CTAs over (tile, k-chunk) units for split-K calls (SPLIT:
 // the split epilogue compiled in).
 template <typename T, int BM, int BN, int BK, int WARPS_M, int WARPS_N, int STAGES, int MINB,
-          bool PAIR = false, bool SPLIT = false>
+          bool SPLIT = false>
 __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p) {
   constexpr int NT = 256;
   constexpr int WTM = BM / WARPS_M, WTN = BN / WARPS_N;
@@ -246,13 +223,6 @@ __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p)
   const int wm = warp % WARPS_M, wn = warp / WARPS_M;
   const int ty = lane >> 3, tx = lane & 7;
 
-  // PAIR (FP32 only): accumulators as column pairs updated with the packed
-  // sm_100 FMA (__ffma2_rn: two correctly rounded fmaf per instruction), so
-  // the FMA stream takes half the issue slots and the loads and address
-  // arithmetic fit beside it.  Each element's result is that of fmaf.
-  static_assert(!PAIR || (sizeof(T) == 4 && TN % 2 == 0), "pairs are FP32 column pairs");
-  constexpr int TNP = PAIR ? TN / 2 : TN;
-  using Acc = typename std::conditional<PAIR, float2, T>::type;
 
   // Persistent CTAs take units from p.work; without it, the CTA computes
   // unit blockIdx.x alone.  Unit u is k-chunk u % S of tile u / S.
@@ -301,14 +271,11 @@ __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p)
       const int kt_begin = min(tile_kt1, tile_kt0 + chunk * per);
       const int kt_end = min(tile_kt1, kt_begin + per);
 
-      Acc acc[TM][TNP];
+      T acc[TM][TN];
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TNP; ++j) {
-          if constexpr (PAIR) acc[i][j] = make_float2(0.f, 0.f);
-          else acc[i][j] = T(0);
-        }
+        for (int j = 0; j < TN; ++j) acc[i][j] = T(0);
 
       auto load_stage = [&](int stage, int kt) {
         const T *ga = p.ap + (long)kt * BK * p.lda + m0;
@@ -363,13 +330,7 @@ __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p)
 #pragma unroll
           for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TNP; ++j) {
-              if constexpr (PAIR)
-                acc[i][j] = __ffma2_rn(make_float2(af[i], af[i]),
-                                       make_float2(bf[2 * j], bf[2 * j + 1]), acc[i][j]);
-              else
-                acc[i][j] = fma(af[i], bf[j], acc[i][j]);
-            }
+            for (int j = 0; j < TN; ++j) acc[i][j] = fma(af[i], bf[j], acc[i][j]);
         }
       }
       cp_async_wait<0>();
@@ -386,10 +347,7 @@ __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p)
         for (int i = 0; i < TM; ++i)
 #pragma unroll
           for (int j = 0; j < TN; ++j) {
-            T v;
-            if constexpr (PAIR) v = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
-            else v = acc[i][j];
-            mine[(i * TN + j) * NT + tid] = v;
+            mine[(i * TN + j) * NT + tid] = acc[i][j];
           }
         __threadfence();
         __syncthreads();
@@ -405,12 +363,7 @@ __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p)
             for (int j = 0; j < TN; ++j) {
               T v = __ldcg(first + (i * TN + j) * NT + tid);
               for (int c = 1; c < S; ++c) v += __ldcg(first + ((size_t)c * E + i * TN + j) * NT + tid);
-              if constexpr (PAIR) {
-                if (j & 1) acc[i][j >> 1].y = v;
-                else acc[i][j >> 1].x = v;
-              } else {
-                acc[i][j] = v;
-              }
+              acc[i][j] = v;
             }
           if (tid == 0) p.arrivals[tslot] = 0;
         }
@@ -435,9 +388,7 @@ __global__ void __launch_bounds__(256, MINB) simt_gemm_kernel(SimtGemmArgs<T> p)
           for (int j = 0; j < TN; ++j) {
             const long gj = n0 + wn * WTN + (j / CW) * NSP + tx * CW + (j % CW);
             if (gj >= p.n || !b200_rel(p.ji, gj, gi)) continue;
-            T v;
-            if constexpr (PAIR) v = alpha * ((j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x);
-            else v = alpha * acc[i][j];
+            T v = alpha * acc[i][j];
             if (beta != T(0)) v = fma(beta, cv[j], v);
             p.c[gi * p.rs_c + gj * p.cs_c] = v;
           }
@@ -478,12 +429,12 @@ int resident_per_sm(K kern, size_t smem) {
   return nb;
 }
 
-template <typename T, int BM, int BN, int WM, int WN, int ST, int MINB, bool PAIR = false>
+template <typename T, int BM, int BN, int WM, int WN, int ST, int MINB>
 int launch_cfg(const SimtGemmArgs<T> &a0, cudaStream_t s, const SimtPolicy *pol) {
   constexpr int BK = SimtConfig<T>::BK;
   constexpr int E = (BM / WM / 4) * (BN / WN / 8);  // accumulators per thread
-  auto kern = simt_tile_kernel<T, BM, BN, BK, WM, WN, ST, MINB, PAIR>;
-  auto kern_split = simt_gemm_kernel<T, BM, BN, BK, WM, WN, ST, MINB, PAIR, true>;
+  auto kern = simt_tile_kernel<T, BM, BN, BK, WM, WN, ST, MINB>;
+  auto kern_split = simt_gemm_kernel<T, BM, BN, BK, WM, WN, ST, MINB, true>;
   const size_t smem = (size_t)ST * BK * (BM + BN) * sizeof(T);
   static std::once_flag once;
   static int conf = B200_OK, per_sm = 0;
@@ -504,7 +455,7 @@ int launch_cfg(const SimtGemmArgs<T> &a0, cudaStream_t s, const SimtPolicy *pol)
   const int S = pol ? b200_split_for(pol->m_full, pol->n_full, a0.k, BM, BN, BK, dom, slots, 4.0)
                     : 1;
   if (S == 1) {  // nothing allocated
-    B200ProfScope prof(sizeof(T) == 4 ? "simt_sgemm" : "simt_dgemm", s);
+    B200ProfScope prof("simt_dgemm", s);
     kern<<<(unsigned)tiles, 256, smem, s>>>(a0);
     B200_LAUNCH_CHECK();
     return B200_OK;
@@ -541,7 +492,7 @@ int launch_cfg(const SimtGemmArgs<T> &a0, cudaStream_t s, const SimtPolicy *pol)
     a.ntiles = (int)ntiles;
     a.splits = S;
     a.partials = S > 1 ? (T *)(scratch + off_part) : nullptr;
-    B200ProfScope prof(sizeof(T) == 4 ? "simt_sgemm" : "simt_dgemm", s);
+    B200ProfScope prof("simt_dgemm", s);
     kern_split<<<(unsigned)std::min(units, slots), 256, smem, s>>>(a);
     if (cudaGetLastError() != cudaSuccess) st = b200_set_error(B200_ECUDA, "gemm: launch failed");
   }
@@ -559,18 +510,6 @@ int simt_variant(bool dbl) {
 }
 
 }  // namespace
-
-template <>
-int launch_simt_gemm<float>(const SimtGemmArgs<float> &a, cudaStream_t s, const SimtPolicy *pol) {
-  switch (simt_variant(false)) {
-  case 1: return launch_cfg<float, 128, 128, 2, 4, 4, 2>(a, s, pol);
-  case 2: return launch_cfg<float, 128, 128, 4, 2, 3, 1>(a, s, pol);
-  case 3: return launch_cfg<float, 128, 128, 4, 2, 4, 2>(a, s, pol);  // scalar fmaf, 4 stages
-  case 4: return launch_cfg<float, 128, 128, 4, 2, 4, 2, true>(a, s, pol);  // packed, 4 stages
-  // Packed FMA, 2-stage cp.async ring: 52.4 (scalar, 4 stages) -> 58.1 TF/s at 8192^3.
-  default: return launch_cfg<float, 128, 128, 4, 2, 2, 2, true>(a, s, pol);
-  }
-}
 
 template <>
 int launch_simt_gemm<double>(const SimtGemmArgs<double> &a, cudaStream_t s, const SimtPolicy *pol) {
@@ -597,16 +536,10 @@ int launch_scale(int m, int n, T beta, T *c, long rs, long cs, int ji, cudaStrea
 template int launch_scale<float>(int, int, float, float *, long, long, int, cudaStream_t);
 template int launch_scale<double>(int, int, double, double *, long, long, int, cudaStream_t);
 
-// Loads the kernels of the allocation-free SGEMM on the current device (the
-// driver loads a kernel's code, and takes memory for it, at its first use).
-int b200_simt_preload() {
-  using C = SimtConfig<float>;
+// Loads the FP32 kernel on the current device (the driver loads a kernel's
+// code, and takes memory for it, at its first use).
+int b200_scale_preload() {
   cudaFuncAttributes fa;
-  SimtGemmArgs<float> none;
-  none.m = none.n = 0;
-  B200_TRY(launch_simt_gemm<float>(none, nullptr));  // no tiles: sets the kernel up only
-  B200_CUDA_TRY(cudaFuncGetAttributes(
-      &fa, simt_tile_kernel<float, C::BM, C::BN, C::BK, 4, 2, 2, 2, true>));
   B200_CUDA_TRY(cudaFuncGetAttributes(&fa, scale_kernel<float>));
   return B200_OK;
 }

@@ -155,7 +155,11 @@ template <typename T>
 int launch_pack(const PackView &v, bool b_side, long mn_len, long k_len, long mn_pad,
                 long kk0, long kk1, const PackOut &o, cudaStream_t s);
 
-// Plain FP32 / FP64 GEMM on the FMA pipes over packed MN-major panels.
+// Output tiles that a launch's parameters can list (restricted domains);
+// longer lists are uploaded.
+constexpr int B200_MAX_LISTED_TILES = 1024;
+
+// Plain FP64 GEMM on the FMA pipe over packed MN-major panels.
 template <typename T>
 struct SimtGemmArgs {
   const T *ap;  // [Kpad][Mpad]
@@ -185,6 +189,34 @@ struct SimtGemmArgs {
 struct SimtPolicy {
   long m_full, n_full;
 };
+
+// Plain FP32 GEMM on the FMA pipe (gemm_ffma.cu).  Each operand is one or two
+// (SYR2K read in place) 2-D TMA sources with m (n) innermost.
+constexpr int B200_FFMA_TILE = 128, B200_FFMA_BK = 16;
+struct FfmaGemmArgs {
+  CUtensorMap ta[2], tb[2];
+  int a_kpair = 0x7fffffff, b_kpair = 0x7fffffff;  // k at which the second source begins
+  float *c = nullptr;
+  long rs_c = 1, cs_c = 1;
+  int m = 0, n = 0, k = 0;
+  float alpha = 0.f, beta = 0.f;
+  int jp = MUBLIS_L3_ALL, ji = MUBLIS_L3_ALL, pi = MUBLIS_L3_ALL;
+  // Filled by the launcher.
+  int *err = nullptr;
+  int tiles_m = 0, tiles_n = 0, ntiles = 0, splits = 1, listed = 0;
+  int fold = 0x7fffffff;  // k-blocks added in a row
+  const int2 *tile_list = nullptr;
+  int *arrivals = nullptr;    // per (tile, warp): k-chunks finished, splits > 1
+  float *partials = nullptr;  // per unit: its k-chunk's sums, splits > 1
+  uint16_t tiles[B200_MAX_LISTED_TILES];  // tm << 8 | tn
+};
+// The whole call's output size (a column panel carries the call's).
+struct FfmaPolicy {
+  long m_full, n_full;
+};
+// pol == nullptr: no split-K, no domain, nothing allocated.
+int launch_ffma_gemm(FfmaGemmArgs &a, const FfmaPolicy *pol, cudaStream_t s);
+int b200_ffma_preload();
 
 // Plain FP64 GEMM on the FP64 tensor pipe over PACK_FRAG64 panels.
 struct DmmaGemmArgs {
@@ -226,10 +258,6 @@ template <typename T>
 struct SimtConfig;
 
 template <>
-struct SimtConfig<float> {
-  static constexpr int BM = 128, BN = 128, BK = 16;  // panel padding (tiles may be smaller)
-};
-template <>
 struct SimtConfig<double> {
   static constexpr int BM = 128, BN = 128, BK = 16;  // panel padding (tiles may be smaller)
 };
@@ -252,6 +280,13 @@ struct b200_tile_domain_t {
 // clipping its k range to jp / pi (l3_driver.c:130,148-150,163,171).
 void b200_tile_list(long m, long n, long k, int BM, int BN, int BK, b200_tile_domain_t dom,
                     std::vector<int2> *list, std::vector<int> *costs);
+
+// Reverses every other round of `grid` entries of a heaviest-first list that
+// `grid` persistent CTAs take round-robin, so that CTA 0 does not get the
+// heaviest of every round.
+void b200_snake(std::vector<int2> &list, int grid);
+// Writes the list as tm << 8 | tn, if it fits `tiles`.
+bool b200_list_tiles(const std::vector<int2> &list, uint16_t (&tiles)[B200_MAX_LISTED_TILES]);
 
 // Split-K factor for a whole call (m_full x n_full x k) on `slots` resident
 // persistent CTAs that take units (tile, k-chunk) heaviest tile first: the
@@ -277,6 +312,6 @@ int launch_direct_gemm(const b200_l3_desc_t *d, const b200_direct_choice_t &ch);
 template <typename T>
 int launch_scale(int m, int n, T beta, T *c, long rs, long cs, int ji, cudaStream_t s);
 
-// Load the kernels that the allocation-free SGEMM runs (noalloc.cu).
-int b200_simt_preload();
+// Load the kernels that the allocation-free SGEMM runs besides its GEMM.
 int b200_pack_preload();
+int b200_scale_preload();

@@ -319,42 +319,103 @@ int run_dmma(const b200_l3_desc_t *d) {
   return st;
 }
 
-template <typename T>
-int run_plain(const b200_l3_desc_t *d) {
-  if (sizeof(T) == 8 && use_dmma()) return run_dmma(d);
-  using C = SimtConfig<T>;
+// One operand of the FP32 kernel: read in place when it is general and
+// unmasked, its unit stride runs along m (n), its lines start on 16 bytes and
+// it shares no memory with C (SYR2K: and its first pair ends on a k-block);
+// else packed into *panel (both pairs as one).
+int ffma_operand(const b200_l3_desc_t *d, bool b_side, long len, CUtensorMap (&map)[2], int *kpair,
+                 void **panel, cudaStream_t s) {
+  const mublis_l3_product_t &pr = d->product;
+  const mublis_l3_operand_t &o = b_side ? pr.b : pr.a;
+  const int mask = b_side ? (int)pr.domain.jp : (int)pr.domain.pi;
+  const void *const *x = b_side ? d->b : d->a;
+  const long *rs = b_side ? d->rs_b : d->rs_a, *cs = b_side ? d->cs_b : d->cs_a;
+  const int T = B200_FFMA_TILE, BK = B200_FFMA_BK;
+  bool direct = direct_on() && o.struc == MUBLIS_STRUC_GENERAL && mask == MUBLIS_L3_ALL &&
+                (d->npairs == 1 || d->k % BK == 0);
+  for (int t = 0; t < d->npairs && direct; ++t) {
+    const long s_mn = b_side ? cs[t] : rs[t], s_k = b_side ? rs[t] : cs[t];
+    direct = s_mn == 1 && s_k >= len && s_k % 4 == 0 && ((uintptr_t)x[t] & 15) == 0 &&
+             !b200_views_overlap(d->c, d->rs_c, d->cs_c, d->m, d->n, x[t], rs[t], cs[t],
+                                 b_side ? d->k : d->m, b_side ? d->n : d->k, 4) &&
+             b200_make_tmap_f32(&map[t], x[t], len, d->k, s_k, T, BK) == B200_OK;
+  }
+  if (direct) {
+    if (d->npairs == 2) *kpair = d->k;
+    return B200_OK;
+  }
+  const long pad = b200_round_up(len, T), kpad = b200_round_up((long)d->k * d->npairs, BK);
+  B200_TRY(b200_alloc(panel, sizeof(float) * pad * kpad));
+  const PackOut out{*panel, pad, 0, PACK_MN_MAJOR, PACK_COPY, 1, nullptr};
+  for (int t = 0; t < d->npairs; ++t) {
+    const long kk0 = (long)t * d->k, kk1 = t + 1 == d->npairs ? kpad : kk0 + d->k;
+    const PackView v{x[t], rs[t], cs[t], (int)o.struc, (int)o.uplo, (int)o.diag, mask};
+    B200_TRY(launch_pack<float>(v, b_side, len, d->k, pad, kk0, kk1, out, s));
+  }
+  return b200_make_tmap_f32(&map[0], *panel, pad, kpad, pad, T, BK);
+}
+
+int run_sgemm(const b200_l3_desc_t *d) {
+  cudaStream_t s = b200_cur_stream();
+  FfmaGemmArgs g;
+  void *ap = nullptr, *bp = nullptr;
+  int st = ffma_operand(d, false, d->m, g.ta, &g.a_kpair, &ap, s);
+  if (st == B200_OK) st = ffma_operand(d, true, d->n, g.tb, &g.b_kpair, &bp, s);
+  if (st == B200_OK) {
+    g.c = (float *)d->c;
+    g.rs_c = d->rs_c;
+    g.cs_c = d->cs_c;
+    g.m = d->m;
+    g.n = d->n;
+    g.k = d->k * d->npairs;
+    g.alpha = (float)d->alpha;
+    g.beta = (float)d->beta;
+    g.jp = d->product.domain.jp;
+    g.ji = d->product.domain.ji;
+    g.pi = d->product.domain.pi;
+    const FfmaPolicy pol = {d->policy_m > 0 ? d->policy_m : d->m, d->policy_n > 0 ? d->policy_n : d->n};
+    st = launch_ffma_gemm(g, &pol, s);
+  }
+  b200_free(ap);
+  b200_free(bp);
+  return st;
+}
+
+// FP64 on the FMA pipe (MUBLIS_B200_DGEMM=simt).
+int run_simt_dgemm(const b200_l3_desc_t *d) {
+  using C = SimtConfig<double>;
   cudaStream_t s = b200_cur_stream();
   const long ktot = (long)d->k * d->npairs;
   const long mpad = b200_round_up(d->m, C::BM), npad = b200_round_up(d->n, C::BN);
   const long kpad = b200_round_up(ktot, C::BK);
   void *ap = nullptr, *bp = nullptr;
-  B200_TRY(b200_alloc(&ap, sizeof(T) * mpad * kpad));
-  int st = b200_alloc(&bp, sizeof(T) * npad * kpad);
+  B200_TRY(b200_alloc(&ap, sizeof(double) * mpad * kpad));
+  int st = b200_alloc(&bp, sizeof(double) * npad * kpad);
   if (st == B200_OK) {
     PackOut oa{ap, mpad, 0, PACK_MN_MAJOR, PACK_COPY, 1, nullptr};
     PackOut ob{bp, npad, 0, PACK_MN_MAJOR, PACK_COPY, 1, nullptr};
-    st = pack_pairs<T>(d, oa, mpad, ob, npad, kpad, s);
+    st = pack_pairs<double>(d, oa, mpad, ob, npad, kpad, s);
   }
   if (st == B200_OK) {
-    SimtGemmArgs<T> g;
-    g.ap = (const T *)ap;
-    g.bp = (const T *)bp;
+    SimtGemmArgs<double> g;
+    g.ap = (const double *)ap;
+    g.bp = (const double *)bp;
     g.lda = mpad;
     g.ldb = npad;
-    g.c = (T *)d->c;
+    g.c = (double *)d->c;
     g.rs_c = d->rs_c;
     g.cs_c = d->cs_c;
     g.m = d->m;
     g.n = d->n;
     g.k = (int)ktot;
-    g.alpha = (T)d->alpha;
-    g.beta = (T)d->beta;
+    g.alpha = d->alpha;
+    g.beta = d->beta;
     g.jp = d->product.domain.jp;
     g.ji = d->product.domain.ji;
     g.pi = d->product.domain.pi;
     const SimtPolicy pol = {d->policy_m > 0 ? d->policy_m : d->m,
                             d->policy_n > 0 ? d->policy_n : d->n};
-    st = launch_simt_gemm<T>(g, s, &pol);
+    st = launch_simt_gemm<double>(g, s, &pol);
   }
   b200_free(ap);
   b200_free(bp);
@@ -442,6 +503,6 @@ extern "C" int b200_l3_run(const b200_l3_desc_t *d) {
   }
   int st;
   if (try_direct(d, &st)) return st;
-  if (d->dtype == B200_F32) return run_plain<float>(d);
-  return run_plain<double>(d);
+  if (d->dtype == B200_F32) return run_sgemm(d);
+  return use_dmma() ? run_dmma(d) : run_simt_dgemm(d);
 }

@@ -33,6 +33,7 @@
 #include <mutex>
 
 #include "kernels.cuh"
+#include "tc_common.cuh"
 #include "../../include/mublis_b200.h"
 
 #define NOALLOC_SCRATCH_FLOATS (8L << 20) /* 32 MiB of FP32 */
@@ -83,7 +84,8 @@ int scratch_on_current_device(float **out) {
 extern "C" void b200_noalloc_setup(void) {
   float *unused = nullptr;
   (void)scratch_on_current_device(&unused);
-  (void)b200_simt_preload();
+  (void)b200_ffma_preload();
+  (void)b200_scale_preload();
   (void)b200_pack_preload();
 }
 
@@ -107,15 +109,15 @@ extern "C" int mublis_b200_sgemm_noalloc(mublis_trans_t trans_a, mublis_trans_t 
     return b200_stream_sync();
   }
 
-  using Cfg = SimtConfig<float>;
-  const long mpad = b200_round_up(m, Cfg::BM), npad = b200_round_up(n, Cfg::BN);
-  const long kpad = b200_round_up(k, Cfg::BK);
+  constexpr int T = B200_FFMA_TILE, BK = B200_FFMA_BK;
+  const long mpad = b200_round_up(m, T), npad = b200_round_up(n, T);
+  const long kpad = b200_round_up(k, BK);
   if ((mpad + npad) * kpad > NOALLOC_SCRATCH_FLOATS) {
     char msg[256];
     snprintf(msg, sizeof msg,
              "sgemm_noalloc: m=%d n=%d k=%d needs %ld scratch floats "
              "((roundup(m,%d) + roundup(n,%d)) * roundup(k,%d)); the maximum is %ld",
-             m, n, k, (mpad + npad) * kpad, Cfg::BM, Cfg::BN, Cfg::BK, NOALLOC_SCRATCH_FLOATS);
+             m, n, k, (mpad + npad) * kpad, T, T, BK, NOALLOC_SCRATCH_FLOATS);
     return b200_set_error(B200_EINVAL, msg);
   }
   float *scratch = nullptr;
@@ -135,11 +137,9 @@ extern "C" int mublis_b200_sgemm_noalloc(mublis_trans_t trans_a, mublis_trans_t 
   B200_TRY(launch_pack<float>(va, false, m, k, mpad, 0, kpad, oa, s));
   B200_TRY(launch_pack<float>(vb, true, n, k, npad, 0, kpad, ob, s));
 
-  SimtGemmArgs<float> g;
-  g.ap = ap;
-  g.bp = bp;
-  g.lda = mpad;
-  g.ldb = npad;
+  FfmaGemmArgs g;
+  B200_TRY(b200_make_tmap_f32(&g.ta[0], ap, mpad, kpad, mpad, T, BK));
+  B200_TRY(b200_make_tmap_f32(&g.tb[0], bp, npad, kpad, npad, T, BK));
   g.c = c;
   g.rs_c = rs_c;
   g.cs_c = cs_c;
@@ -148,7 +148,6 @@ extern "C" int mublis_b200_sgemm_noalloc(mublis_trans_t trans_a, mublis_trans_t 
   g.k = k;
   g.alpha = alpha;
   g.beta = beta;
-  g.jp = g.ji = g.pi = MUBLIS_L3_ALL;
-  B200_TRY(launch_simt_gemm<float>(g, s));
+  B200_TRY(launch_ffma_gemm(g, nullptr, s));
   return b200_stream_sync();
 }

@@ -41,10 +41,10 @@ void b200_tile_list(long m, long n, long k, int BM, int BN, int BK, b200_tile_do
       const long cost = ke > kb ? (ke + BK - 1) / BK - kb / BK : 0;
       tl.push_back({(int)cost, make_int2((int)tm, (int)tn)});
     }
-  std::stable_sort(tl.begin(), tl.end(), [](const std::pair<int, int2> &x,
-                                            const std::pair<int, int2> &y) {
+  const auto heavier = [](const std::pair<int, int2> &x, const std::pair<int, int2> &y) {
     return x.first > y.first;
-  });
+  };
+  if (!std::is_sorted(tl.begin(), tl.end(), heavier)) std::stable_sort(tl.begin(), tl.end(), heavier);
   if (list) {
     list->resize(tl.size());
     for (size_t i = 0; i < tl.size(); ++i) (*list)[i] = tl[i].second;
@@ -53,6 +53,20 @@ void b200_tile_list(long m, long n, long k, int BM, int BN, int BK, b200_tile_do
     costs->resize(tl.size());
     for (size_t i = 0; i < tl.size(); ++i) (*costs)[i] = tl[i].first;
   }
+}
+
+void b200_snake(std::vector<int2> &list, int grid) {
+  const size_t g = (size_t)std::max(1, std::min((int)list.size(), grid));
+  for (size_t r0 = g; r0 < list.size(); r0 += 2 * g)
+    std::reverse(list.begin() + r0, list.begin() + std::min(list.size(), r0 + g));
+}
+
+bool b200_list_tiles(const std::vector<int2> &list, uint16_t (&tiles)[B200_MAX_LISTED_TILES]) {
+  if (list.size() > B200_MAX_LISTED_TILES) return false;
+  for (const int2 &t : list)
+    if (t.x > 255 || t.y > 255) return false;
+  for (size_t i = 0; i < list.size(); ++i) tiles[i] = (uint16_t)(list[i].x << 8 | list[i].y);
+  return true;
 }
 
 namespace {

@@ -103,6 +103,24 @@ __device__ __forceinline__ void bulk_load_1d(void *smem_dst, const void *gsrc, u
       : "memory");
 }
 
+// One thread: asks for the tile of C that starts at (m0, n0) in L2, line by line
+// along C's unit stride (lines that start on 16 bytes; others are left), so
+// that the epilogue's reads of C find it there instead of in HBM.
+template <typename T>
+__device__ __forceinline__ void prefetch_tile_l2(const T *c, long rs, long cs, int m, int n, int m0,
+                                                 int n0, int tile) {
+  const bool rows = rs == 1;  // the unit stride runs along m
+  if (!rows && cs != 1) return;
+  const long ld = rows ? cs : rs;
+  const T *base = c + m0 * rs + n0 * cs;
+  const int len = min(tile, rows ? m - m0 : n - n0), lines = min(tile, rows ? n - n0 : m - m0);
+  const uint32_t bytes = (uint32_t)(len * sizeof(T)) & ~15u;
+  if (((uintptr_t)base & 15) != 0 || (ld * (long)sizeof(T)) % 16 != 0 || bytes == 0) return;
+  for (int i = 0; i < lines; ++i)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + i * ld), "r"(bytes)
+                 : "memory");
+}
+
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -371,6 +389,8 @@ int b200_make_tmap(CUtensorMap *map, const void *base, int is_bf16, long k, long
 // Host: encode a 2-D FP64 tensor map over a strided matrix: `inner`
 // elements along the unit-stride dimension, `outer` along the other (outer
 // stride in elements), box box_inner x box_outer, 128-byte swizzle or none.
+int b200_make_tmap_f32(CUtensorMap *map, const void *base, long inner, long outer,
+                       long outer_stride, int box_inner, int box_outer);
 int b200_make_tmap_f64(CUtensorMap *map, const void *base, long inner, long outer,
                        long outer_stride, int box_inner, int box_outer, int swizzle128);
 
