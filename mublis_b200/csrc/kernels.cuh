@@ -56,18 +56,19 @@ enum PackLayout {
 
 // Offset of element (mn, kk) of a PACK_FRAG64 panel (Kpad = ld, a multiple
 // of 16; Mpad a multiple of 128).  The panel is a sequence of 128-row
-// strips; a strip is a sequence of k-quads (4 consecutive kk); a k-quad of a
-// strip is 8 blocks of 16 rows, each 32 lanes x 2 doubles in the order an
-// mma.m16n8k4 .f64 fragment is held: lane = 4 (mn % 8) + kk % 4 holds rows
-// mn % 16 < 8 and >= 8 of its block as one 16-byte pair.  An A operand
-// strip is a 16-row block fragment (a0, a1) per lane; a B operand strip is
-// two 8-column fragments (b0 of columns 0-7, b0 of columns 8-15) per lane.
-// So one k-block of 16 of one strip is 16 KB contiguous, and every warp
-// fragment load is 512 contiguous bytes.
+// strips; a strip is a sequence of MMA steps of 4 k (step s of a 16-k block
+// holds k = 8 (s / 2) + 2 t + s % 2, t = 0..3); a step of a strip is 8 blocks
+// of 16 rows, each 32 lanes x 2 doubles in the order an mma.m16n8k4 .f64
+// fragment is held: lane = 4 (mn % 16 / 2) + t holds rows mn % 16 even and odd
+// as one 16-byte pair.  An A operand strip is a 16-row block fragment (a0, a1)
+// per lane; a B operand strip is two 8-column fragments (even columns, odd
+// columns) per lane.  So one k-block of 16 of one strip is 16 KB contiguous,
+// and every warp fragment load is 512 contiguous bytes.
 __host__ __device__ inline long b200_frag64_offset(long mn, long kk, long kpad) {
-  return (((((mn >> 7) * (kpad >> 2) + (kk >> 2)) * 8 + ((mn & 127) >> 4)) * 32 +
-           (((mn & 7) << 2) | (kk & 3))) << 1) |
-         ((mn >> 3) & 1);
+  const long step = (kk >> 4) * 4 + ((kk >> 2) & 2) + (kk & 1);
+  return (((((mn >> 7) * (kpad >> 2) + step) * 8 + ((mn & 127) >> 4)) * 32 +
+           ((((mn >> 1) & 7) << 2) | ((kk >> 1) & 3))) << 1) |
+         (mn & 1);
 }
 
 enum PackXform {
@@ -227,7 +228,8 @@ struct DmmaGemmArgs {
   int m, n, k;
   int tiles_m, tiles_n;
   const int2 *tile_list;  // (tm, tn) of the tiles to compute, or null: all tiles
-  int ntiles;             // entries of tile_list
+  int ntiles;             // tiles to compute
+  int listed = 0;         // they are listed in `tiles`
   double alpha, beta;
   int jp, ji, pi;
   int *err;
@@ -240,19 +242,18 @@ struct DmmaGemmArgs {
   int splits = 1;
   int *arrivals = nullptr;
   double *partials = nullptr;
-  // Direct operand loads (no pack pass): 2-D TMA tiles read straight from
-  // the caller's op(A) and op(B), one tensor map per operand and pair (a
-  // SYR2K's two pairs split k at kpair, a multiple of the k-block).
-  // a_kcontig / b_kcontig: the operand's unit stride runs along k (tiles
-  // then land 128-byte swizzled, k innermost); otherwise along m / n.
-  int direct = 0;
-  int a_kcontig = 0, b_kcontig = 0;
-  int npairs = 1;
-  long kpair = 0;
+  // Each operand's layout (B200_DMMA_*): packed panels (ap / bp), or 2-D TMA
+  // tiles straight from the caller's matrices, one tensor map per pair (a
+  // SYR2K's second pair begins at k = a_kpair / b_kpair, a multiple of the
+  // k-block).
+  int a_layout = 0, b_layout = 0;
+  long a_kpair = 0x7fffffff, b_kpair = 0x7fffffff;
   CUtensorMap ta[2], tb[2];
+  uint16_t tiles[B200_MAX_LISTED_TILES];  // tm << 8 | tn
 };
 int launch_dmma_gemm(const DmmaGemmArgs &a, cudaStream_t s);
 constexpr int B200_DMMA_TILE = 128, B200_DMMA_BK = 16;
+enum { B200_DMMA_PACKED = 0, B200_DMMA_MN = 1 /* unit stride along m / n */, B200_DMMA_K = 2 /* along k */ };
 
 template <typename T>
 struct SimtConfig;

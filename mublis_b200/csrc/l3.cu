@@ -149,57 +149,52 @@ bool overlaps_operand(const b200_l3_desc_t *d) {
   return false;
 }
 
-// The FP64 tensor-pipe kernel can read op(A) and op(B) straight from the
-// caller's memory (2-D TMA tiles) instead of packed panels when no element
-// needs changing on the way: general operands, no jp / pi mask, every pair
-// with the same orientation, a SYR2K's pairs meeting on a k-block boundary,
-// and C overlapping no operand (an in-place product must read its operand
-// before it is overwritten, which only a copy guarantees).
-bool dmma_direct(const b200_l3_desc_t *d, DmmaGemmArgs *g) {
+// One operand of the FP64 tensor-pipe kernel: read in place (2-D TMA tiles)
+// when no element needs changing on the way -- a general, unmasked operand,
+// every pair with the same orientation, a SYR2K's pairs meeting on a k-block
+// boundary -- and it shares no memory with C (an in-place product must read its
+// operand before it is overwritten, which only a copy guarantees); else packed
+// into *panel in fragment order, both pairs as one.  Every route adds the same
+// products in the same order.
+int dmma_operand(const b200_l3_desc_t *d, bool b_side, CUtensorMap (&map)[2], int *layout, long *kpair,
+                 void **panel, cudaStream_t s) {
   const mublis_l3_product_t &pr = d->product;
-  if (!direct_on() || pr.a.struc != MUBLIS_STRUC_GENERAL || pr.b.struc != MUBLIS_STRUC_GENERAL ||
-      pr.domain.jp != MUBLIS_L3_ALL || pr.domain.pi != MUBLIS_L3_ALL)
-    return false;
-  if (d->npairs == 2 && d->k % B200_DMMA_BK != 0) return false;
-  if (overlaps_operand(d)) return false;
-  bool a_mc = false, b_kc = false;
-  for (int t = 0; t < d->npairs; ++t) {
-    bool ac, bc;
-    if (!tma_view_ok(d->a[t], d->rs_a[t], d->cs_a[t], d->m, d->k, &ac) ||
-        !tma_view_ok(d->b[t], d->rs_b[t], d->cs_b[t], d->k, d->n, &bc))
-      return false;
-    if (t == 0) {
-      a_mc = ac;
-      b_kc = bc;
-    } else if (ac != a_mc || bc != b_kc) {
-      return false;
-    }
+  const mublis_l3_operand_t &o = b_side ? pr.b : pr.a;
+  const int mask = b_side ? (int)pr.domain.jp : (int)pr.domain.pi;
+  const void *const *x = b_side ? d->b : d->a;
+  const long *rs = b_side ? d->rs_b : d->rs_a, *cs = b_side ? d->cs_b : d->cs_a;
+  const long rows = b_side ? d->k : d->m, cols = b_side ? d->n : d->k, len = b_side ? d->n : d->m;
+  const int T = B200_DMMA_TILE, BK = B200_DMMA_BK;
+  bool direct = direct_on() && o.struc == MUBLIS_STRUC_GENERAL && mask == MUBLIS_L3_ALL &&
+                (d->npairs == 1 || d->k % BK == 0);
+  for (int t = 0; t < d->npairs && direct; ++t) {
+    bool rows_contig;
+    direct = tma_view_ok(x[t], rs[t], cs[t], rows, cols, &rows_contig) &&
+             !b200_views_overlap(d->c, d->rs_c, d->cs_c, d->m, d->n, x[t], rs[t], cs[t], rows, cols, 8);
+    if (!direct) break;
+    const int lay = rows_contig == b_side ? B200_DMMA_K : B200_DMMA_MN;
+    if (t == 0) *layout = lay;
+    // k innermost: 16 k x 128 rows; m / n innermost: boxes of 16 x 16 k.
+    direct = lay == *layout &&
+             (lay == B200_DMMA_K
+                  ? b200_make_tmap_f64(&map[t], x[t], d->k, len, b_side ? cs[t] : rs[t], BK, T, 1)
+                  : b200_make_tmap_f64(&map[t], x[t], len, d->k, b_side ? rs[t] : cs[t], 16, BK, 1)) ==
+                 B200_OK;
   }
-  // Tensor maps: op(A) tile 128 (m) x 16 (k), op(B) tile 16 (k) x 128 (n);
-  // k innermost tiles are 16 doubles = 128 bytes, 128-byte swizzled.
-  memset(g->ta, 0, sizeof g->ta);
-  memset(g->tb, 0, sizeof g->tb);
-  for (int t = 0; t < d->npairs; ++t) {
-    int st = a_mc ? b200_make_tmap_f64(&g->ta[t], d->a[t], d->m, d->k, d->cs_a[t],
-                                       B200_DMMA_TILE, B200_DMMA_BK, 0)
-                  : b200_make_tmap_f64(&g->ta[t], d->a[t], d->k, d->m, d->rs_a[t],
-                                       B200_DMMA_BK, B200_DMMA_TILE, 1);
-    if (st == B200_OK)
-      st = b_kc ? b200_make_tmap_f64(&g->tb[t], d->b[t], d->k, d->n, d->cs_b[t], B200_DMMA_BK,
-                                     B200_DMMA_TILE, 1)
-                : b200_make_tmap_f64(&g->tb[t], d->b[t], d->n, d->k, d->rs_b[t],
-                                     B200_DMMA_TILE, B200_DMMA_BK, 0);
-    if (st != B200_OK) {
-      b200_set_error(B200_OK, "");  // not an error: fall back to the pack pass
-      return false;
-    }
+  if (direct) {
+    if (d->npairs == 2) *kpair = d->k;
+    return B200_OK;
   }
-  g->direct = 1;
-  g->a_kcontig = !a_mc;
-  g->b_kcontig = b_kc;
-  g->npairs = d->npairs;
-  g->kpair = d->k;
-  return true;
+  *layout = B200_DMMA_PACKED;
+  const long pad = b200_round_up(len, T), kpad = b200_round_up((long)d->k * d->npairs, BK);
+  B200_TRY(b200_alloc(panel, sizeof(double) * pad * kpad));
+  const PackOut out{*panel, kpad, 0, PACK_FRAG64, PACK_COPY, 1, nullptr};
+  for (int t = 0; t < d->npairs; ++t) {
+    const long kk0 = (long)t * d->k, kk1 = t + 1 == d->npairs ? kpad : kk0 + d->k;
+    const PackView v{x[t], rs[t], cs[t], (int)o.struc, (int)o.uplo, (int)o.diag, mask};
+    B200_TRY(launch_pack<double>(v, b_side, len, d->k, pad, kk0, kk1, out, s));
+  }
+  return B200_OK;
 }
 
 int run_dmma(const b200_l3_desc_t *d) {
@@ -209,60 +204,30 @@ int run_dmma(const b200_l3_desc_t *d) {
   const long npad = b200_round_up(d->n, B200_DMMA_TILE);
   const long kpad = b200_round_up(ktot, B200_DMMA_BK);
   DmmaGemmArgs g;
-  const bool direct = dmma_direct(d, &g);
   void *ap = nullptr, *bp = nullptr;
-  int st = B200_OK;
-  if (!direct) {
-    B200_TRY(b200_alloc(&ap, sizeof(double) * mpad * kpad));
-    st = b200_alloc(&bp, sizeof(double) * npad * kpad);
-    if (st == B200_OK) {
-      PackOut oa{ap, kpad, 0, PACK_FRAG64, PACK_COPY, 1, nullptr};
-      PackOut ob{bp, kpad, 0, PACK_FRAG64, PACK_COPY, 1, nullptr};
-      st = pack_pairs<double>(d, oa, mpad, ob, npad, kpad, s);
-    }
-  }
-  // Restricted domains: list the tiles that write (ji) with their k-range
-  // (jp, pi), heaviest first (the host twin of the kernel's tile_krange).
+  int st = dmma_operand(d, false, g.ta, &g.a_layout, &g.a_kpair, &ap, s);
+  if (st == B200_OK) st = dmma_operand(d, true, g.tb, &g.b_layout, &g.b_kpair, &bp, s);
+  // Restricted domains: the tiles that write, heaviest first; in the launch's
+  // parameters when there are few, else uploaded.
   const int tiles_m = (int)(mpad / B200_DMMA_TILE), tiles_n = (int)(npad / B200_DMMA_TILE);
   const mublis_l3_domain_t &dom = d->product.domain;
   void *list = nullptr;
-  int ntiles = 0;
+  int ntiles = tiles_m * tiles_n;
   if (st == B200_OK &&
       (dom.ji != MUBLIS_L3_ALL || dom.jp != MUBLIS_L3_ALL || dom.pi != MUBLIS_L3_ALL)) {
-    std::vector<std::pair<long, int2>> tl;
-    const long T = B200_DMMA_TILE, BK = B200_DMMA_BK;
-    for (int tm = 0; tm < tiles_m; ++tm)
-      for (int tn = 0; tn < tiles_n; ++tn) {
-        const long m0 = tm * T, n0 = tn * T;
-        if (dom.ji == MUBLIS_L3_LOWER && n0 >= m0 + T) continue;
-        if (dom.ji == MUBLIS_L3_UPPER && n0 + T <= m0) continue;
-        long kb = 0, ke = ktot;
-        if (dom.jp == MUBLIS_L3_LOWER) kb = std::max(kb, n0);
-        if (dom.jp == MUBLIS_L3_UPPER) ke = std::min(ke, n0 + T);
-        if (dom.pi == MUBLIS_L3_LOWER) ke = std::min(ke, m0 + T);
-        if (dom.pi == MUBLIS_L3_UPPER) kb = std::max(kb, m0);
-        const long cost = ke > kb ? (ke + BK - 1) / BK - kb / BK : 0;
-        tl.push_back({cost, make_int2(tm, tn)});
-      }
-    std::stable_sort(tl.begin(), tl.end(),
-                     [](const std::pair<long, int2> &x, const std::pair<long, int2> &y) {
-                       return x.first > y.first;
-                     });
-    std::vector<int2> flat(tl.size());
-    for (size_t i = 0; i < tl.size(); ++i) flat[i] = tl[i].second;
+    std::vector<int2> flat;
+    b200_tile_list(d->m, d->n, ktot, B200_DMMA_TILE, B200_DMMA_TILE, B200_DMMA_BK,
+                   {dom.jp, dom.ji, dom.pi}, &flat, nullptr);
     ntiles = (int)flat.size();
-    // The persistent CTAs take tiles round-robin (tile CTA + round * grid);
-    // with the list heaviest first, reversing every other round ("snake")
-    // evens out each CTA's total instead of giving CTA 0 the heaviest tile
-    // of every round.
-    const size_t grid = (size_t)std::min(ntiles, b200_sm_count());
-    for (size_t r0 = grid; grid > 0 && r0 < flat.size(); r0 += 2 * grid)
-      std::reverse(flat.begin() + r0, flat.begin() + std::min(flat.size(), r0 + grid));
-    st = b200_alloc(&list, sizeof(int2) * (ntiles > 0 ? ntiles : 1));
-    if (st == B200_OK && ntiles > 0 &&
-        cudaMemcpyAsync(list, flat.data(), sizeof(int2) * ntiles, cudaMemcpyHostToDevice, s) !=
-            cudaSuccess)
-      st = b200_set_error(B200_ECUDA, "dgemm: tile list upload failed");
+    b200_snake(flat, b200_sm_count());
+    g.listed = b200_list_tiles(flat, g.tiles);
+    if (!g.listed) {
+      st = b200_alloc(&list, sizeof(int2) * ntiles);
+      if (st == B200_OK &&
+          cudaMemcpyAsync(list, flat.data(), sizeof(int2) * ntiles, cudaMemcpyHostToDevice, s) !=
+              cudaSuccess)
+        st = b200_set_error(B200_ECUDA, "dgemm: tile list upload failed");
+    }
   }
   // Split-K from the whole call's shape (column panels carry the call's m
   // and n), so panels split their tiles' k ranges as the whole call does.
@@ -270,15 +235,15 @@ int run_dmma(const b200_l3_desc_t *d) {
                                d->policy_n > 0 ? d->policy_n : d->n, ktot, B200_DMMA_TILE,
                                B200_DMMA_TILE, B200_DMMA_BK, {dom.jp, dom.ji, dom.pi},
                                b200_sm_count(), 8.0);  // 128 KB of partials per split unit
-  const long sched_tiles = list ? ntiles : (long)tiles_m * tiles_n;
+  const long sched_tiles = ntiles;
   void *split_ws = nullptr;
-  if (st == B200_OK && S > 1) {
+  if (st == B200_OK && S > 1 && ntiles > 0) {
     const size_t ints = b200_round_up(sizeof(int) * sched_tiles * 8, 256);
     st = b200_alloc(&split_ws, ints + sizeof(double) * (size_t)sched_tiles * S * 64 * 256);
     if (st == B200_OK && cudaMemsetAsync(split_ws, 0, ints, s) != cudaSuccess)
       st = b200_set_error(B200_ECUDA, "dgemm: split-K counters");
   }
-  if (st == B200_OK && (list == nullptr || ntiles > 0)) {
+  if (st == B200_OK && ntiles > 0) {
     g.ap = (const double *)ap;
     g.bp = (const double *)bp;
     g.kq = kpad / 4;

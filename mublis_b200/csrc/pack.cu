@@ -46,17 +46,18 @@ __global__ void __launch_bounds__(256) pack_kernel(PackView v, bool b_side, long
 
   if (o.layout == PACK_FRAG64) {
     // Fragment-order panel (doubles only): each thread stores the pair
-    // (mn, mn + 8) of one kk as 16 bytes; a warp covers one 16-row block of
-    // one k-quad (512 contiguous bytes when kk_base is a multiple of 4).
+    // (mn, mn + 1) of one kk as 16 bytes; a warp covers one 16-row block of
+    // one MMA step (512 contiguous bytes when kk_base is a multiple of 16).
     if constexpr (sizeof(T) == 8) {
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const int combo = ty + 8 * q;  // 2 blocks of 16 rows x 8 k-quads
-        const int mn_l = (combo & 1) * 16 + (tx >> 2), kk_l = (combo >> 1) * 4 + (tx & 3);
+        const int combo = ty + 8 * q, st = combo >> 1;  // 2 blocks of 16 rows x 8 steps
+        const int mn_l = (combo & 1) * 16 + 2 * (tx >> 2);
+        const int kk_l = (st >> 1) * 8 + 2 * (tx & 3) + (st & 1);
         const long mn = mn_base + mn_l, kk = kk_base + kk_l;
         if (kk >= kk1) continue;
         *reinterpret_cast<double2 *>((double *)o.out + b200_frag64_offset(mn, kk, o.ld)) =
-            make_double2(tile[kk_l][mn_l], tile[kk_l][mn_l + 8]);
+            make_double2(tile[kk_l][mn_l], tile[kk_l][mn_l + 1]);
       }
     }
     return;
@@ -164,13 +165,14 @@ __global__ void __launch_bounds__(256)
     if constexpr (sizeof(T) == 8) {
 #pragma unroll
       for (int q = 0; q < KT / 16; ++q) {
-        const int combo = ty + 8 * q;  // 2 blocks of 16 rows x KT / 4 k-quads
-        const int mn_l = (combo & 1) * 16 + (tx >> 2), kk_l = (combo >> 1) * 4 + (tx & 3);
+        const int combo = ty + 8 * q, st = combo >> 1;  // 2 blocks of 16 rows x KT / 4 steps
+        const int mn_l = (combo & 1) * 16 + 2 * (tx >> 2);
+        const int kk_l = (st >> 1) * 8 + 2 * (tx & 3) + (st & 1);
         const long kk = kk_base + kk_l;
         if (kk >= kk1) continue;
         *reinterpret_cast<double2 *>((double *)o.out +
                                      b200_frag64_offset(mn_base + mn_l, kk, o.ld)) =
-            make_double2(tile[kk_l][mn_l], tile[kk_l][mn_l + 8]);
+            make_double2(tile[kk_l][mn_l], tile[kk_l][mn_l + 1]);
       }
     }
     return;
