@@ -89,15 +89,14 @@ enum PackXform {
 // the tensor cores ran the product noticeably slower on subnormal halves).
 constexpr int B200_FP16_SCALE_EXP = 15;
 
-// Pairwise coprime moduli (<= 256) of the modular (CRT) Ozaki form and the
-// constants that reduce an integer modulo each of them without division:
-// c19/c38 = 2^19/2^38 mod m; mg = ceil(2^39 / m); bias = floor(m/2) + K m
-// with K m >= 2^29 (see b200_sym_mod).
+// Pairwise coprime moduli (<= 256, the first one 256) of the modular (CRT)
+// Ozaki form and the constants of the pack pass's residues (b200_residue).
 constexpr int B200_MAX_MODULI = 16;
 struct B200Moduli {
   int n;
-  int m[B200_MAX_MODULI], c19[B200_MAX_MODULI], c38[B200_MAX_MODULI], bias[B200_MAX_MODULI];
-  unsigned mg[B200_MAX_MODULI];
+  int lo[B200_MAX_MODULI], hi[B200_MAX_MODULI];  // 256^0..3 and 256^4..7 mod m as signed bytes
+  int base[B200_MAX_MODULI];                     // 2^23 as a float's bits, plus an offset
+  float inv[B200_MAX_MODULI], neg_m[B200_MAX_MODULI];  // 1 / m, -m
 };
 
 struct PackOut {
@@ -105,10 +104,32 @@ struct PackOut {
   long ld;
   long plane_stride;  // elements between planes
   int layout, xform, terms;
-  const unsigned long long *absmax;  // INT8 forms: bits of max |x| per mn
+  const int *exps;                   // scaled forms: e of each mn (b200_scale_exp)
   int bits;                          // PACK_INT8_MODULI: |X| <= 2^bits
   B200Moduli mod;                    // PACK_INT8_MODULI
 };
+
+// The symmetric residue of X + 2^56 - (2^56 mod m) ~ X modulo m in the low byte,
+// for |X| <= 2^56 given as the two words of X + 2^56 (unsigned bytes b0 .. b7).
+// v = sum of b_i (256^i mod m) + offset by two byte dot products; the offset (a
+// multiple of m, less 2^56 mod m) keeps v in [0, 2^20), so that with `base` the
+// sum is at once the bits of the float 2^23 + v.  Then r = v - m rint(v / m) in
+// FP32: v < 2^20 and m >= 193 make the quotient's error below 4e-4, while v / m
+// is at least 0.5 / m > 0.0019 away from a half for odd m, so the quotient is
+// exact and r the unique residue in [-(m - 1) / 2, (m - 1) / 2].  (m = 256: the
+// low byte itself.)  Eight instructions, most of them on the FP32 pipe; cutting X
+// into 19-bit pieces in FP64 and reducing with integer multiplies took eleven.
+__device__ __forceinline__ uint32_t b200_residue(uint32_t lo, uint32_t hi, const B200Moduli &mod,
+                                                 int l) {
+  if (l == 0) return lo;
+  int v;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(v) : "r"(lo), "r"(mod.lo[l]), "r"(mod.base[l]));
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(v) : "r"(hi), "r"(mod.hi[l]), "r"(v));
+  const float f = __int_as_float(v) - 8388608.f;
+  const float q = __fadd_rn(__fmaf_rn(f, mod.inv[l], 12582912.f), -12582912.f);
+  const float r = __fmaf_rn(q, mod.neg_m[l], f);
+  return (uint32_t)__float_as_int(__fadd_rn(r, 12582912.f));  // 1.5 2^23 + r
+}
 
 // Symmetric residue of t modulo m, in [-floor(m/2), m - 1 - floor(m/2)]
 // (within [-128, 127] for m <= 256), for |t| <= 2^29.  u = t + bias lies in
@@ -151,6 +172,23 @@ __device__ __forceinline__ double b200_pow2_scale(double x, int e) {
   return e >= -1022 && e <= 1023 ? x * __longlong_as_double((long long)(e + 1023) << 52)
                                  : ldexp(x, e);
 }
+
+// x * 2^sh for sh within [-300, 300], as two multiplications by exact powers
+// of two: the first is the whole factor whenever 2^sh is a normal float (then
+// it is one rounding of the exact product, as ldexpf gives); for larger |sh|
+// the factor is cut in two.
+__device__ __forceinline__ void b200_pow2_factors(int sh, float &f1, float &f2) {
+  const int s1 = sh > 127 ? 127 : (sh < -126 ? -126 : sh);
+  f1 = __int_as_float((s1 + 127) << 23);
+  f2 = __int_as_float((sh - s1 + 127) << 23);
+}
+
+// Scale exponents (exps, mn_pad of them) and packed planes of a whole operand in
+// one pass over it, for k [0, kk1): false, with nothing launched, when the
+// operand or the form is not one it takes (then absmax, scale_exps and pack).
+template <typename T>
+bool launch_scale_pack(const PackView &v, bool b_side, long mn_len, long k_len, long mn_pad, long kk1,
+                       int *exps, const PackOut &o, cudaStream_t s);
 
 template <typename T>
 int launch_pack(const PackView &v, bool b_side, long mn_len, long k_len, long mn_pad,

@@ -16,9 +16,19 @@
 //     (hi = rn(x), lo = rn(x - hi), lo2 = rn(x - hi - lo)) in the same pass.
 // Elements outside the stored triangle of a structured operand are never
 // read (the reference's tests poison them with NaN).
+#include <cstring>
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace {
+
+// X = rint(x * 2^sh), |X| <= 2^56, as the two words of X + 2^56.
+__device__ __forceinline__ void modular_integer(double x, int sh, uint32_t &lo, uint32_t &hi) {
+  const long long v = __double2ll_rn(b200_pow2_scale(x, sh)) + (1ll << 56);
+  lo = (uint32_t)v;
+  hi = (uint32_t)((unsigned long long)v >> 32);
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256) pack_kernel(PackView v, bool b_side, long mn_len,
@@ -78,7 +88,7 @@ __global__ void __launch_bounds__(256) pack_kernel(PackView v, bool b_side, long
       // Error-free 7-bit slicing (truncation keeps every slice in [-127, 127]):
       // r = x * 2^(7 - e) in (-128, 128); q_t = trunc(r); r = (r - q_t) * 128.
       int8_t *out = (int8_t *)o.out;
-      double r = ldexp((double)val, 7 - b200_scale_exp(o.absmax[mn]));
+      double r = ldexp((double)val, 7 - o.exps[mn]);
       for (int t = 0; t < o.terms; ++t) {
         double q = trunc(r);
         out[off + t * o.plane_stride] = (int8_t)(int)q;
@@ -86,26 +96,18 @@ __global__ void __launch_bounds__(256) pack_kernel(PackView v, bool b_side, long
       }
     } else if (o.xform == PACK_FP16_SPLIT) {
       __half *out = (__half *)o.out;
-      const float xs = ldexpf((float)val, B200_FP16_SCALE_EXP - b200_scale_exp(o.absmax[mn]));
+      const float xs = ldexpf((float)val, B200_FP16_SCALE_EXP - o.exps[mn]);
       const __half hi = __float2half_rn(xs);
       out[off] = hi;
       out[off + o.plane_stride] = __float2half_rn(xs - __half2float(hi));
     } else if (o.xform == PACK_INT8_MODULI) {
-      // X = rint(x * 2^(bits - e)) is an integer with |X| <= 2^bits <= 2^56,
-      // exact in FP64.  Cut it into 19-bit pieces X = x2 2^38 + x1 2^19 + x0
-      // (every step exact), so that X mod m is the residue of
-      // x2 c38 + x1 c19 + x0, an int32 below 2^28 in magnitude.
+      uint32_t lo, hi;
+      modular_integer((double)val, o.bits - o.exps[mn], lo, hi);
       int8_t *out = (int8_t *)o.out;
-      const double x = rint(ldexp((double)val, o.bits - b200_scale_exp(o.absmax[mn])));
-      const double d2 = floor(x * 0x1p-38), r2 = fma(-d2, 0x1p38, x);
-      const double d1 = floor(r2 * 0x1p-19);
-      const int x2 = (int)d2, x1 = (int)d1, x0 = (int)fma(-d1, 0x1p19, r2);
 #pragma unroll
       for (int t = 0; t < B200_MAX_MODULI; ++t) {  // constant indices: no local copy
         if (t >= o.terms) break;
-        const int v = x2 * o.mod.c38[t] + x1 * o.mod.c19[t] + x0;
-        out[off + t * o.plane_stride] =
-            (int8_t)b200_sym_mod(v, o.mod.m[t], o.mod.mg[t], o.mod.bias[t]);
+        out[off + t * o.plane_stride] = (int8_t)b200_residue(lo, hi, o.mod, t);
       }
     } else {
       __nv_bfloat16 *out = (__nv_bfloat16 *)o.out;
@@ -186,16 +188,16 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// K-major panels (the tensor-core forms): a CTA covers 32 rows (mn) x 64 k.
-// Each thread turns 8 consecutive k of one row into every output plane and
-// writes them as one vector per plane (16 bytes of bf16, 8 bytes of int8,
-// 32/64 bytes of T), so a warp writes 4 rows x 128 contiguous bytes of bf16
-// per plane instead of 2-byte scattered stores.  Requires kk0 and the
-// panel's row pitch to be multiples of 8 (every K-major panel is padded to
-// the MMA k-block).
-template <typename T>
-__device__ __forceinline__ void kmajor_store8(const PackOut &o, long mn, long off, const T (&v)[8]) {
-  if (o.xform == PACK_BF16_SPLIT) {
+// K-major panels (the tensor-core forms).  A thread turns 8 consecutive k of one
+// row (mn) into every output plane and writes each as one vector (16 bytes of
+// bf16 / fp16, 8 bytes of int8), so a warp writes whole 128-byte lines.
+// Requires kk0 and the panel's row pitch to be multiples of 8 (every K-major
+// panel is padded to the MMA k-block).  What bounds it is HBM for the
+// two- and three-plane splits and the residue arithmetic for the int8 moduli.
+// e: the row's scale exponent (scaled forms).
+template <typename T, int XF>
+__device__ __forceinline__ void kmajor_store8(const PackOut &o, int e, long off, const T (&v)[8]) {
+  if constexpr (XF == PACK_BF16_SPLIT) {
     __nv_bfloat16 *out = (__nv_bfloat16 *)o.out;
     __align__(16) __nv_bfloat16 h[8], l[8], l2[8];
 #pragma unroll
@@ -211,44 +213,42 @@ __device__ __forceinline__ void kmajor_store8(const PackOut &o, long mn, long of
     if (o.terms > 2)
       *reinterpret_cast<uint4 *>(out + off + 2 * o.plane_stride) =
           *reinterpret_cast<const uint4 *>(l2);
-  } else if (o.xform == PACK_FP16_SPLIT) {
+  } else if constexpr (XF == PACK_FP16_SPLIT) {
     __half *out = (__half *)o.out;
-    const int sh = B200_FP16_SCALE_EXP - b200_scale_exp(o.absmax[mn]);
-    __align__(16) __half h[8], l[8];
+    float f1, f2;
+    b200_pow2_factors(B200_FP16_SCALE_EXP - e, f1, f2);
+    __align__(16) __half2 h[4], l[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float xs = ldexpf((float)v[j], sh);
-      h[j] = __float2half_rn(xs);
-      l[j] = __float2half_rn(xs - __half2float(h[j]));
+    for (int j = 0; j < 4; ++j) {  // two elements per conversion
+      const float a = ((float)v[2 * j] * f1) * f2, b = ((float)v[2 * j + 1] * f1) * f2;
+      h[j] = __floats2half2_rn(a, b);
+      const float2 hf = __half22float2(h[j]);
+      l[j] = __floats2half2_rn(a - hf.x, b - hf.y);
     }
     *reinterpret_cast<uint4 *>(out + off) = *reinterpret_cast<const uint4 *>(h);
     *reinterpret_cast<uint4 *>(out + off + o.plane_stride) = *reinterpret_cast<const uint4 *>(l);
-  } else if (o.xform == PACK_INT8_MODULI) {
+  } else if constexpr (XF == PACK_INT8_MODULI) {
     int8_t *out = (int8_t *)o.out;
-    const int sh = o.bits - b200_scale_exp(o.absmax[mn]);
-    int x2[8], x1[8], x0[8];
+    const int sh = o.bits - e;
+    uint32_t lo[8], hi[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const double x = rint(ldexp((double)v[j], sh));
-      const double d2 = floor(x * 0x1p-38), r2 = fma(-d2, 0x1p38, x);
-      const double d1 = floor(r2 * 0x1p-19);
-      x2[j] = (int)d2, x1[j] = (int)d1, x0[j] = (int)fma(-d1, 0x1p19, r2);
-    }
+    for (int j = 0; j < 8; ++j) modular_integer((double)v[j], sh, lo[j], hi[j]);
 #pragma unroll
     for (int t = 0; t < B200_MAX_MODULI; ++t) {
       if (t >= o.terms) break;
-      uint32_t w[2] = {0, 0};
+      uint32_t w[2];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int r = b200_sym_mod(x2[j] * o.mod.c38[t] + x1[j] * o.mod.c19[t] + x0[j],
-                                   o.mod.m[t], o.mod.mg[t], o.mod.bias[t]);
-        w[j >> 2] |= (uint32_t)(r & 0xff) << (8 * (j & 3));
+      for (int q = 0; q < 2; ++q) {
+        uint32_t r[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = b200_residue(lo[4 * q + j], hi[4 * q + j], o.mod, t);
+        w[q] = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
       }
       *reinterpret_cast<uint2 *>(out + off + t * o.plane_stride) = make_uint2(w[0], w[1]);
     }
-  } else if (o.xform == PACK_INT8_SLICES) {
+  } else if constexpr (XF == PACK_INT8_SLICES) {
     int8_t *out = (int8_t *)o.out;
-    const int sh = 7 - b200_scale_exp(o.absmax[mn]);
+    const int sh = 7 - e;
     double r[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) r[j] = ldexp((double)v[j], sh);
@@ -262,33 +262,38 @@ __device__ __forceinline__ void kmajor_store8(const PackOut &o, long mn, long of
       }
       *reinterpret_cast<uint2 *>(out + off + t * o.plane_stride) = make_uint2(w[0], w[1]);
     }
-  } else {
-    T *out = (T *)o.out + off;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) out[j] = v[j];
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256) pack_kmajor_kernel(PackView v, bool b_side, long mn_len,
-                                                          long k_len, long kk0, long kk1,
-                                                          PackOut o, bool mn_fast_load) {
+// A CTA covers 32 rows (mn) x 64 k through shared memory.  DENSE: a general,
+// unmasked operand (no element needs looking at).
+template <typename T, int XF, bool DENSE>
+__global__ void __launch_bounds__(256) pack_kmajor_kernel(const __grid_constant__ PackView v,
+                                                          bool b_side, long mn_len, long k_len,
+                                                          long kk0, long kk1,
+                                                          const __grid_constant__ PackOut o,
+                                                          bool mn_fast_load) {
   __shared__ T tile[64][33];  // [kk_local][mn_local]
   const int tid = threadIdx.x;
   const long mn_base = (long)blockIdx.x * 32;
   const long kk_base = kk0 + (long)blockIdx.y * 64;
+  const long s_mn = b_side ? v.cs : v.rs, s_k = b_side ? v.rs : v.cs;
+  T val[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int e = tid + 256 * q;  // 2048 elements
     const int mn_l = mn_fast_load ? e & 31 : e >> 6;
     const int kk_l = mn_fast_load ? e >> 5 : e & 63;
     const long mn = mn_base + mn_l, kk = kk_base + kk_l, kl = kk - kk0;
-    T val = T(0);
-    if (mn < mn_len && kl < k_len && kk < kk1) {
-      const long r = b_side ? kl : mn, c = b_side ? mn : kl;
-      val = load_logical<T>(v, r, c);
-    }
-    tile[kk_l][mn_l] = val;
+    val[q] = T(0);
+    if (mn < mn_len && kl < k_len && kk < kk1)
+      val[q] = DENSE ? ((const T *)v.x)[mn * s_mn + kl * s_k]
+                     : load_logical<T>(v, b_side ? kl : mn, b_side ? mn : kl);
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int e = tid + 256 * q;
+    tile[mn_fast_load ? e >> 5 : e & 63][mn_fast_load ? e & 31 : e >> 6] = val[q];
   }
   __syncthreads();
   const int mn_l = tid >> 3, kc = (tid & 7) * 8;
@@ -297,7 +302,181 @@ __global__ void __launch_bounds__(256) pack_kmajor_kernel(PackView v, bool b_sid
   T vals[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) vals[j] = tile[kc + j][mn_l];
-  kmajor_store8<T>(o, mn, mn * o.ld + kk, vals);
+  kmajor_store8<T, XF>(o, XF == PACK_BF16_SPLIT ? 0 : o.exps[mn], mn * o.ld + kk, vals);
+}
+
+// A general, unmasked operand whose unit stride runs along k, every row on 16
+// bytes: no transpose, so straight from 16-byte loads.  A warp covers 256 k of
+// one row, a CTA 8 warps x ROWS rows; all of a thread's loads go out first.
+template <typename T, int XF>
+__global__ void __launch_bounds__(256) pack_kmajor_rows_kernel(const T *__restrict__ x, long s_mn,
+                                                               long mn_len, long mn_pad, long k_len,
+                                                               long kk0, long kk1,
+                                                               const __grid_constant__ PackOut o) {
+  constexpr int ROWS = sizeof(T) == 4 ? 4 : 2, VEC = 16 / sizeof(T);
+  const long kl = ((long)blockIdx.y * 32 + (threadIdx.x & 31)) * 8;
+  const long mn0 = ((long)blockIdx.x * 8 + (threadIdx.x >> 5)) * ROWS;
+  if (kk0 + kl >= kk1) return;
+  T v[ROWS][8];
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r) {
+    const T *src = x + (mn0 + r) * s_mn + kl;
+    if (mn0 + r < mn_len && kl + 8 <= k_len) {
+#pragma unroll
+      for (int c = 0; c < 8 / VEC; ++c) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(src) + c);
+        memcpy(&v[r][c * VEC], &w, 16);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[r][j] = mn0 + r < mn_len && kl + j < k_len ? src[j] : T(0);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < ROWS; ++r)
+    if (mn0 + r < mn_pad)
+      kmajor_store8<T, XF>(o, XF == PACK_BF16_SPLIT ? 0 : o.exps[mn0 + r],
+                           (mn0 + r) * o.ld + kk0 + kl, v[r]);
+}
+
+// A general, unmasked operand whose unit stride runs along mn, every k row on 16
+// bytes: 16-byte loads of a TILE_MN x 64 k tile (four per thread in flight),
+// transposed through shared memory.  8192^2 FP32 into two fp16 planes: 150 us
+// with the 32 x 64 tiles of 4-byte loads above, 91 here (the copy alone: 80).
+template <typename T, int XF>
+__global__ void __launch_bounds__(256) pack_kmajor_cols_kernel(const T *__restrict__ x, long s_k,
+                                                               long mn_len, long mn_pad, long k_len,
+                                                               long kk0, long kk1,
+                                                               const __grid_constant__ PackOut o) {
+  constexpr int VEC = 16 / sizeof(T), TILE_MN = 16 * VEC, LOADS = 4;
+  __shared__ T tile[64][TILE_MN + 1];
+  const int tid = threadIdx.x;
+  const long mn_base = (long)blockIdx.x * TILE_MN, kl_base = (long)blockIdx.y * 64;
+  const int c = (tid & 15) * VEC, k_l = tid >> 4;
+  T v[LOADS][VEC];
+#pragma unroll
+  for (int q = 0; q < LOADS; ++q) {
+    const long mn = mn_base + c, kl = kl_base + k_l + 16 * q;
+    const T *src = x + kl * s_k + mn;
+    if (kl < k_len && mn + VEC <= mn_len) {
+      const uint4 w = __ldg(reinterpret_cast<const uint4 *>(src));
+      memcpy(v[q], &w, 16);
+    } else {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) v[q][j] = kl < k_len && mn + j < mn_len ? src[j] : T(0);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < LOADS; ++q)
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) tile[k_l + 16 * q][c + j] = v[q][j];
+  __syncthreads();
+  const int kc = (tid & 7) * 8;
+  if (kk0 + kl_base + kc >= kk1) return;
+#pragma unroll
+  for (int mn_l = tid >> 3; mn_l < TILE_MN; mn_l += 32) {
+    const long mn = mn_base + mn_l;
+    if (mn >= mn_pad) return;
+    T vals[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) vals[j] = tile[kc + j][mn_l];
+    kmajor_store8<T, XF>(o, XF == PACK_BF16_SPLIT ? 0 : o.exps[mn], mn * o.ld + kk0 + kl_base + kc,
+                         vals);
+  }
+}
+
+// absmax and pack in one pass over HBM, for a general, unmasked operand whose unit
+// stride runs along k and whose scale covers this k alone (one pair): WARPS
+// warps find a row's abs-max, write its exponent and read the row again, from
+// L2, to pack it.  8192^2 FP32 into two fp16 planes: 94 us for both (the copy
+// alone takes 80), 72 + 89 as two kernels.
+// ALIGNED: every row on 16 bytes.
+template <typename T, int XF, int WARPS, bool ALIGNED>
+__global__ void __launch_bounds__(256) scale_pack_rows_kernel(const T *__restrict__ x, long s_mn,
+                                                              long mn_len, long mn_pad, long k_len,
+                                                              long kk1, int *__restrict__ exps,
+                                                              const __grid_constant__ PackOut o) {
+  constexpr int VEC = 16 / sizeof(T), TEAM = 32 * WARPS, TEAMS = 256 / TEAM;
+  const int t = threadIdx.x % TEAM;
+  const long mn = (long)blockIdx.x * TEAMS + threadIdx.x / TEAM;
+  if (TEAMS > 1 && mn >= mn_pad) return;  // (one team: the grid is mn_pad)
+  const T *row = x + mn * s_mn;
+  const bool exists = mn < mn_len;
+  const long k_full = exists && ALIGNED ? k_len / VEC * VEC : 0;
+  T mx = T(0);
+#pragma unroll 4
+  for (long k = (long)t * VEC; k < k_full; k += TEAM * VEC) {
+    const uint4 w = *reinterpret_cast<const uint4 *>(row + k);
+    T v[VEC];
+    memcpy(v, &w, 16);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) mx = fmax(mx, fabs(v[j]));
+  }
+  if (exists) {
+#pragma unroll 8
+    for (long k = k_full + t; k < k_len; k += TEAM) mx = fmax(mx, fabs(row[k]));
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, s));
+  if constexpr (WARPS > 1) {
+    __shared__ T part[8];
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = part[0];
+#pragma unroll
+    for (int q = 1; q < WARPS; ++q) mx = fmax(mx, part[q]);
+  }
+  const int e = b200_scale_exp((unsigned long long)__double_as_longlong((double)mx));
+  if (t == 0) exps[mn] = e;
+  for (long k = (long)t * 8; k < kk1; k += TEAM * 8) {
+    T v[8];
+    if (ALIGNED && exists && k + 8 <= k_len) {
+#pragma unroll
+      for (int c = 0; c < 8 / VEC; ++c) {
+        const uint4 w = *(reinterpret_cast<const uint4 *>(row + k) + c);
+        memcpy(&v[c * VEC], &w, 16);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = exists && k + j < k_len ? row[k + j] : T(0);
+    }
+    kmajor_store8<T, XF>(o, e, mn * o.ld + k, v);
+  }
+}
+
+template <typename T, int XF>
+int launch_kmajor(const PackView &v, bool b_side, long mn_len, long k_len, long mn_pad, long kk0,
+                  long kk1, const PackOut &o, cudaStream_t s) {
+  const long s_mn = b_side ? v.cs : v.rs, s_k = b_side ? v.rs : v.cs;
+  const bool dense = v.struc == MUBLIS_STRUC_GENERAL && v.mask_rel == MUBLIS_L3_ALL;
+  if (dense && s_k == 1 && s_mn > 0 && s_mn * sizeof(T) % 16 == 0 && ((uintptr_t)v.x & 15) == 0) {
+    constexpr int ROWS = sizeof(T) == 4 ? 4 : 2;
+    dim3 grid((unsigned)b200_ceil_div(mn_pad, 8 * ROWS), (unsigned)b200_ceil_div(kk1 - kk0, 256));
+    if (grid.y > 65535) return b200_set_error(B200_EINVAL, "pack: k extent too large");
+    pack_kmajor_rows_kernel<T, XF>
+        <<<grid, 256, 0, s>>>((const T *)v.x, s_mn, mn_len, mn_pad, k_len, kk0, kk1, o);
+    B200_LAUNCH_CHECK();
+    return B200_OK;
+  }
+  if (dense && s_mn == 1 && s_k > 0 && s_k * sizeof(T) % 16 == 0 && ((uintptr_t)v.x & 15) == 0) {
+    dim3 grid((unsigned)b200_ceil_div(mn_pad, 256 / sizeof(T)), (unsigned)b200_ceil_div(kk1 - kk0, 64));
+    if (grid.y > 65535) return b200_set_error(B200_EINVAL, "pack: k extent too large");
+    pack_kmajor_cols_kernel<T, XF>
+        <<<grid, 256, 0, s>>>((const T *)v.x, s_k, mn_len, mn_pad, k_len, kk0, kk1, o);
+    B200_LAUNCH_CHECK();
+    return B200_OK;
+  }
+  dim3 grid((unsigned)b200_ceil_div(mn_pad, 32), (unsigned)b200_ceil_div(kk1 - kk0, 64));
+  if (grid.y > 65535) return b200_set_error(B200_EINVAL, "pack: k extent too large");
+  const bool mn_fast = labs(s_mn) <= labs(s_k);
+  if (dense)
+    pack_kmajor_kernel<T, XF, true>
+        <<<grid, 256, 0, s>>>(v, b_side, mn_len, k_len, kk0, kk1, o, mn_fast);
+  else
+    pack_kmajor_kernel<T, XF, false>
+        <<<grid, 256, 0, s>>>(v, b_side, mn_len, k_len, kk0, kk1, o, mn_fast);
+  B200_LAUNCH_CHECK();
+  return B200_OK;
 }
 
 // Abs-max per row of op(A) / column of op(B), for the power-of-two scaling
@@ -308,22 +487,24 @@ __global__ void __launch_bounds__(256) pack_kmajor_kernel(PackView v, bool b_sid
 //
 // absmax_kernel is the general form (structured and masked operands, any
 // strides): 32 rows per block, loads along whichever index is contiguous.
-template <typename T>
+template <typename T, bool DENSE>
 __global__ void __launch_bounds__(256) absmax_kernel(PackView v, bool b_side, long mn_len,
                                                      long k_len, long kch, bool mn_fast_load,
                                                      unsigned long long *absmax) {
-  __shared__ double part[8][33];
+  __shared__ T part[8][33];
+  const T *x = (const T *)v.x;
+  const long s_mn = b_side ? v.cs : v.rs, s_k = b_side ? v.rs : v.cs;
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   const long mn_base = (long)blockIdx.x * 32, k0 = (long)blockIdx.y * kch;
   const long k1 = k0 + kch < k_len ? k0 + kch : k_len;
   if (mn_fast_load) {
     const long mn = mn_base + tx;
-    double mx = 0.0;
+    T mx = T(0);
     if (mn < mn_len) {
-#pragma unroll 4
+#pragma unroll 8
       for (long kk = k0 + ty; kk < k1; kk += 8) {
         long r = b_side ? kk : mn, c = b_side ? mn : kk;
-        mx = fmax(mx, fabs((double)load_logical<T>(v, r, c)));
+        mx = fmax(mx, fabs(DENSE ? x[mn * s_mn + kk * s_k] : load_logical<T>(v, r, c)));
       }
     }
     part[ty][tx] = mx;
@@ -331,8 +512,8 @@ __global__ void __launch_bounds__(256) absmax_kernel(PackView v, bool b_side, lo
     if (ty == 0) {
 #pragma unroll
       for (int q = 1; q < 8; ++q) mx = fmax(mx, part[q][tx]);
-      if (mn < mn_len && mx > 0.0)
-        atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong(mx));
+      if (mn < mn_len && mx > T(0))
+        atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong((double)mx));
     }
     return;
   }
@@ -340,16 +521,16 @@ __global__ void __launch_bounds__(256) absmax_kernel(PackView v, bool b_side, lo
   for (int q = 0; q < 4; ++q) {
     const long mn = mn_base + ty + 8 * q;
     if (mn >= mn_len) break;  // uniform across the warp
-    double mx = 0.0;
-#pragma unroll 4
+    T mx = T(0);
+#pragma unroll 8
     for (long kk = k0 + tx; kk < k1; kk += 32) {
       long r = b_side ? kk : mn, c = b_side ? mn : kk;
-      mx = fmax(mx, fabs((double)load_logical<T>(v, r, c)));
+      mx = fmax(mx, fabs(DENSE ? x[mn * s_mn + kk * s_k] : load_logical<T>(v, r, c)));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (tx == 0 && mx > 0.0)
-      atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong(mx));
+    if (tx == 0 && mx > T(0))
+      atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong((double)mx));
   }
 }
 
@@ -358,13 +539,12 @@ template <typename T> struct Vec16;
 template <> struct Vec16<float> {
   using V = float4;
   static constexpr int N = 4;
-  __device__ static void fold(double (&m)[4], const V &x) {
-    m[0] = fmax(m[0], fabs((double)x.x)); m[1] = fmax(m[1], fabs((double)x.y));
-    m[2] = fmax(m[2], fabs((double)x.z)); m[3] = fmax(m[3], fabs((double)x.w));
+  __device__ static void fold(float (&m)[4], const V &x) {
+    m[0] = fmaxf(m[0], fabsf(x.x)); m[1] = fmaxf(m[1], fabsf(x.y));
+    m[2] = fmaxf(m[2], fabsf(x.z)); m[3] = fmaxf(m[3], fabsf(x.w));
   }
-  __device__ static double fold1(const V &x) {
-    return fmax(fmax(fabs((double)x.x), fabs((double)x.y)),
-                fmax(fabs((double)x.z), fabs((double)x.w)));
+  __device__ static float fold1(const V &x) {
+    return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w)));
   }
 };
 template <> struct Vec16<double> {
@@ -395,47 +575,47 @@ __global__ void __launch_bounds__(256) absmax_dense_kernel(const T *x, long ld, 
   const long k0 = (long)blockIdx.y * kch;
   const long k1 = k0 + kch < k_len ? k0 + kch : k_len;
   if (MN_CONTIG) {
-    __shared__ double part[8][32 * VN];
+    __shared__ T part[8][32 * VN];
     const long mn0 = (long)blockIdx.x * (32 * VN) + lane * VN;
-    double m[VN];
+    T m[VN];
 #pragma unroll
-    for (int e = 0; e < VN; ++e) m[e] = 0.0;
+    for (int e = 0; e < VN; ++e) m[e] = T(0);
     if (mn0 + VN <= mn_len) {
 #pragma unroll 4
       for (long kk = k0 + warp; kk < k1; kk += 8) VT::fold(m, *(const V *)(x + kk * ld + mn0));
     } else if (mn0 < mn_len) {
       for (long kk = k0 + warp; kk < k1; kk += 8)
         for (int e = 0; e < VN && mn0 + e < mn_len; ++e)
-          m[e] = fmax(m[e], fabs((double)x[kk * ld + mn0 + e]));
+          m[e] = fmax(m[e], fabs(x[kk * ld + mn0 + e]));
     }
 #pragma unroll
     for (int e = 0; e < VN; ++e) part[warp][lane * VN + e] = m[e];
     __syncthreads();
     if (threadIdx.x < 32 * VN) {
       const long mn = (long)blockIdx.x * (32 * VN) + threadIdx.x;
-      double mx = part[0][threadIdx.x];
+      T mx = part[0][threadIdx.x];
 #pragma unroll
       for (int q = 1; q < 8; ++q) mx = fmax(mx, part[q][threadIdx.x]);
-      if (mn < mn_len && mx > 0.0)
-        atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong(mx));
+      if (mn < mn_len && mx > T(0))
+        atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong((double)mx));
     }
   } else {
     const long mn = (long)blockIdx.x * 8 + warp;
     if (mn >= mn_len) return;  // whole warp
     const T *row = x + mn * ld;
-    double mx = 0.0;
+    T mx = T(0);
 #pragma unroll 8
     for (long kk = k0 + lane * VN; kk < k1; kk += 32 * VN) {
       if (kk + VN <= k1) {
         mx = fmax(mx, VT::fold1(*(const V *)(row + kk)));
       } else {
-        for (long t = kk; t < k1; ++t) mx = fmax(mx, fabs((double)row[t]));
+        for (long t = kk; t < k1; ++t) mx = fmax(mx, fabs(row[t]));
       }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (lane == 0 && mx > 0.0)
-      atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong(mx));
+    if (lane == 0 && mx > T(0))
+      atomicMax(&absmax[mn], (unsigned long long)__double_as_longlong((double)mx));
   }
 }
 
@@ -485,7 +665,9 @@ int launch_absmax(const PackView &v, bool b_side, long mn_len, long k_len,
   const long kch = absmax_kch(bx, k_len, 64, 1024);
   dim3 grid((unsigned)bx, (unsigned)b200_ceil_div(k_len, kch));
   if (grid.y > 65535) return b200_set_error(B200_EINVAL, "absmax: k extent too large");
-  absmax_kernel<T><<<grid, dim3(32, 8), 0, s>>>(v, b_side, mn_len, k_len, kch, mn_fast, absmax);
+  const bool plain = v.struc == MUBLIS_STRUC_GENERAL && v.mask_rel == MUBLIS_L3_ALL;
+  auto kern = plain ? absmax_kernel<T, true> : absmax_kernel<T, false>;
+  kern<<<grid, dim3(32, 8), 0, s>>>(v, b_side, mn_len, k_len, kch, mn_fast, absmax);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -506,6 +688,45 @@ int launch_scale_exps(const unsigned long long *absmax, int *exps, long count, c
 }
 
 template <typename T>
+bool launch_scale_pack(const PackView &v, bool b_side, long mn_len, long k_len, long mn_pad, long kk1,
+                       int *exps, const PackOut &o, cudaStream_t s) {
+  const long s_mn = b_side ? v.cs : v.rs, s_k = b_side ? v.rs : v.cs;
+  if (v.struc != MUBLIS_STRUC_GENERAL || v.mask_rel != MUBLIS_L3_ALL || s_k != 1 || s_mn <= 0 ||
+      o.layout != PACK_K_MAJOR || kk1 % 8 != 0 || o.ld % 8 != 0 || mn_pad % 8 != 0 ||
+      mn_pad > 0x7fffffffL)
+    return false;
+  const bool aligned = s_mn * sizeof(T) % 16 == 0 && ((uintptr_t)v.x & 15) == 0;
+  auto launch = [&](auto xf) {
+    constexpr int XF = decltype(xf)::value;
+    // Rows of up to 1024 k: a warp each; longer ones: the whole CTA.
+    const bool wide = kk1 > 1024;
+    auto kern = wide ? (aligned ? scale_pack_rows_kernel<T, XF, 8, true>
+                                : scale_pack_rows_kernel<T, XF, 8, false>)
+                     : (aligned ? scale_pack_rows_kernel<T, XF, 1, true>
+                                : scale_pack_rows_kernel<T, XF, 1, false>);
+    B200ProfScope prof("pack", s);
+    kern<<<(unsigned)(wide ? mn_pad : mn_pad / 8), 256, 0, s>>>((const T *)v.x, s_mn, mn_len, mn_pad,
+                                                                k_len, kk1, exps, o);
+  };
+  if (o.xform == PACK_INT8_MODULI) {
+    launch(std::integral_constant<int, PACK_INT8_MODULI>());
+    return true;
+  }
+  if constexpr (sizeof(T) == 4) {
+    if (o.xform == PACK_FP16_SPLIT) {
+      launch(std::integral_constant<int, PACK_FP16_SPLIT>());
+      return true;
+    }
+  }
+  return false;
+}
+
+template bool launch_scale_pack<float>(const PackView &, bool, long, long, long, long, int *,
+                                       const PackOut &, cudaStream_t);
+template bool launch_scale_pack<double>(const PackView &, bool, long, long, long, long, int *,
+                                        const PackOut &, cudaStream_t);
+
+template <typename T>
 int launch_pack(const PackView &v, bool b_side, long mn_len, long k_len, long mn_pad, long kk0,
                 long kk1, const PackOut &o, cudaStream_t s) {
   if (mn_pad <= 0 || kk1 <= kk0) return B200_OK;
@@ -515,11 +736,16 @@ int launch_pack(const PackView &v, bool b_side, long mn_len, long k_len, long mn
   B200ProfScope prof("pack", s);
   if (o.layout == PACK_K_MAJOR && mn_pad % 32 == 0 && kk0 % 8 == 0 && (kk1 - kk0) % 8 == 0 &&
       o.ld % 8 == 0) {
-    dim3 grid((unsigned)b200_ceil_div(mn_pad, 32), (unsigned)b200_ceil_div(kk1 - kk0, 64));
-    if (grid.y > 65535) return b200_set_error(B200_EINVAL, "pack: k extent too large");
-    pack_kmajor_kernel<T><<<grid, 256, 0, s>>>(v, b_side, mn_len, k_len, kk0, kk1, o, mn_fast);
-    B200_LAUNCH_CHECK();
-    return B200_OK;
+    auto launch = [&](auto xf) {
+      return launch_kmajor<T, decltype(xf)::value>(v, b_side, mn_len, k_len, mn_pad, kk0, kk1, o, s);
+    };
+    if (o.xform == PACK_INT8_MODULI) return launch(std::integral_constant<int, PACK_INT8_MODULI>());
+    if constexpr (sizeof(T) == 4) {
+      if (o.xform == PACK_BF16_SPLIT) return launch(std::integral_constant<int, PACK_BF16_SPLIT>());
+      if (o.xform == PACK_FP16_SPLIT) return launch(std::integral_constant<int, PACK_FP16_SPLIT>());
+    } else {
+      if (o.xform == PACK_INT8_SLICES) return launch(std::integral_constant<int, PACK_INT8_SLICES>());
+    }
   }
   const bool plain_copy = v.struc == MUBLIS_STRUC_GENERAL && v.mask_rel == MUBLIS_L3_ALL &&
                           o.xform == PACK_COPY && mn_stride > 0 && kk_stride > 0 &&

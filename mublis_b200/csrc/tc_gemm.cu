@@ -787,6 +787,32 @@ int launch_bf16(const CUtensorMap &ta, const CUtensorMap &tb, const Bf16Params &
 
 }  // namespace
 
+namespace {
+
+// Scales and packs one operand of a scaled form: the exponents of its rows
+// (columns) over the whole, concatenated k, then its planes.  amax: mn_pad
+// words of scratch.
+template <typename T>
+int scale_and_pack(const PackView (&v)[2], int npairs, bool b_side, long mn_len, long k_len,
+                   long mn_pad, long kpad, unsigned long long *amax, int *exps, const PackOut &o,
+                   cudaStream_t s) {
+  if (npairs == 1 && launch_scale_pack<T>(v[0], b_side, mn_len, k_len, mn_pad, kpad, exps, o, s)) {
+    B200_LAUNCH_CHECK();
+    return B200_OK;
+  }
+  B200_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * mn_pad, s));
+  for (int t = 0; t < npairs; ++t)
+    B200_TRY(launch_absmax<T>(v[t], b_side, mn_len, k_len, amax, s));
+  B200_TRY(launch_scale_exps(amax, exps, mn_pad, s));
+  for (int t = 0; t < npairs; ++t) {
+    const long kk0 = (long)t * k_len, kk1 = t + 1 == npairs ? kpad : kk0 + k_len;
+    B200_TRY(launch_pack<T>(v[t], b_side, mn_len, k_len, mn_pad, kk0, kk1, o, s));
+  }
+  return B200_OK;
+}
+
+}  // namespace
+
 // Packs the FP32 operands into TERMS bf16 planes (K-major, padded) and runs
 // the tcgen05 kernel.  The fp16x3 form (Ootomo and Yokota's FP16 split with
 // per-row / per-column power-of-two scaling) scales row i of op(A) by
@@ -825,27 +851,23 @@ int tc_run_bf16(const b200_l3_desc_t *d, int form) {
     vb[t] = PackView{d->b[t], d->rs_b[t], d->cs_b[t], (int)pr.b.struc, (int)pr.b.uplo,
                      (int)pr.b.diag, (int)pr.domain.jp};
   }
-  unsigned long long *am = nullptr, *bm = nullptr;
   int *ae = nullptr;
-  if (f16 && st == B200_OK) {  // scales over the whole (concatenated) k
+  if (f16 && st == B200_OK) {
     st = b200_alloc(&amax, (sizeof(unsigned long long) + sizeof(int)) * (mpad + npad));
-    am = (unsigned long long *)amax;
-    bm = am + mpad;
-    ae = (int *)(am + mpad + npad);
-    if (st == B200_OK &&
-        cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * (mpad + npad), s) != cudaSuccess)
-      st = b200_set_error(B200_ECUDA, "memset failed");
-    for (int t = 0; t < d->npairs && st == B200_OK; ++t) {
-      st = launch_absmax<float>(va[t], false, d->m, d->k, am, s);
-      if (st == B200_OK) st = launch_absmax<float>(vb[t], true, d->n, d->k, bm, s);
-    }
-    if (st == B200_OK) st = launch_scale_exps(am, ae, mpad + npad, s);
+    ae = (int *)((unsigned long long *)amax + mpad + npad);
   }
-  const int xform = f16 ? PACK_FP16_SPLIT : PACK_BF16_SPLIT;
-  for (int t = 0; t < d->npairs && st == B200_OK; ++t) {
-    long kk0 = (long)t * d->k, kk1 = t + 1 == d->npairs ? kpad : kk0 + d->k;
-    PackOut oa{ap, kpad, mpad * kpad, PACK_K_MAJOR, xform, terms, am};
-    PackOut ob{bp, kpad, npad * kpad, PACK_K_MAJOR, xform, terms, bm};
+  const PackOut oa{ap, kpad, mpad * kpad, PACK_K_MAJOR, f16 ? PACK_FP16_SPLIT : PACK_BF16_SPLIT, terms, ae};
+  const PackOut ob{bp, kpad, npad * kpad, PACK_K_MAJOR, f16 ? PACK_FP16_SPLIT : PACK_BF16_SPLIT, terms,
+                   ae ? ae + mpad : nullptr};
+  if (f16) {
+    unsigned long long *am = (unsigned long long *)amax;
+    if (st == B200_OK)
+      st = scale_and_pack<float>(va, d->npairs, false, d->m, d->k, mpad, kpad, am, ae, oa, s);
+    if (st == B200_OK)
+      st = scale_and_pack<float>(vb, d->npairs, true, d->n, d->k, npad, kpad, am + mpad, ae + mpad, ob, s);
+  }
+  for (int t = 0; t < d->npairs && !f16 && st == B200_OK; ++t) {
+    const long kk0 = (long)t * d->k, kk1 = t + 1 == d->npairs ? kpad : kk0 + d->k;
     st = launch_pack<float>(va[t], false, d->m, d->k, mpad, kk0, kk1, oa, s);
     if (st == B200_OK) st = launch_pack<float>(vb[t], true, d->n, d->k, npad, kk0, kk1, ob, s);
   }
@@ -1646,11 +1668,22 @@ int oz2_setup(int N, long k, int pmax, B200Moduli *mod, OzCrt *crt, int *pa, int
   };
   for (int l = 0; l < N; ++l) {
     const int m = OZ2_MODULI[l];
-    mod->m[l] = crt->m[l] = m;
-    mod->c19[l] = (int)((1u << 19) % (unsigned)m);
-    mod->c38[l] = (int)((((u128)1) << 38) % (u128)m);
-    mod->mg[l] = crt->mg[l] = (unsigned)(((1ull << 39) + (unsigned long long)m - 1) / m);
-    mod->bias[l] = crt->bias[l] = m / 2 + (int)(((1u << 29) + m - 1) / m) * m;
+    crt->m[l] = m;
+    crt->mg[l] = (unsigned)(((1ull << 39) + (unsigned long long)m - 1) / m);
+    crt->bias[l] = m / 2 + (int)(((1u << 29) + m - 1) / m) * m;
+    // b200_residue: 256^i mod m as signed bytes, and the offset that makes the
+    // byte sum non-negative and takes 2^56 off again.
+    unsigned bytes[2] = {0, 0}, p256 = 1, p56 = 0;
+    for (int i = 0; i < 8; ++i, p256 = p256 * 256 % (unsigned)m) {
+      const int c = (int)p256 > m / 2 ? (int)p256 - m : (int)p256;
+      bytes[i / 4] |= (unsigned)(c & 0xff) << (8 * (i % 4));
+      if (i == 7) p56 = p256;  // 256^7 = 2^56
+    }
+    mod->lo[l] = (int)bytes[0];
+    mod->hi[l] = (int)bytes[1];
+    mod->base[l] = 0x4B000000 + ((1 << 18) / m + 2) * m - (int)p56;
+    mod->inv[l] = 1.0f / (float)m;
+    mod->neg_m[l] = -(float)m;
     const u128 Ml = M / (u128)m;
     const int r = (int)(Ml % (u128)m);
     int y = 1;
@@ -1763,16 +1796,9 @@ int run_ozaki(const b200_l3_desc_t *d, bool mod) {
     grid = 2 * (tiles < clusters ? tiles : clusters);
   }
 
-  void *ap = nullptr, *bp = nullptr, *amax = nullptr, *bmax = nullptr, *work = nullptr;
+  void *ap = nullptr, *bp = nullptr, *amax = nullptr, *work = nullptr;
   int st = b200_alloc(&amax, (sizeof(unsigned long long) + sizeof(int)) * (mpad + npad));
-  int *exps = nullptr;
-  if (st == B200_OK) {
-    bmax = (unsigned long long *)amax + mpad;
-    exps = (int *)((unsigned long long *)amax + mpad + npad);
-    st = cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * (mpad + npad), s) == cudaSuccess
-             ? B200_OK
-             : b200_set_error(B200_ECUDA, "memset failed");
-  }
+  int *exps = (int *)((unsigned long long *)amax + mpad + npad);
   if (st == B200_OK) st = b200_alloc(&ap, (size_t)slices * mpad * kpad);
   if (st == B200_OK) st = b200_alloc(&bp, (size_t)slices * npad * kpad);
   const size_t work_bytes = pair ? (size_t)grid * slices * OzPairCfg::BM * OzPairCfg::TILE_N
@@ -1787,22 +1813,14 @@ int run_ozaki(const b200_l3_desc_t *d, bool mod) {
     vb[t] = PackView{d->b[t], d->rs_b[t], d->cs_b[t], (int)pr.b.struc, (int)pr.b.uplo,
                      (int)pr.b.diag, (int)pr.domain.jp};
   }
-  // Scales over the whole (concatenated) k of every row / column.
-  for (int t = 0; t < d->npairs && st == B200_OK; ++t) {
-    st = launch_absmax<T>(va[t], false, d->m, d->k, (unsigned long long *)amax, s);
-    if (st == B200_OK)
-      st = launch_absmax<T>(vb[t], true, d->n, d->k, (unsigned long long *)bmax, s);
-  }
-  if (st == B200_OK) st = launch_scale_exps((const unsigned long long *)amax, exps, mpad + npad, s);
-  for (int t = 0; t < d->npairs && st == B200_OK; ++t) {
-    long kk0 = (long)t * d->k, kk1 = t + 1 == d->npairs ? kpad : kk0 + d->k;
+  if (st == B200_OK) {
     const int xform = mod ? PACK_INT8_MODULI : PACK_INT8_SLICES;
-    PackOut oa{ap, kpad, mpad * kpad, PACK_K_MAJOR, xform, slices,
-               (const unsigned long long *)amax, pa, moduli};
-    PackOut ob{bp, kpad, npad * kpad, PACK_K_MAJOR, xform, slices,
-               (const unsigned long long *)bmax, pb, moduli};
-    st = launch_pack<T>(va[t], false, d->m, d->k, mpad, kk0, kk1, oa, s);
-    if (st == B200_OK) st = launch_pack<T>(vb[t], true, d->n, d->k, npad, kk0, kk1, ob, s);
+    const PackOut oa{ap, kpad, mpad * kpad, PACK_K_MAJOR, xform, slices, exps, pa, moduli};
+    const PackOut ob{bp, kpad, npad * kpad, PACK_K_MAJOR, xform, slices, exps + mpad, pb, moduli};
+    unsigned long long *am = (unsigned long long *)amax;
+    st = scale_and_pack<T>(va, d->npairs, false, d->m, d->k, mpad, kpad, am, exps, oa, s);
+    if (st == B200_OK)
+      st = scale_and_pack<T>(vb, d->npairs, true, d->n, d->k, npad, kpad, am + mpad, exps + mpad, ob, s);
   }
   CUtensorMap ta, tb;
   // Boxes of one CTA's share of a tile: 256 rows, or 128 on CTA pairs.

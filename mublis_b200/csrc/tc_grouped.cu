@@ -98,18 +98,6 @@ __device__ __forceinline__ int tcg_swz(int r, int ch) {
   return r * TCG_ROW + ((ch ^ ((r >> 1) & 3)) << 4);
 }
 
-// x * 2^(15 - e) for the fp16 split, as two multiplications by exact
-// powers of two: the first is the whole factor whenever 2^(15 - e) is a
-// normal float (then it is one rounding of the exact product, as ldexpf
-// gives); for rows whose maximum is below 2^-112 the factor is cut in two,
-// each scaling up exactly.
-__device__ __forceinline__ void tcg_scale_factors(int e, float &f1, float &f2) {
-  const int sh = B200_FP16_SCALE_EXP - e;
-  const int s1 = sh > 127 ? 127 : (sh < -126 ? -126 : sh);
-  f1 = __int_as_float((s1 + 127) << 23);
-  f2 = __int_as_float((sh - s1 + 127) << 23);
-}
-
 // The scale exponent of b200_scale_exp (frexp's: max|x| < 2^e, 0 for an
 // all-zero row) from the bits of a non-negative float, by integer
 // arithmetic: normal E - 126, subnormal -117 - clz(mantissa); infinity and
@@ -282,7 +270,7 @@ __global__ void __launch_bounds__(TCG_PACK_WARPS * 32, 1) tcg_pack_kernel(const 
         const int ch = it & 3, r = (it >> 2) & 31, cl = it >> 7;
         if (r >= nr) continue;
         float f1, f2;
-        tcg_scale_factors(tcg_exp_of(rmax[r]), f1, f2);
+        b200_pow2_factors(B200_FP16_SCALE_EXP - tcg_exp_of(rmax[r]), f1, f2);
         const float *src = buf + r * ld + cl * TCG_BK + ch * 8;
         __align__(16) __half2 h[4], l[4];
 #pragma unroll
