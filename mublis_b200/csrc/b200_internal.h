@@ -233,12 +233,6 @@ int b200_grouped_gemm_async(int dtype, const b200_l3_desc_t *const *descs, int c
                             void *stream);
 int b200_grouped_trsm_async(int dtype, const b200_trsm_desc_t *const *descs, int count,
                             void *stream);
-/* One plain GEMM read directly from its operands (no pack pass, no scratch),
- * on the calling thread's stream. */
-int b200_gemm_direct(const b200_l3_desc_t *d);
-/* Same, with tiles at least min_rows tall (for in-place products). */
-int b200_gemm_direct_min_rows(const b200_l3_desc_t *d, int min_rows);
-
 /* serve.cu: when a request server is attached, the host front routes calls
  * whose operands are all device-resident through it (blocking until done).
  * b200_serve_attached() is 0 when none is attached. */

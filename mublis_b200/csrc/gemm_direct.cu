@@ -24,6 +24,8 @@
 //   * Operands move in 16-byte copies where the unit stride runs along m (n)
 //     and every row starts on 16 bytes, else element by element along
 //     whichever stride is smaller; copies past the edge fill zeros.
+//   * A group of many products (grouped.cu) runs the same tiles, one CTA each,
+//     from a table of problems.
 //   * The sums go through shared memory to C, so C is read and written along
 //     its own unit stride.
 #include <algorithm>
@@ -242,8 +244,8 @@ __device__ __forceinline__ int block_class(const DirectOperand<T> &o, long mn0, 
 // PLAIN: both operands general and unmasked.  (SYR2K's two pairs are plain;
 // each pair takes whole k-blocks, the last one filled up with zeros.)
 template <typename T, int TILE, bool PLAIN>
-__global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, TILE == 32 && !PLAIN ? 3 : 4)
-    direct_gemm_kernel(const __grid_constant__ DirectArgs<T> p) {
+__device__ __forceinline__ void direct_tile(const DirectArgs<T> &p, const int tile, const int rank,
+                                            const int S) {
   using C = DirectCfg<T, TILE>;
   constexpr bool F64 = sizeof(T) == 8;
   constexpr int BM = TILE, BN = TILE, BK = C::BK, LD = C::LD, CLD = C::CLD, STAGES = C::STAGES;
@@ -251,8 +253,6 @@ __global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, TILE == 32 && !PLAIN ?
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *ring = reinterpret_cast<T *>(smem_raw);
 
-  const int S = p.splits;
-  const int tile = blockIdx.x / S, rank = blockIdx.x % S;
   const long m0 = (long)(tile % p.tiles_m) * BM, n0 = (long)(tile / p.tiles_m) * BN;
   // Outside the written triangle (l3_driver.c:145-147,165-171): the whole
   // cluster leaves.
@@ -465,6 +465,41 @@ __global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, TILE == 32 && !PLAIN ?
 }
 
 template <typename T, int TILE, bool PLAIN>
+__global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, TILE == 32 && !PLAIN ? 3 : 4)
+    direct_gemm_kernel(const __grid_constant__ DirectArgs<T> p) {
+  direct_tile<T, TILE, PLAIN>(p, blockIdx.x / p.splits, blockIdx.x % p.splits, p.splits);
+}
+
+// Many independent products: CTA b computes tile b of the group, of problem
+// tile_prob[b] of the table.
+template <typename T, int TILE>
+__global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, 4)
+    direct_group_kernel(const b200_group_gemm_t *__restrict__ table, const int *__restrict__ tile_prob) {
+  const b200_group_gemm_t &e = table[tile_prob[blockIdx.x]];
+  DirectArgs<T> p;
+  p.a.x[0] = (const T *)e.a;
+  p.a.s_mn[0] = e.rs_a;
+  p.a.s_k[0] = e.cs_a;
+  p.a.vec[0] = e.vec & 1;
+  p.b.x[0] = (const T *)e.b;
+  p.b.s_mn[0] = e.cs_b;
+  p.b.s_k[0] = e.rs_b;
+  p.b.vec[0] = e.vec >> 1;
+  p.npairs = 1;
+  p.c = (T *)e.c;
+  p.rs_c = e.rs_c;
+  p.cs_c = e.cs_c;
+  p.m = e.m;
+  p.n = e.n;
+  p.k = e.k;
+  p.tiles_m = e.tiles_m;
+  p.alpha = (T)e.alpha;
+  p.beta = (T)e.beta;
+  p.jp = p.ji = p.pi = MUBLIS_L3_ALL;
+  direct_tile<T, TILE, true>(p, blockIdx.x - e.tile0, 0, 1);
+}
+
+template <typename T, int TILE, bool PLAIN>
 int launch_tile(DirectArgs<T> &p, cudaStream_t s) {
   using C = DirectCfg<T, TILE>;
   auto kern = direct_gemm_kernel<T, TILE, PLAIN>;
@@ -548,7 +583,43 @@ int run_direct(const b200_l3_desc_t *d, const b200_direct_choice_t &ch) {
   return plain ? launch_tile<T, 32, true>(p, s) : launch_tile<T, 32, false>(p, s);
 }
 
+template <typename T, int TILE>
+int launch_group_tile(const b200_group_gemm_t *table, const int *tile_prob, int tiles, cudaStream_t s) {
+  using C = DirectCfg<T, TILE>;
+  auto kern = direct_group_kernel<T, TILE>;
+  static std::once_flag once;
+  static int conf = B200_OK;
+  B200_TRY(b200_once(once, conf, "grouped gemm: set-up failed", [&]() -> int {
+    cudaFuncAttributes fa;
+    B200_CUDA_TRY(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));  // loads it: a capture must not
+    return B200_OK;
+  }));
+  if (tiles <= 0) return B200_OK;
+  B200ProfScope prof(sizeof(T) == 4 ? "grouped_sgemm" : "grouped_dgemm", s);
+  kern<<<tiles, C::NT, C::SMEM, s>>>(table, tile_prob);
+  B200_LAUNCH_CHECK();
+  return B200_OK;
+}
+
 }  // namespace
+
+int b200_group_vec(const b200_group_gemm_t &e, int elt) {
+  auto vec = [elt](const void *x, long s_mn, long s_k) {
+    return s_mn == 1 && s_k > 0 && s_k * elt % 16 == 0 && ((uintptr_t)x & 15) == 0;
+  };
+  return (vec(e.a, e.rs_a, e.cs_a) ? 1 : 0) | (vec(e.b, e.cs_b, e.rs_b) ? 2 : 0);
+}
+
+int launch_direct_group(int dtype, int tile, const b200_group_gemm_t *table, const int *tile_prob,
+                        int tiles, cudaStream_t s) {
+  if (dtype == B200_F64)
+    return tile == 64 ? launch_group_tile<double, 64>(table, tile_prob, tiles, s)
+                      : launch_group_tile<double, 32>(table, tile_prob, tiles, s);
+  return tile == 64 ? launch_group_tile<float, 64>(table, tile_prob, tiles, s)
+                    : launch_group_tile<float, 32>(table, tile_prob, tiles, s);
+}
 
 // Which calls run here, and how: the least of the estimates below, in us, from
 // the whole call's shape (a column panel of a larger call carries the call's m

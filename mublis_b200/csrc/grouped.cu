@@ -19,190 +19,13 @@
 #include <type_traits>
 #include <vector>
 
-#include "common.cuh"
+#include "kernels.cuh"
 #include "../../include/mublis_b200.h"
 #include "tc_gemm.cuh"
 
 namespace {
 
-struct GemmEntry {
-  long m, n, k;
-  double alpha, beta;
-  const void *a;
-  long rs_a, cs_a;  // element (i, p) of op(A) at a[i*rs_a + p*cs_a]
-  const void *b;
-  long rs_b, cs_b;  // element (p, j) of op(B) at b[p*rs_b + j*cs_b]
-  void *c;
-  long rs_c, cs_c;  // element (i, j) of C at c[i*rs_c + j*cs_c]
-  int tile0;        // first global tile index of this problem
-  int tiles_m;
-};
-
-// ---- grouped GEMM kernel --------------------------------------------------------
-//
-// 256 threads as a 16 x 16 grid; each thread a TM x TN register tile, so a CTA
-// covers (16*TM) x (16*TN).  Double-buffered shared memory with register
-// prefetch of the next k-block; loads follow whichever operand stride is 1.
-
-// Copies a run of V elements from shared memory (16- or 8-byte aligned when
-// the run is that long) into registers with one vector load.
-template <typename T, int V>
-__device__ __forceinline__ void lds_run(T *dst, const T *src) {
-  if constexpr (V * sizeof(T) == 16) {
-    const uint4 x = *reinterpret_cast<const uint4 *>(src);
-    memcpy(dst, &x, 16);
-  } else if constexpr (V * sizeof(T) == 8) {
-    const uint2 x = *reinterpret_cast<const uint2 *>(src);
-    memcpy(dst, &x, 8);
-  } else {
-#pragma unroll
-    for (int v = 0; v < V; ++v) dst[v] = src[v];
-  }
-}
-
-// `table` may be null: then the single problem `one` (passed by value in the
-// launch parameters) is the whole group -- the direct path for one small GEMM,
-// with no table upload.
-template <typename T, int TM, int TN>
-__global__ void __launch_bounds__(256) grouped_gemm_kernel(const GemmEntry *__restrict__ table,
-                                                           int nprob, int total_tiles,
-                                                           const __grid_constant__ GemmEntry one) {
-  constexpr int BM = 16 * TM, BN = 16 * TN, BK = sizeof(T) == 8 ? 8 : 16;
-  constexpr int A_PER = BM * BK / 256, B_PER = BK * BN / 256;
-  __shared__ __align__(16) T As[2][BK][BM];
-  __shared__ __align__(16) T Bs[2][BK][BN];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  // Thread (tx, ty) holds rows row0 + (i % VM) + 16 VM (i / VM) and columns
-  // col0 + (j % VN) + 16 VN (j / VN): runs of up to 16 bytes, so each k step
-  // reads its A and B fragments with vector shared loads (one 16-byte load
-  // per four floats instead of four 4-byte loads).
-  constexpr int VM = TM * sizeof(T) >= 16 ? 16 / (int)sizeof(T) : TM;
-  constexpr int VN = TN * sizeof(T) >= 16 ? 16 / (int)sizeof(T) : TN;
-  const int row0 = ty * VM, col0 = tx * VN;
-
-  // The table is followed by one int per output tile: the tile's problem.
-  const int *tile_prob = table ? reinterpret_cast<const int *>(table + nprob) : nullptr;
-  for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-    const GemmEntry &e = table ? table[tile_prob[tile]] : one;
-    const int local = tile - e.tile0;
-    const long m0 = (long)(local % e.tiles_m) * BM, n0 = (long)(local / e.tiles_m) * BN;
-    const T *A = (const T *)e.a, *B = (const T *)e.b;
-    const bool a_mfast = e.rs_a <= e.cs_a;  // i contiguous in memory
-    const bool b_kfast = e.rs_b <= e.cs_b;  // p contiguous in memory
-
-    T ra[A_PER], rb[B_PER];
-    auto gload = [&](long k0) {
-#pragma unroll
-      for (int q = 0; q < A_PER; ++q) {
-        int idx = tid + 256 * q;
-        int i = a_mfast ? idx % BM : idx / BK, p = a_mfast ? idx / BM : idx % BK;
-        long gi = m0 + i, gp = k0 + p;
-        ra[q] = (gi < e.m && gp < e.k) ? A[gi * e.rs_a + gp * e.cs_a] : T(0);
-      }
-#pragma unroll
-      for (int q = 0; q < B_PER; ++q) {
-        int idx = tid + 256 * q;
-        int p = b_kfast ? idx % BK : idx / BN, j = b_kfast ? idx / BK : idx % BN;
-        long gp = k0 + p, gj = n0 + j;
-        rb[q] = (gp < e.k && gj < e.n) ? B[gp * e.rs_b + gj * e.cs_b] : T(0);
-      }
-    };
-    auto sstore = [&](int buf) {
-#pragma unroll
-      for (int q = 0; q < A_PER; ++q) {
-        int idx = tid + 256 * q;
-        int i = a_mfast ? idx % BM : idx / BK, p = a_mfast ? idx / BM : idx % BK;
-        As[buf][p][i] = ra[q];
-      }
-#pragma unroll
-      for (int q = 0; q < B_PER; ++q) {
-        int idx = tid + 256 * q;
-        int p = b_kfast ? idx % BK : idx / BN, j = b_kfast ? idx / BK : idx % BN;
-        Bs[buf][p][j] = rb[q];
-      }
-    };
-
-    // FP32 accumulates column pairs with the packed sm_100 FMA (__ffma2_rn:
-    // two correctly rounded fmaf per instruction), halving the FMA issue
-    // slots; each element's result is that of fmaf.
-    constexpr bool PAIR = sizeof(T) == 4;
-    constexpr int TNP = PAIR ? TN / 2 : TN;
-    using Acc = typename std::conditional<PAIR, float2, T>::type;
-    Acc acc[TM][TNP];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-      for (int j = 0; j < TNP; ++j) {
-        if constexpr (PAIR) acc[i][j] = make_float2(0.f, 0.f);
-        else acc[i][j] = T(0);
-      }
-
-    const int kblocks = (int)((e.k + BK - 1) / BK);
-    __syncthreads();  // previous tile's readers are done with the buffers
-    if (kblocks > 0) {
-      gload(0);
-      sstore(0);
-    }
-    __syncthreads();
-    for (int kb = 0; kb < kblocks; ++kb) {
-      const int cur = kb & 1;
-      if (kb + 1 < kblocks) gload((long)(kb + 1) * BK);
-#pragma unroll
-      for (int p = 0; p < BK; ++p) {
-        T af[TM], bf[TN];
-#pragma unroll
-        for (int g = 0; g < TM / VM; ++g) lds_run<T, VM>(af + g * VM, &As[cur][p][row0 + 16 * VM * g]);
-#pragma unroll
-        for (int g = 0; g < TN / VN; ++g) lds_run<T, VN>(bf + g * VN, &Bs[cur][p][col0 + 16 * VN * g]);
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TNP; ++j) {
-            if constexpr (PAIR)
-              acc[i][j] = __ffma2_rn(make_float2(af[i], af[i]),
-                                     make_float2(bf[2 * j], bf[2 * j + 1]), acc[i][j]);
-            else
-              acc[i][j] = fma(af[i], bf[j], acc[i][j]);
-          }
-      }
-      if (kb + 1 < kblocks) sstore(cur ^ 1);
-      __syncthreads();
-    }
-
-    // Per row, the TN loads of C are issued before its stores (one memory
-    // round trip per row rather than per element; small problems spend a
-    // large share of their time here).  The FP64 8 x 8 variant, already at
-    // 255 registers, keeps one element at a time.
-    constexpr bool ROW_BATCH = !(sizeof(T) == 8 && TM * TN >= 64);
-    const T alpha = (T)e.alpha, beta = (T)e.beta;
-    T *Cm = (T *)e.c;
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const long gi = m0 + row0 + i % VM + 16 * VM * (i / VM);
-      if (gi >= e.m) continue;
-      T cv[TN];
-      if constexpr (ROW_BATCH) {
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-          const long gj = n0 + col0 + j % VN + 16 * VN * (j / VN);
-          cv[j] = gj < e.n && beta != T(0) ? Cm[gi * e.rs_c + gj * e.cs_c] : T(0);
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const long gj = n0 + col0 + j % VN + 16 * VN * (j / VN);
-        if (gj >= e.n) continue;
-        T *cij = Cm + gi * e.rs_c + gj * e.cs_c;
-        T aij;
-        if constexpr (PAIR) aij = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
-        else aij = acc[i][j];
-        T v = alpha * aij;
-        if (beta != T(0)) v = fma(beta, ROW_BATCH ? cv[j] : *cij, v);
-        *cij = v;
-      }
-    }
-  }
-}
+using GemmEntry = b200_group_gemm_t;
 
 // ---- grouped TRSM kernel ----------------------------------------------------------
 //
@@ -299,29 +122,16 @@ __global__ void __launch_bounds__(256) grouped_trsm_kernel(const TrsmEntry *__re
 
 // ---- host side ------------------------------------------------------------------
 
-enum { TILE_32 = 0, TILE_64 = 1, TILE_128x64 = 2, TILE_128 = 3, TILE_VARIANTS = 4 };
-const int kTileBM[TILE_VARIANTS] = {32, 64, 128, 128};
-const int kTileBN[TILE_VARIANTS] = {32, 64, 64, 128};
+// Tiles of the group kernel (gemm_direct.cu).
+enum { TILE_32 = 0, TILE_64 = 1, TILE_VARIANTS = 2 };
+const int kTile[TILE_VARIANTS] = {32, 64};
 
 int sm_count() { return b200_sm_count(); }
 
 template <typename T>
-int launch_gemm_variant(int variant, const GemmEntry *dtable, int nprob, int tiles,
-                        cudaStream_t s, const GemmEntry *one = nullptr) {
-  if (tiles <= 0) return B200_OK;
-  const int grid = std::min(tiles, sm_count() * 4);
-  GemmEntry single;
-  if (one) single = *one; else memset(&single, 0, sizeof single);
-  B200ProfScope prof(one ? (sizeof(T) == 4 ? "direct_sgemm" : "direct_dgemm")
-                         : (sizeof(T) == 4 ? "grouped_sgemm" : "grouped_dgemm"), s);
-  switch (variant) {
-  case TILE_32: grouped_gemm_kernel<T, 2, 2><<<grid, 256, 0, s>>>(dtable, nprob, tiles, single); break;
-  case TILE_64: grouped_gemm_kernel<T, 4, 4><<<grid, 256, 0, s>>>(dtable, nprob, tiles, single); break;
-  case TILE_128x64: grouped_gemm_kernel<T, 8, 4><<<grid, 256, 0, s>>>(dtable, nprob, tiles, single); break;
-  default: grouped_gemm_kernel<T, 8, 8><<<grid, 256, 0, s>>>(dtable, nprob, tiles, single); break;
-  }
-  B200_LAUNCH_CHECK();
-  return B200_OK;
+int launch_gemm_variant(int variant, const GemmEntry *dtable, int nprob, int tiles, cudaStream_t s) {
+  return launch_direct_group(sizeof(T) == 8 ? B200_F64 : B200_F32, kTile[variant], dtable,
+                             (const int *)(dtable + nprob), tiles, s);
 }
 
 // Size classes the autotuner chooses a tile shape for (by max(m, n)).
@@ -348,8 +158,8 @@ std::vector<char> table_image(std::vector<GemmEntry> &es, int v, int &tiles) {
   int t = 0;
   for (auto &e : es) {
     e.tile0 = t;
-    e.tiles_m = (int)b200_ceil_div(e.m, kTileBM[v]);
-    t += e.tiles_m * (int)b200_ceil_div(e.n, kTileBN[v]);
+    e.tiles_m = (int)b200_ceil_div(e.m, kTile[v]);
+    t += e.tiles_m * (int)b200_ceil_div(e.n, kTile[v]);
   }
   tiles = t;
   const size_t head = sizeof(GemmEntry) * es.size();
@@ -406,14 +216,14 @@ int to_entries(char dtype, const mublis_b200_gemm_problem_t *p, int count,
     e.c = x.c;
     e.rs_c = 1;
     e.cs_c = x.ldc;
+    e.vec = b200_group_vec(e, dtype == 'd' ? 8 : 4);
     cls[size_class(x.m, x.n)].push_back(e);
   }
-  (void)dtype;
   return B200_OK;
 }
 
 // Default tile per class, used until the autotuner has timed the classes.
-const int kDefaultVariant[NCLASS] = {TILE_32, TILE_64, TILE_128};
+const int kDefaultVariant[NCLASS] = {TILE_32, TILE_64, TILE_64};
 
 template <typename T>
 int run_groups(GemmGroup (&g)[NCLASS], cudaStream_t s) {
@@ -500,9 +310,9 @@ int tune_load(const char *path, int *entries) {
         }
         int dt, c, b, v;
         if (sscanf(line, "gemm %d %d %d %d", &dt, &c, &b, &v) != 4) continue;
-        if (dt < 0 || dt > 1 || c < 0 || c >= NCLASS || b < 0 || b >= 32 || v < 0 ||
-            v >= TILE_VARIANTS)
-          continue;
+        // (Variants 2 and 3 of older files named larger tiles.)
+        if (dt < 0 || dt > 1 || c < 0 || c >= NCLASS || b < 0 || b >= 32 || v < 0 || v > 3) continue;
+        v = std::min(v, TILE_VARIANTS - 1);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tuned[dt][c][b] = v + 1;
         ++loaded;
@@ -635,16 +445,18 @@ int to_trsm(const mublis_b200_trsm_problem_t *p, int count, TrsmGroup &g, cudaSt
 
 template <typename T>
 int launch_trsm_group(TrsmGroup &g, cudaStream_t s) {
-  if (g.slabs == 0) return B200_OK;
-  const int grid = std::min(g.slabs, sm_count() * 4);
   const size_t smem = sizeof(T) * (TRSM_MAX_ORDER * (TRSM_SLAB + 1) + 32 * 33);
   static std::once_flag once;
   static int conf = B200_OK;
   B200_TRY(b200_once(once, conf, "grouped trsm: set-up failed", [&]() -> int {
+    cudaFuncAttributes fa;
     B200_CUDA_TRY(cudaFuncSetAttribute(grouped_trsm_kernel<T>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, grouped_trsm_kernel<T>));  // loads it: a capture must not
     return B200_OK;
   }));
+  if (g.slabs == 0) return B200_OK;
+  const int grid = std::min(g.slabs, sm_count() * 4);
   B200ProfScope prof(sizeof(T) == 4 ? "grouped_strsm" : "grouped_dtrsm", s);
   grouped_trsm_kernel<T><<<grid, 256, smem, s>>>(g.dtable, (int)g.entries.size(), g.slabs);
   B200_LAUNCH_CHECK();
@@ -688,6 +500,9 @@ int plan_gemm(mublis_b200_plan *pl, const mublis_b200_gemm_problem_t *p, int cou
   cudaStream_t s = b200_cur_stream();
   std::vector<GemmEntry> cls[NCLASS];
   B200_TRY(to_entries(pl->dtype, p, count, cls));
+  // Longest products first: a launch ends with its short ones.
+  for (auto &c : cls)
+    std::stable_sort(c.begin(), c.end(), [](const GemmEntry &x, const GemmEntry &y) { return x.k > y.k; });
   // The tuner's trials are real executions; keep every C and put it back.
   std::vector<void *> saved(count, nullptr);
   for (int q = 0; q < count; ++q) {
@@ -713,8 +528,27 @@ bool tc_grouped(char dtype) {
   return dtype == 's' && b200_get_default_form(B200_F32) == B200_FORM_FP16X3;
 }
 
+// Sets up the kernels a plan launches: a capture fails when one of its launches
+// is the process's first (loading code and taking host memory are not allowed
+// then), and a plan whose tiles come from a table, or that has no trial runs,
+// may be just that.
+int setup(mublis_b200_plan *pl) {
+  if (pl->tcg) return b200_tcg_setup();
+  if (pl->kind == 1) {
+    TrsmGroup none;
+    return pl->dtype == 'd' ? launch_trsm_group<double>(none, nullptr)
+                            : launch_trsm_group<float>(none, nullptr);
+  }
+  for (const auto &g : pl->gg)
+    if (g.tiles)
+      B200_TRY(pl->dtype == 'd' ? launch_gemm_variant<double>(g.variant, nullptr, 0, 0, nullptr)
+                                : launch_gemm_variant<float>(g.variant, nullptr, 0, 0, nullptr));
+  return B200_OK;
+}
+
 int capture(mublis_b200_plan *pl) {
   cudaStream_t s = b200_cur_stream();
+  B200_TRY(setup(pl));
   B200_TRY(b200_stream_sync());
   B200_CUDA_TRY(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   int st;
@@ -742,20 +576,12 @@ extern "C" int b200_l3_is_plain_gemm(const b200_l3_desc_t *d) {
          p.b.struc == MUBLIS_STRUC_GENERAL;
 }
 
-// Without a tuned choice: the class's default tile, stepped down to smaller
-// tiles while the group would leave more than half of the SMs without a
-// tile (a few 512 x 512 products, as TRSM's inverse doubling issues, are 16
-// tiles each at 128 x 128).
+// Without a tuned choice: the class's default tile, or the small one when the
+// group would leave more than half of the SMs without a tile.
 int fill_variant(const std::vector<GemmEntry> &es, int v) {
-  static const int smaller[TILE_VARIANTS] = {-1, TILE_32, TILE_64, TILE_128x64};
-  auto tiles = [&](int var) {
-    long t = 0;
-    for (const auto &e : es)
-      t += b200_ceil_div(e.m, kTileBM[var]) * b200_ceil_div(e.n, kTileBN[var]);
-    return t;
-  };
-  while (smaller[v] >= 0 && 2 * tiles(v) < sm_count()) v = smaller[v];
-  return v;
+  long tiles = 0;
+  for (const auto &e : es) tiles += b200_ceil_div(e.m, kTile[v]) * b200_ceil_div(e.n, kTile[v]);
+  return 2 * tiles < sm_count() ? TILE_32 : v;
 }
 
 extern "C" int b200_grouped_gemm_async(int dtype, const b200_l3_desc_t *const *descs, int count,
@@ -783,6 +609,7 @@ extern "C" int b200_grouped_gemm_async(int dtype, const b200_l3_desc_t *const *d
     e.c = d.c;
     e.rs_c = d.rs_c;
     e.cs_c = d.cs_c;
+    e.vec = b200_group_vec(e, dtype == B200_F64 ? 8 : 4);
     cls[size_class(d.m, d.n)].push_back(e);
   }
   GemmGroup g[NCLASS];
@@ -811,44 +638,6 @@ extern "C" int b200_grouped_gemm_async(int dtype, const b200_l3_desc_t *const *d
   for (auto &x : g)
     if (x.dtable) cudaFreeAsync(x.dtable, s);
   return st;
-}
-
-// One small plain GEMM without packing: the grouped kernel with the problem
-// in its launch parameters (used by the TRSM recursion for thin updates).
-extern "C" int b200_gemm_direct_min_rows(const b200_l3_desc_t *d, int min_rows);
-
-extern "C" int b200_gemm_direct(const b200_l3_desc_t *d) { return b200_gemm_direct_min_rows(d, 0); }
-
-// min_rows: smallest tile height allowed (an in-place product needs a tile
-// to cover all rows of the block it overwrites).
-extern "C" int b200_gemm_direct_min_rows(const b200_l3_desc_t *d, int min_rows) {
-  if (d->m <= 0 || d->n <= 0) return B200_OK;
-  if (!b200_l3_is_plain_gemm(d)) return b200_set_error(B200_EINVAL, "direct gemm: not plain");
-  GemmEntry e;
-  memset(&e, 0, sizeof e);
-  e.m = d->m;
-  e.n = d->n;
-  e.k = d->alpha != 0.0 ? d->k : 0;
-  e.alpha = d->alpha;
-  e.beta = d->beta;
-  e.a = d->a[0];
-  e.rs_a = d->rs_a[0];
-  e.cs_a = d->cs_a[0];
-  e.b = d->b[0];
-  e.rs_b = d->rs_b[0];
-  e.cs_b = d->cs_b[0];
-  e.c = d->c;
-  e.rs_c = d->rs_c;
-  e.cs_c = d->cs_c;
-  int v = std::max(d->m, d->n) <= 64 ? TILE_32 : (std::min(d->m, d->n) <= 128 ? TILE_64 : TILE_128);
-  while (kTileBM[v] < min_rows && v < TILE_128) ++v;
-  if (kTileBM[v] < min_rows) return b200_set_error(B200_EINVAL, "direct gemm: tile too short");
-  e.tile0 = 0;
-  e.tiles_m = (int)b200_ceil_div(e.m, kTileBM[v]);
-  const int tiles = e.tiles_m * (int)b200_ceil_div(e.n, kTileBN[v]);
-  cudaStream_t s = b200_cur_stream();
-  return d->dtype == B200_F64 ? launch_gemm_variant<double>(v, nullptr, 1, tiles, s, &e)
-                              : launch_gemm_variant<float>(v, nullptr, 1, tiles, s, &e);
 }
 
 extern "C" int b200_grouped_trsm_async(int dtype, const b200_trsm_desc_t *const *descs, int count,

@@ -348,6 +348,24 @@ b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d);
 // On the calling thread's stream; C must overlap no operand.
 int launch_direct_gemm(const b200_l3_desc_t *d, const b200_direct_choice_t &ch);
 
+// One problem of a group on the device: op(A) element (i, p) at a[i rs_a + p
+// cs_a], op(B) (p, j) at b[p rs_b + j cs_b], C (i, j) at c[i rs_c + j cs_c].
+struct b200_group_gemm_t {
+  const void *a, *b;
+  void *c;
+  long rs_a, cs_a, rs_b, cs_b, rs_c, cs_c;
+  double alpha, beta;
+  int m, n, k;
+  int tile0, tiles_m;  // the problem's first tile in the group, tiles along m
+  int vec;             // b200_group_vec
+};
+// Operands that move in 16-byte copies: 1 op(A), 2 op(B).
+int b200_group_vec(const b200_group_gemm_t &e, int elt);
+// tile: 32 or 64; tile_prob: the problem of each of the `tiles` tiles (0: sets
+// the kernel up only, as a stream capture of the launch needs).
+int launch_direct_group(int dtype, int tile, const b200_group_gemm_t *table, const int *tile_prob,
+                        int tiles, cudaStream_t s);
+
 template <typename T>
 int launch_scale(int m, int n, T beta, T *c, long rs, long cs, int ji, cudaStream_t s);
 

@@ -16,6 +16,7 @@ int tc_run_ozaki(const b200_l3_desc_t *d);
 struct b200_tcg;
 int b200_tcg_create(const mublis_b200_gemm_problem_t *p, int count, b200_tcg **out);
 int b200_tcg_run(b200_tcg *g, cudaStream_t s);
+int b200_tcg_setup();  // before a capture of b200_tcg_run
 void b200_tcg_destroy(b200_tcg *g);
 
 #include <string>

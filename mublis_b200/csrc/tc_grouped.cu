@@ -698,7 +698,9 @@ int b200_tcg_create(const mublis_b200_gemm_problem_t *p, int count, b200_tcg **o
   return B200_OK;
 }
 
-int b200_tcg_run(b200_tcg *g, cudaStream_t s) {
+// Everything the launches need beforehand (kernel attributes and code, the error
+// word's host memory): what a stream capture would not survive.
+int b200_tcg_setup() {
   static std::once_flag once;
   static int conf = B200_OK;
   B200_TRY(b200_once(once, conf, "grouped fp16x3 kernels: set-up failed", []() -> int {
@@ -714,8 +716,15 @@ int b200_tcg_run(b200_tcg *g, cudaStream_t s) {
     if (fa.numRegs < TCG_PRODUCER_REGS ||
         128L * (fa.numRegs - TCG_PRODUCER_REGS) < 256L * (TCG_EPILOGUE_REGS - fa.numRegs))
       return b200_set_error(B200_EINVAL, "grouped fp16x3 kernel: register split does not fit");
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, tcg_pack_kernel));
+    b200_device_error_word();
     return B200_OK;
   }));
+  return B200_OK;
+}
+
+int b200_tcg_run(b200_tcg *g, cudaStream_t s) {
+  B200_TRY(b200_tcg_setup());
   if (g->ntasks > 0) {
     const int ks = std::min(g->kpad_max, TCG_PACK_KS);
     const size_t smem = sizeof(float) * TCG_PACK_NBUF * 32 * (ks + 1);
