@@ -27,98 +27,9 @@ namespace {
 
 using GemmEntry = b200_group_gemm_t;
 
-// ---- grouped TRSM kernel ----------------------------------------------------------
-//
-// One CTA per (problem, 32-column slab of B): the slab (order <= 256 rows)
-// lives in shared memory; the diagonal is walked in 32-row blocks: warp 0
-// solves the block (reciprocal diagonal, multiplied), then all 8 warps
-// update the rows below (lower) or above (upper) with the solved block.
-
-struct TrsmEntry {
-  long m, n;           // order and right-hand-side count
-  double alpha;
-  const void *a;
-  long rs_a, cs_a;     // op(A) element (i, p) at a[i*rs_a + p*cs_a]
-  void *b;
-  long rs_b, cs_b;     // element (i, j) of B at b[i*rs_b + j*cs_b]
-  int lower, unit;
-  int slab0;           // first global slab index
-};
-
-constexpr int TRSM_MAX_ORDER = 256;
-constexpr int TRSM_SLAB = 32;
-
-template <typename T>
-__global__ void __launch_bounds__(256) grouped_trsm_kernel(const TrsmEntry *__restrict__ table,
-                                                           int nprob, int total_slabs) {
-  extern __shared__ __align__(16) unsigned char trsm_smem[];
-  T(*X)[TRSM_SLAB + 1] = reinterpret_cast<T(*)[TRSM_SLAB + 1]>(trsm_smem);
-  T(*L)[33] = reinterpret_cast<T(*)[33]>(trsm_smem + sizeof(T) * TRSM_MAX_ORDER * (TRSM_SLAB + 1));
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // The table is followed by one int per slab: the slab's problem.
-  const int *slab_prob = reinterpret_cast<const int *>(table + nprob);
-  for (int slab = blockIdx.x; slab < total_slabs; slab += gridDim.x) {
-    const TrsmEntry &e = table[slab_prob[slab]];
-    const long j0 = (long)(slab - e.slab0) * TRSM_SLAB;
-    const int ncol = (int)min((long)TRSM_SLAB, e.n - j0);
-    const int m = (int)e.m;
-    const T *A = (const T *)e.a;
-    T *Bm = (T *)e.b;
-    const T alpha = (T)e.alpha;
-    __syncthreads();
-    for (int idx = tid; idx < m * TRSM_SLAB; idx += 256) {
-      int i = idx % m, j = idx / m;
-      X[i][j] = j < ncol ? alpha * Bm[i * e.rs_b + (j0 + j) * e.cs_b] : T(0);
-    }
-    __syncthreads();
-    const int nblk = (m + 31) / 32;
-    for (int q = 0; q < nblk; ++q) {
-      const int b = e.lower ? q : nblk - 1 - q;
-      const int r0 = b * 32, rb = min(32, m - r0);
-      // diagonal block with reciprocal diagonal; the unstored triangle and a
-      // unit diagonal are never read
-      for (int idx = tid; idx < 32 * 32; idx += 256) {
-        int i = idx % 32, p = idx / 32;
-        T v = T(0);
-        if (i < rb && p < rb) {
-          if (i == p) v = e.unit ? T(1) : T(1) / A[(r0 + i) * e.rs_a + (r0 + i) * e.cs_a];
-          else if (e.lower ? p < i : p > i) v = A[(r0 + i) * e.rs_a + (r0 + p) * e.cs_a];
-        }
-        L[i][p] = v;
-      }
-      __syncthreads();
-      if (warp == 0) {  // lane = column of the slab
-        if (e.lower) {
-          for (int i = 0; i < rb; ++i) {
-            T r = X[r0 + i][lane];
-            for (int p = 0; p < i; ++p) r = fma(-L[i][p], X[r0 + p][lane], r);
-            X[r0 + i][lane] = r * L[i][i];
-          }
-        } else {
-          for (int i = rb - 1; i >= 0; --i) {
-            T r = X[r0 + i][lane];
-            for (int p = i + 1; p < rb; ++p) r = fma(-L[i][p], X[r0 + p][lane], r);
-            X[r0 + i][lane] = r * L[i][i];
-          }
-        }
-      }
-      __syncthreads();
-      // rows still to solve: below the block (lower) or above it (upper)
-      const int u0 = e.lower ? r0 + rb : 0, u1 = e.lower ? m : r0;
-      for (int idx = tid; idx < (u1 - u0) * TRSM_SLAB; idx += 256) {
-        int i = u0 + idx / TRSM_SLAB, j = idx % TRSM_SLAB;
-        T s = X[i][j];
-        for (int p = 0; p < rb; ++p) s = fma(-A[i * e.rs_a + (r0 + p) * e.cs_a], X[r0 + p][j], s);
-        X[i][j] = s;
-      }
-      __syncthreads();
-    }
-    for (int idx = tid; idx < m * TRSM_SLAB; idx += 256) {
-      int i = idx % m, j = idx / m;
-      if (j < ncol) Bm[i * e.rs_b + (j0 + j) * e.cs_b] = X[i][j];
-    }
-  }
-}
+using TrsmEntry = b200_small_trsm_t;
+constexpr int TRSM_MAX_ORDER = B200_TRSM_SMALL;
+constexpr int TRSM_SLAB = B200_TRSM_SMALL_COLS;
 
 // ---- host side ------------------------------------------------------------------
 
@@ -402,8 +313,19 @@ std::vector<char> trsm_table_image(const TrsmGroup &g) {
   return img;
 }
 
+// The group's entries by order (up to B200_TRSM_SMALL_HALF first: two launches),
+// and their slabs.
+void order_slabs(TrsmGroup &g) {
+  std::stable_partition(g.entries.begin(), g.entries.end(),
+                        [](const TrsmEntry &e) { return e.m <= B200_TRSM_SMALL_HALF; });
+  g.slabs = 0;
+  for (auto &e : g.entries) {
+    e.slab0 = g.slabs;
+    g.slabs += (int)b200_ceil_div(e.n, TRSM_SLAB);
+  }
+}
+
 int to_trsm(const mublis_b200_trsm_problem_t *p, int count, TrsmGroup &g, cudaStream_t s) {
-  int slabs = 0;
   for (int q = 0; q < count; ++q) {
     const mublis_b200_trsm_problem_t &x = p[q];
     if (x.m < 0 || x.n < 0) return b200_set_error(B200_EINVAL, "grouped trsm: negative size");
@@ -431,11 +353,9 @@ int to_trsm(const mublis_b200_trsm_problem_t *p, int count, TrsmGroup &g, cudaSt
     e.b = x.b;
     e.rs_b = 1;
     e.cs_b = x.ldb;
-    e.slab0 = slabs;
-    slabs += (int)b200_ceil_div(x.n, TRSM_SLAB);
     g.entries.push_back(e);
   }
-  g.slabs = slabs;
+  order_slabs(g);
   if (g.entries.empty()) return B200_OK;
   const std::vector<char> img = trsm_table_image(g);
   B200_TRY(b200_alloc((void **)&g.dtable, img.size()));
@@ -443,23 +363,17 @@ int to_trsm(const mublis_b200_trsm_problem_t *p, int count, TrsmGroup &g, cudaSt
   return B200_OK;
 }
 
-template <typename T>
-int launch_trsm_group(TrsmGroup &g, cudaStream_t s) {
-  const size_t smem = sizeof(T) * (TRSM_MAX_ORDER * (TRSM_SLAB + 1) + 32 * 33);
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "grouped trsm: set-up failed", [&]() -> int {
-    cudaFuncAttributes fa;
-    B200_CUDA_TRY(cudaFuncSetAttribute(grouped_trsm_kernel<T>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, grouped_trsm_kernel<T>));  // loads it: a capture must not
-    return B200_OK;
-  }));
-  if (g.slabs == 0) return B200_OK;
-  const int grid = std::min(g.slabs, sm_count() * 4);
-  B200ProfScope prof(sizeof(T) == 4 ? "grouped_strsm" : "grouped_dtrsm", s);
-  grouped_trsm_kernel<T><<<grid, 256, smem, s>>>(g.dtable, (int)g.entries.size(), g.slabs);
-  B200_LAUNCH_CHECK();
+int launch_trsm_group(int dtype, const TrsmGroup &g, cudaStream_t s) {
+  int order[2] = {0, 0}, slabs[2] = {0, 0};
+  for (const auto &e : g.entries) {
+    const int big = e.m > B200_TRSM_SMALL_HALF;
+    order[big] = std::max(order[big], e.m);
+    slabs[big] += (int)b200_ceil_div(e.n, TRSM_SLAB);
+  }
+  const int *slab_prob = (const int *)(g.dtable + g.entries.size());
+  for (int big = 0; big < 2; ++big)
+    if (slabs[big])
+      B200_TRY(launch_small_trsm(dtype, g.dtable, slab_prob, big ? slabs[0] : 0, slabs[big], order[big], s));
   return B200_OK;
 }
 
@@ -535,9 +449,9 @@ bool tc_grouped(char dtype) {
 int setup(mublis_b200_plan *pl) {
   if (pl->tcg) return b200_tcg_setup();
   if (pl->kind == 1) {
-    TrsmGroup none;
-    return pl->dtype == 'd' ? launch_trsm_group<double>(none, nullptr)
-                            : launch_trsm_group<float>(none, nullptr);
+    const int dt = pl->dtype == 'd' ? B200_F64 : B200_F32;
+    B200_TRY(launch_small_trsm(dt, nullptr, nullptr, 0, 0, 1, nullptr));
+    return launch_small_trsm(dt, nullptr, nullptr, 0, 0, B200_TRSM_SMALL, nullptr);
   }
   for (const auto &g : pl->gg)
     if (g.tiles)
@@ -557,7 +471,7 @@ int capture(mublis_b200_plan *pl) {
   else if (pl->kind == 0)
     st = pl->dtype == 'd' ? run_groups<double>(pl->gg, s) : run_groups<float>(pl->gg, s);
   else
-    st = pl->dtype == 'd' ? launch_trsm_group<double>(pl->tg, s) : launch_trsm_group<float>(pl->tg, s);
+    st = launch_trsm_group(pl->dtype == 'd' ? B200_F64 : B200_F32, pl->tg, s);
   cudaError_t e = cudaStreamEndCapture(s, &pl->graph);
   if (st != B200_OK) return st;
   B200_CUDA_TRY(e);
@@ -644,7 +558,6 @@ extern "C" int b200_grouped_trsm_async(int dtype, const b200_trsm_desc_t *const 
                                        void *stream) {
   cudaStream_t s = (cudaStream_t)stream;
   TrsmGroup g;
-  int slabs = 0;
   for (int q = 0; q < count; ++q) {
     const b200_trsm_desc_t &d = *descs[q];
     if (d.m <= 0 || d.n <= 0) continue;
@@ -663,17 +576,15 @@ extern "C" int b200_grouped_trsm_async(int dtype, const b200_trsm_desc_t *const 
     e.b = d.b;
     e.rs_b = d.rs_b;
     e.cs_b = d.cs_b;
-    e.slab0 = slabs;
-    slabs += (int)b200_ceil_div(d.n, TRSM_SLAB);
     g.entries.push_back(e);
   }
-  g.slabs = slabs;
+  order_slabs(g);
   if (g.entries.empty()) return B200_OK;
   const std::vector<char> img = trsm_table_image(g);
   if (cudaMallocAsync((void **)&g.dtable, img.size(), s) != cudaSuccess ||
       cudaMemcpyAsync(g.dtable, img.data(), img.size(), cudaMemcpyHostToDevice, s) != cudaSuccess)
     return b200_set_error(B200_ECUDA, "grouped: table upload failed");
-  int st = dtype == B200_F64 ? launch_trsm_group<double>(g, s) : launch_trsm_group<float>(g, s);
+  int st = launch_trsm_group(dtype, g, s);
   cudaFreeAsync(g.dtable, s);
   return st;
 }
@@ -721,7 +632,7 @@ int mublis_b200_trsm_grouped(char dtype, const mublis_b200_trsm_problem_t *probl
   cudaStream_t s = b200_cur_stream();
   TrsmGroup g;
   int st = to_trsm(problems, count, g, s);
-  if (st == B200_OK) st = dtype == 'd' ? launch_trsm_group<double>(g, s) : launch_trsm_group<float>(g, s);
+  if (st == B200_OK) st = launch_trsm_group(dtype == 'd' ? B200_F64 : B200_F32, g, s);
   if (st == B200_OK) st = b200_stream_sync();
   b200_free(g.dtable);
   if (st == B200_OK) st = b200_stream_sync();

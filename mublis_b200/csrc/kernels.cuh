@@ -366,6 +366,29 @@ int b200_group_vec(const b200_group_gemm_t &e, int elt);
 int launch_direct_group(int dtype, int tile, const b200_group_gemm_t *table, const int *tile_prob,
                         int tiles, cudaStream_t s);
 
+// ---- small triangular solves (trsm_small.cu)
+
+constexpr int B200_TRSM_SMALL = 256;      // largest order
+constexpr int B200_TRSM_SMALL_COLS = 32;  // right-hand sides per CTA (slab)
+// op(A) X = alpha B, X over B: op(A) element (i, p) at a[i rs_a + p cs_a], B
+// (i, j) at b[i rs_b + j cs_b].
+struct b200_small_trsm_t {
+  const void *a;
+  void *b;
+  long rs_a, cs_a, rs_b, cs_b;
+  double alpha;
+  long n;
+  int m, lower, unit;
+  int slab0;  // the problem's first slab in the group
+};
+// Orders up to this one run on half the warps (a group's are best launched apart).
+constexpr int B200_TRSM_SMALL_HALF = 128;
+// A group's slabs first_slab ..: slab_prob names the problem of each (0 slabs:
+// sets the kernel up only, as a stream capture of the launch needs).
+int launch_small_trsm(int dtype, const b200_small_trsm_t *table, const int *slab_prob, int first_slab,
+                      int slabs, int max_order, cudaStream_t s);
+int launch_small_trsm_one(int dtype, const b200_small_trsm_t &e, cudaStream_t s);
+
 template <typename T>
 int launch_scale(int m, int n, T beta, T *c, long rs, long cs, int ji, cudaStream_t s);
 

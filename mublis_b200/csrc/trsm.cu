@@ -75,6 +75,16 @@ bool fused_leaves(int dtype) {
   return forced >= 0 ? forced == 1 : dtype == B200_F64;
 }
 
+// Orders that one launch solves (trsm_small.cu); MUBLIS_B200_TRSM=fused /
+// inverse keeps the leaf methods for them too.
+bool small_solve(long m) {
+  static const bool on = [] {
+    const char *e = getenv("MUBLIS_B200_TRSM");
+    return !(e && (!strcmp(e, "inverse") || !strcmp(e, "fused")));
+  }();
+  return on && m <= B200_TRSM_SMALL;
+}
+
 // One CTA per LEAF block: thread j computes column j of the inverse of the
 // block's (lower or upper) triangle by substitution, L x = e_j.  Rows past
 // the matrix order are padded with the identity.  Output: big block
@@ -431,6 +441,7 @@ extern "C" int b200_trsm_prepare(const b200_trsm_desc_t *d, void **prep) {
   if (d->m <= 0) return B200_OK;
   if (d->uplo != MUBLIS_LOWER && d->uplo != MUBLIS_UPPER)
     return b200_set_error(B200_EINVAL, "trsm: uplo must be lower or upper");
+  if (small_solve(d->m)) return B200_OK;  // nothing to prepare
   TrsmPrep *p = new TrsmPrep{nullptr, 0, nullptr};
   const int st = d->dtype == B200_F32 ? build_inverse<float>(d, p) : build_inverse<double>(d, p);
   if (st != B200_OK) {
@@ -453,6 +464,21 @@ extern "C" int b200_trsm_run(const b200_trsm_desc_t *d) {
   if (d->m <= 0 || d->n <= 0) return B200_OK;
   if (d->uplo != MUBLIS_LOWER && d->uplo != MUBLIS_UPPER)
     return b200_set_error(B200_EINVAL, "trsm: uplo must be lower or upper");
+  if (small_solve(d->m)) {
+    b200_small_trsm_t e = {};
+    e.a = d->a;
+    e.b = d->b;
+    e.rs_a = d->rs_a;
+    e.cs_a = d->cs_a;
+    e.rs_b = d->rs_b;
+    e.cs_b = d->cs_b;
+    e.alpha = d->alpha;
+    e.n = d->n;
+    e.m = d->m;
+    e.lower = d->uplo == MUBLIS_LOWER;
+    e.unit = d->unit_diag != 0;
+    return launch_small_trsm_one(d->dtype, e, b200_cur_stream());
+  }
   if (d->alpha != 1.0)
     B200_TRY(b200_scale_strided(d->dtype, d->m, d->n, d->alpha, d->b, d->rs_b, d->cs_b,
                                 MUBLIS_L3_ALL));
