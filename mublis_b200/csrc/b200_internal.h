@@ -111,7 +111,7 @@ long b200_trsm_leaf_stride(void);
 int b200_trsm_leaf_pack(int dtype, const void *a, long rs_a, long cs_a, int m, int lower,
                         int unit, void *out);
 int b200_trsm_leaf_solve(int dtype, const void *pack, int rows, void *b, long rs_b, long cs_b,
-                         int n);
+                         int n, double alpha);
 
 /* runtime.cu */
 int b200_init(void);

@@ -8,11 +8,12 @@
 //   * recursive halving: solve the top half, update the bottom half with one
 //     GEMM (k = half the order, so it runs at GEMM speed), solve the bottom
 //     half (upper: mirror image);
-//   * FP64 leaves (512 rows) are solved by the fused GEMMTRSM kernel
+//   * leaves (512 rows) are solved by the fused GEMMTRSM kernel
 //     (trsm_leaf.cu): diagonal 16 x 16 blocks in shared memory, the updates
-//     between them on the FP64 tensor pipe, every right-hand side of the
-//     chain in one launch;
-//   * FP32 leaves are the 512 x 512 (1024 x 1024 for large solves) diagonal
+//     between them on the FP64 tensor pipe or the FMA units, every right-hand
+//     side of the chain in one launch;
+//   * FP32 solves that are large, or long with few right-hand sides
+//     (fused_leaves), take as leaves the 512 x 512 (1024 x 1024) diagonal
 //     blocks, inverted up front: one launch inverts every 64 x 64 diagonal
 //     block by substitution against the reciprocal diagonal (computed once
 //     and multiplied -- never divided -- as the reference does), then
@@ -26,8 +27,8 @@
 //     at least 128 output tiles of 128 x 128 for 148 SMs (256-row leaves
 //     gave 64);
 //   * the unit diagonal and the unstored triangle are never read.
-// alpha is applied once up front (the reference's alpha_eff on the first
-// block, trsm.c:96-97).
+// alpha goes into the first product or solve that touches a row (a pass of its
+// own over B took 2-3%: DTRSM 1000 x 1000 233 -> 226 us, 4096 x 4096 2776 -> 2722).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -58,21 +59,27 @@ int leaf_order(long m, long n) {
   return m >= 4096 && n >= 2048 ? 1024 : 512;
 }
 
-// Leaves: FP64 solves use the fused leaf kernel (trsm_leaf.cu), FP32 solves
-// the inverted diagonal blocks applied as products; MUBLIS_B200_TRSM=fused /
-// inverse selects one for both.  Measured at n = 4096 (device operands):
-// DTRSM 22.4 TF/s fused vs 20.3 inverse (the leaf's updates run on the FP64
-// tensor pipe, and it executes the triangle's flops only, not the 1.25 to 2x
-// of a product with the inverse); STRSM 31.0 fused vs 33.3 inverse (FP32 has
-// no tensor-pipe form, and the inverse products run at the SIMT GEMM's rate).
-bool fused_leaves(int dtype) {
+// Leaves: the fused leaf kernel (trsm_leaf.cu), or the inverted diagonal blocks
+// applied as products; MUBLIS_B200_TRSM=fused / inverse selects one for all.
+// FP64 always takes the kernel (its updates run on the FP64 tensor pipe, and it
+// executes the triangle's flops only, not the 1.25 to 2x of a product with the
+// inverse).  FP32 (us, kernel / inverse): 500 x 300 92 / 153, 1001 x 1500
+// 184 / 271, 2048 x 500 321 / 341, 3000 x 1000 605 / 663, 3500 x 3500 1304 / 1557,
+// 6000 x 2500 2389 / 2453; but 4096 x 3000 1452 / 1437, 4096 x 4096 1798 / 1752,
+// 8192 x 8192 10141 / 9498, where the products are large enough for the GEMM's
+// rate, and 3000 x 200 451 / 395, 4096 x 300 667 / 569, 8000 x 500 1737 / 1560,
+// where a leaf is latency and all of the inverses are built at once.  n is the
+// whole call's, so that every panel of a solve takes the same leaves.
+bool fused_leaves(int dtype, long m, long n) {
   static const int forced = [] {
     const char *e = getenv("MUBLIS_B200_TRSM");
     if (e && !strcmp(e, "inverse")) return 0;
     if (e && !strcmp(e, "fused")) return 1;
     return -1;
   }();
-  return forced >= 0 ? forced == 1 : dtype == B200_F64;
+  if (forced >= 0) return forced == 1;
+  if (dtype == B200_F64) return true;
+  return n <= 512 ? m <= 2048 : m < 4096 || n < 3000;
 }
 
 // Orders that one launch solves (trsm_small.cu); MUBLIS_B200_TRSM=fused /
@@ -244,17 +251,19 @@ int for_each_chain(const Chains &ch, Build build) {
   return B200_OK;
 }
 
-// Inverted diagonal blocks of one triangle (FP32: the leaves of the solve,
-// applied as products), or (FP64) the packed leaves of the fused
-// GEMMTRSM kernel (trsm_leaf.cu).
+// Inverted diagonal blocks of one triangle (the leaves of the solve, applied as
+// products), or the packed leaves of the fused GEMMTRSM kernel (trsm_leaf.cu).
 struct TrsmPrep {
   void *inv;
   long big;
   void *leaf;
 };
 
+// Rows [r0, r1) of op(A) X = alpha B.  alpha goes into whatever touches a row
+// first: the leaf's solve or the update's beta (the reference's alpha_eff on
+// the first block, trsm.c:96-97).
 template <typename T>
-int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1) {
+int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1, double alpha) {
   const b200_trsm_desc_t &d0 = *ch.d[0];
   const bool lower = d0.uplo == MUBLIS_LOWER;
   const T *inv = (const T *)prep->inv;
@@ -271,7 +280,7 @@ int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1) {
       T *first = lower ? b + r0 * d.rs_b : b + (r1 - 1) * d.rs_b;
       void *prev = b200_override_stream((void *)ch.streams[c]);
       const int st = b200_trsm_leaf_solve(d.dtype, pack, (int)rows, first,
-                                          lower ? d.rs_b : -d.rs_b, d.cs_b, d.n);
+                                          lower ? d.rs_b : -d.rs_b, d.cs_b, d.n, alpha);
       b200_override_stream(prev);
       B200_TRY(st);
     }
@@ -296,7 +305,7 @@ int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1) {
       g.m = (int)rows;
       g.n = d.n;
       g.k = (int)rows;
-      g.alpha = 1.0;
+      g.alpha = alpha;
       g.beta = 0.0;
       g.a[0] = inv + (r0 / big) * big * big;
       g.rs_a[0] = 1;
@@ -315,7 +324,7 @@ int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1) {
   // Rows solved first (src) and rows updated by them (dst).
   long s0 = lower ? r0 : mid, s1 = lower ? mid : r1;
   long t0 = lower ? mid : r0, t1 = lower ? r1 : mid;
-  B200_TRY(trsm_rec<T>(ch, prep, s0, s1));
+  B200_TRY(trsm_rec<T>(ch, prep, s0, s1, alpha));
   B200_TRY(for_each_chain(ch, [&](const b200_trsm_desc_t &d) {
     const T *a = (const T *)d.a;
     T *b = (T *)d.b;
@@ -325,7 +334,7 @@ int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1) {
     g.n = d.n;
     g.k = (int)(s1 - s0);
     g.alpha = -1.0;
-    g.beta = 1.0;
+    g.beta = alpha;
     g.a[0] = a + t0 * d.rs_a + s0 * d.cs_a;
     g.rs_a[0] = d.rs_a;
     g.cs_a[0] = d.cs_a;
@@ -337,7 +346,7 @@ int trsm_rec(const Chains &ch, const TrsmPrep *prep, long r0, long r1) {
     g.cs_c = d.cs_b;
     return g;
   }));
-  return trsm_rec<T>(ch, prep, t0, t1);
+  return trsm_rec<T>(ch, prep, t0, t1, 1.0);
 }
 
 // Pack every leaf of op(A) for the fused kernel (reciprocal diagonal; FP64
@@ -361,10 +370,11 @@ int build_leaves(const b200_trsm_desc_t *d, TrsmPrep *p) {
 
 template <typename T>
 int build_inverse(const b200_trsm_desc_t *d, TrsmPrep *p) {
-  if (fused_leaves(d->dtype)) return build_leaves(d, p);
+  const long n = d->policy_n > 0 ? d->policy_n : d->n;
+  if (fused_leaves(d->dtype, d->m, n)) return build_leaves(d, p);
   cudaStream_t s = b200_cur_stream();
   T *inv = nullptr, *tmp = nullptr;
-  const long big = leaf_order(d->m, d->policy_n > 0 ? d->policy_n : d->n);
+  const long big = leaf_order(d->m, n);
   const long bigs = b200_ceil_div(d->m, big);
   B200_TRY(b200_alloc((void **)&inv, sizeof(T) * bigs * big * big));
   int st = b200_alloc((void **)&tmp, sizeof(T) * bigs * big * big / 2);
@@ -415,7 +425,7 @@ int trsm_solve(const b200_trsm_desc_t *d) {
         st = b200_set_error(B200_ECUDA, "trsm: stream fork failed");
       if (st == B200_OK) {
         const Chains ch = {{&h0, &h1}, {s, s2}, 2};
-        st = trsm_rec<T>(ch, prep, 0, d->m);
+        st = trsm_rec<T>(ch, prep, 0, d->m, d->alpha);
       }
       // Join even after a failure, so nothing of the second chain is left
       // running on the scratch freed below.
@@ -426,7 +436,7 @@ int trsm_solve(const b200_trsm_desc_t *d) {
       if (e1) cudaEventDestroy(e1);
     } else {
       const Chains ch = {{d, nullptr}, {s, nullptr}, 1};
-      st = trsm_rec<T>(ch, prep, 0, d->m);
+      st = trsm_rec<T>(ch, prep, 0, d->m, d->alpha);
     }
   }
   b200_free(own.inv);
@@ -479,9 +489,6 @@ extern "C" int b200_trsm_run(const b200_trsm_desc_t *d) {
     e.unit = d->unit_diag != 0;
     return launch_small_trsm_one(d->dtype, e, b200_cur_stream());
   }
-  if (d->alpha != 1.0)
-    B200_TRY(b200_scale_strided(d->dtype, d->m, d->n, d->alpha, d->b, d->rs_b, d->cs_b,
-                                MUBLIS_L3_ALL));
   if (d->dtype == B200_F32) return trsm_solve<float>(d);
   return trsm_solve<double>(d);
 }

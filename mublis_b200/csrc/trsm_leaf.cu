@@ -7,26 +7,34 @@
 // gemmtrsm{l,u} micro-kernel (include/mublis_instantiate.h:95-114,
 // targets/avx2/gemmtrsm_ukr.inc:95-215), which forms B11 - A1x * Bx1 and
 // solves the MR x MR diagonal block A11 (packed with its diagonal already
-// inverted, packm.c:143-144) in registers.  Here one CTA owns 32
-// right-hand-side columns of a leaf of 512 rows and keeps the whole 512 x 32
-// block of B in registers (8 warps, each 4 row blocks of 16 rows, assigned
-// cyclically so that every warp keeps working as the solve moves down).  For
-// each diagonal block d of 16 rows:
-//   * the warp that owns block d + 1 first applies block d's update to it,
-//     then solves it in shared memory, X = inv(D) R with the inverse of its
-//     16 x 16 diagonal block -- so the next block is ready by the time the
-//     other warps finish their updates (look-ahead);
-//   * every other warp applies X_d to its blocks below: B_rb -= A_rb,d X_d,
-//     16 x 32 x 16 per block as m16n8k4 .f64 MMAs on the tensor pipe;
-//   * all threads write X_d to B (off the owner's critical path).
-// One barrier per block.  The leaf's A is packed once per solve
-// (trsm_leaf_pack_kernel) into one contiguous segment per step -- the
-// column of 16 x 16 blocks below the diagonal block in MMA fragment order,
-// then the inverse of the next diagonal block, formed by substitution
-// against the reciprocal diagonal (the reference's inverted-diagonal
+// inverted, packm.c:143-144) in registers.  Here a CTA owns 8 or 16 columns (FP32:
+// 32) of a leaf of 512 rows and keeps that whole block of B in registers.  A
+// column group (8 columns of FP64, 32 of FP32) has 4 or 8 of the 8 warps, and its
+// 32 row blocks of 16 go to them in turn.  For each diagonal block d of 16 rows:
+//   * the warp that owns block d + 1 first applies block d's update to it and
+//     solves it, X = inv(D) R with the inverse of its 16 x 16 diagonal block, and
+//     publishes it in shared memory on an mbarrier, so that the other warps find
+//     it when their updates are done (look-ahead);
+//   * every warp then applies X_d to its own blocks below: B_rb -= A_rb,d X_d, as
+//     m16n8k4 .f64 MMAs on the tensor pipe, or FP32 FMAs on 4 x 4 register tiles.
+// Nothing but these mbarriers and the ring's holds the warps together: there is no
+// barrier of the CTA in the loop.  What bounds it is the chain from X_d to X_{d+1}
+// (an update and a solve of one block, 1100-1400 clocks of 32 dependent steps;
+// folding inv(D) into the update, so that the chain is one product, measured 2-5%
+// slower and cost FP32 half a digit), then the FP64 pipe (a step's MMAs take half of
+// it at 16 columns).  A CTA of 32 columns whose 8 warps each updated 16 x 32
+// blocks, with a barrier per step, took 78 us a leaf in FP64 and 82 us in FP32
+// (its FMAs took an A operand from shared memory for every two of them); now 28 us
+// (8 columns) or 43 us (16), and 52 us.  DTRSM 1000 x 1000 225 -> 123 us, 4096 x
+// 4096 2726 -> 2580; STRSM 1001 x 1500 231 -> 184.
+//
+// The leaf's A is packed once per solve (trsm_leaf_pack_kernel) into one contiguous
+// segment per step -- the column of 16 x 16 blocks below the diagonal block (FP64 in
+// MMA fragment order), then the inverse of the next diagonal block, formed by
+// substitution against the reciprocal diagonal (the reference's inverted-diagonal
 // packing, packm.c:143-144, carried to the whole 16 x 16 block) -- and one
-// thread streams segments into a 3-deep shared-memory ring with 1-D bulk
-// copies (TMA), two steps ahead.  Every wait is bounded (tc_common.cuh); a
+// thread of a warpgroup of its own streams segments into a 3-deep shared-memory ring
+// with 1-D bulk copies (TMA).  Every wait is bounded (tc_common.cuh); a
 // CTA that gives up waits for its own copies and returns, and the call
 // reports status 4.
 //
@@ -43,11 +51,14 @@ namespace {
 constexpr int LB = 16;                     // rows of a diagonal block
 constexpr int LEAF_BLOCKS = 32;            // diagonal blocks per leaf
 constexpr int BLK = LB * LB;               // elements of a packed 16 x 16 block
-constexpr int NBC = 32;                    // right-hand-side columns per CTA
-constexpr int XS_LD = 40;                  // padded row of a solved block in smem
 constexpr int SEG_MAX = LEAF_BLOCKS * BLK; // largest segment: 31 panel blocks + 1 diagonal block
 constexpr int RING = 3;
-constexpr int THREADS = 256;
+constexpr int XSLOTS = RING + 1;           // solved tiles kept: X_e is published once every warp is
+                                           // done with step e - 1 - RING (its segment's slot)
+constexpr int WARPS = 8;                   // and a warpgroup of which one thread feeds the ring
+constexpr int THREADS = 32 * (WARPS + 4);  // 168 registers a thread at launch (65536 / 384), then
+constexpr int FEED_REGS = 56;              // 4 * 32 * 56 + 8 * 32 * 216 = 62464 of the block's
+constexpr int SOLVE_REGS = 216;            // 384 * 168 = 64512
 
 // Offset (elements) of step d's segment in a leaf of nb blocks: the leaf
 // starts with diagonal block 0, then segment d = (nb - 1 - d) panel blocks
@@ -62,6 +73,10 @@ __device__ __forceinline__ void dmma(double (&c)[4], double a0, double a1, doubl
       "{%0,%1,%2,%3};\n"
       : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
       : "d"(a0), "d"(a1), "d"(b0));
+}
+
+__device__ __forceinline__ void lds128(double (&v)[2], uint32_t addr) {
+  asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v[0]), "=d"(v[1]) : "r"(addr));
 }
 
 struct LeafPackArgs {
@@ -144,9 +159,7 @@ __global__ void __launch_bounds__(256) trsm_leaf_pack_kernel(const LeafPackArgs 
     __syncthreads();
   }
   T *out = (T *)a.out + (long)leaf * a.leaf_stride + off;
-  if (diag && sizeof(T) == 4) {
-    out[tid] = tile[tid / LB][tid % LB];  // row-major
-  } else if (sizeof(T) == 8) {
+  if (sizeof(T) == 8) {
     // MMA A-fragment order: (ks * 32 + lane) * 2 + h holds row g + 8h,
     // column 4 ks + t (lane = 4 g + t).
     const int ks = tid >> 6, lane = (tid >> 1) & 31, h = tid & 1;
@@ -163,305 +176,318 @@ struct LeafArgs {
   T *b;           // the leaf's first row (lower orientation)
   long rs_b, cs_b;
   int n;          // right-hand sides
+  T alpha;        // B is scaled by it as it is read
   int *err;
   unsigned long long wait_ns;
 };
 
-template <typename T>
-constexpr size_t leaf_smem() {
-  return sizeof(T) * ((size_t)RING * SEG_MAX + BLK + 2 * LB * XS_LD) +
-         sizeof(uint64_t) * (RING + 1) + 16;
-}
+// Shape of a CTA: NCG column groups (8 columns of FP64, 32 of FP32), the rows of
+// each dealt out in blocks of 16 to its RG = 8 / NCG warps in turn.
+template <typename T, int NCG>
+struct Leaf {
+  static constexpr bool F64 = sizeof(T) == 8;
+  static constexpr int RG = WARPS / NCG;
+  static constexpr int NBW = LEAF_BLOCKS / RG;  // row blocks of a warp
+  static constexpr int CW = F64 ? 8 : 32;       // columns of a group
+  static constexpr int NBC = NCG * CW;          // columns of a CTA
+  // Rows of a solved tile in shared memory: 8 doubles make both the fragment's
+  // 16-byte stores and its loads conflict-free; 36 floats keep 16-byte accesses
+  // aligned and the transposed ones at two to a bank.
+  static constexpr int XLD = F64 ? 8 : 36;
+  static constexpr int TILE = LB * XLD;
+  static constexpr int RHS = F64 ? 0 : LEAF_BLOCKS * TILE;  // FP32: B, apart from the sums
+  static constexpr size_t SMEM = sizeof(T) * ((size_t)RING * SEG_MAX + BLK + XSLOTS * NCG * TILE + RHS) +
+                                 sizeof(uint64_t) * (2 * RING + 1 + XSLOTS * NCG) + 16;
+};
 
-// FP64: the updates are m16n8k4 .f64 MMAs, acc[q][j][e] the accumulator of
-// row block warp + 8 q, columns 8 j .. 8 j + 7 (element e: row g + 8 (e >> 1),
-// column 2 t + (e & 1)); panel blocks are packed in A-fragment order.
-// FP32: the updates are packed FP32 FMAs (two rows per instruction), one
-// lane per column, acc[q][i2] rows 2 i2 and 2 i2 + 1 of row block
-// warp + 8 q; panel blocks are packed column-major, the diagonal blocks'
-// inverses row-major.
-template <typename T>
+template <typename T, int NCG>
 __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_constant__ LeafArgs<T> p) {
-  constexpr bool F64 = sizeof(T) == 8;
+  using L = Leaf<T, NCG>;
+  constexpr bool F64 = L::F64;
+  constexpr int RG = L::RG, NBW = L::NBW, XLD = L::XLD, AE = F64 ? 4 : 16;
   extern __shared__ __align__(128) unsigned char smem[];
-  T *seg = (T *)smem;                 // [RING][SEG_MAX]
-  T *diag0 = seg + RING * SEG_MAX;    // [BLK]
-  T *xs = diag0 + BLK;                // [2][LB][XS_LD]
-  uint64_t *bar = (uint64_t *)(xs + 2 * LB * XS_LD);  // RING segments + diagonal block 0
-  volatile int *abort_flag = (volatile int *)(bar + RING + 1);
+  T *seg = (T *)smem;                  // [RING][SEG_MAX]
+  T *diag0 = seg + RING * SEG_MAX;     // [BLK]
+  T *xs = diag0 + BLK;                 // [XSLOTS][NCG][TILE]
+  T *rhs = xs + XSLOTS * NCG * L::TILE;
+  uint64_t *full = (uint64_t *)(rhs + L::RHS);  // [RING] segment landed
+  uint64_t *empty = full + RING;                // [RING] every warp done with it
+  uint64_t *dbar = empty + RING;                // diagonal block 0 landed
+  uint64_t *ready = dbar + 1;                   // [XSLOTS][NCG] X_d published
+  volatile int *abort_flag = (volatile int *)(ready + XSLOTS * NCG);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
   const int nb = (p.rows + LB - 1) / LB;
-  const long col0 = (long)blockIdx.x * NBC;
-  // Coalesced 16 x 32 block transfers between B and shared memory: element
-  // (r, c) of pass e is taken with the stored matrix's unit stride across
-  // the warp.
-  const bool rows_fast = labs(p.rs_b) <= labs(p.cs_b);
-  auto rc_of = [&](int e, int &r, int &c) {
-    const int idx = e * 32 + lane;
-    r = rows_fast ? idx % LB : idx / NBC;
-    c = rows_fast ? idx / LB : idx % NBC;
-  };
 
   if (tid == 0) {
-    for (int i = 0; i <= RING; ++i) tc::mbar_init(&bar[i], 1);
+    for (int i = 0; i < RING; ++i) {
+      tc::mbar_init(&full[i], 1);
+      tc::mbar_init(&empty[i], WARPS);
+    }
+    tc::mbar_init(dbar, 1);
+    for (int i = 0; i < XSLOTS * NCG; ++i) tc::mbar_init(&ready[i], 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
   __syncthreads();
 
-  int issued = 0;  // segments issued (thread 0)
-  auto issue = [&](int d) {
-    const uint32_t bytes = (uint32_t)((nb - d) * BLK * sizeof(T));
-    tc::mbar_arrive_expect_tx(&bar[d % RING], bytes);
-    tc::bulk_load_1d(seg + (d % RING) * SEG_MAX, p.pack + seg_off(d, nb), bytes, &bar[d % RING]);
-    issued = d + 1;
-  };
-  if (tid == 0) {
-    tc::mbar_arrive_expect_tx(&bar[RING], BLK * sizeof(T));
-    tc::bulk_load_1d(diag0, p.pack, BLK * sizeof(T), &bar[RING]);
-    for (int d = 0; d < RING - 1 && d < nb - 1; ++d) issue(d);
-  }
-
-  // The CTA's 512 x 32 block of B, staged through ring slot RING - 1 (not
-  // filled before the first step): warp w owns row blocks w, w + 8, w + 16,
-  // w + 24.
-  using Acc = typename std::conditional<F64, double[4][4][4], float2[4][8]>::type;
-  Acc acc;
-  {
-    T *stage = seg + (RING - 1) * SEG_MAX + warp * LB * XS_LD;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int rb = warp + 8 * q;
-#pragma unroll
-      for (int e = 0; e < LB; ++e) {
-        int r, c;
-        rc_of(e, r, c);
-        const int row = rb * LB + r;
-        const long col = col0 + c;
-        stage[r * XS_LD + c] = row < p.rows && col < p.n ? p.b[row * p.rs_b + col * p.cs_b] : T(0);
+  int issued = 0;  // segments issued (the producer's lane 0)
+  if (warp >= WARPS) {
+    tc::setmaxnreg_dec<FEED_REGS>();
+    if (warp == WARPS && lane == 0) {
+      tc::mbar_arrive_expect_tx(dbar, BLK * sizeof(T));
+      tc::bulk_load_1d(diag0, p.pack, BLK * sizeof(T), dbar);
+      for (int d = 0; d < nb - 1; ++d) {
+        const int slot = d % RING;
+        if (d >= RING &&
+            !tc::mbar_wait(&empty[slot], (d / RING - 1) & 1, abort_flag, p.err, p.wait_ns))
+          break;
+        const uint32_t bytes = (uint32_t)((nb - d) * BLK * sizeof(T));
+        tc::mbar_arrive_expect_tx(&full[slot], bytes);
+        tc::bulk_load_1d(seg + slot * SEG_MAX, p.pack + seg_off(d, nb), bytes, &full[slot]);
+        issued = d + 1;
       }
-      __syncwarp();
-      if constexpr (F64) {
+    }
+  } else {
+    tc::setmaxnreg_inc<SOLVE_REGS>();
+    const int cg = warp % NCG, rg = warp / NCG;
+    const long col0 = (long)blockIdx.x * L::NBC + cg * L::CW;
+    const int g = F64 ? lane >> 2 : lane >> 3;  // FP64: rows g, g + 8; FP32: rows 4 g .. 4 g + 3
+    const int t = F64 ? lane & 3 : lane & 7;    // FP64: columns 2 t, 2 t + 1; FP32: 4 t .. 4 t + 3
+    const bool rows_fast = labs(p.rs_b) <= labs(p.cs_b);
+    auto wait = [&](uint64_t *bar, int use) {
+      const bool ok = tc::mbar_wait(bar, use & 1, abort_flag, p.err, p.wait_ns);
+      return __all_sync(0xffffffffu, ok) != 0;
+    };
+    auto xtile = [&](int d) { return xs + ((d % XSLOTS) * NCG + cg) * L::TILE; };
+
+    // acc[0] is always the warp's next block to solve.  FP64: B minus the updates
+    // so far; FP32: minus the updates' sum, B itself waits in shared memory, so
+    // that the updates' roundings are of their (smaller) sum.
+    T acc[NBW][AE];
+    if constexpr (F64) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+      for (int q = 0; q < NBW; ++q)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int row = (rg + RG * q) * LB + g + 8 * (e >> 1);
+          const long col = col0 + 2 * t + (e & 1);
+          acc[q][e] = row < p.rows && col < p.n ? p.b[row * p.rs_b + col * p.cs_b] : T(0);
+        }
+      if (p.alpha != T(1)) {
+#pragma unroll
+        for (int q = 0; q < NBW; ++q)
 #pragma unroll
           for (int e = 0; e < 4; ++e)
-            acc[q][j][e] = stage[(g + 8 * (e >> 1)) * XS_LD + 8 * j + 2 * t + (e & 1)];
-      } else {
-#pragma unroll
-        for (int i2 = 0; i2 < 8; ++i2)
-          acc[q][i2] = make_float2(stage[(2 * i2) * XS_LD + lane], stage[(2 * i2 + 1) * XS_LD + lane]);
-      }
-      __syncwarp();
-    }
-  }
-  // The staging slot is free (and its generic-proxy writes ordered before
-  // the bulk copy that refills it) before any copy targets it.
-  tc::fence_proxy_async();
-  __syncthreads();
-
-  // Owner of a block (warp blk % 8, accumulators acc[q] with q = blk / 8,
-  // fully updated): X = inv(D) R with the packed inverse of its diagonal
-  // block, into xout (row-major, XS_LD) for the other warps' updates.
-  auto solve = [&](int q, const T *dinv, T *xout) {
-    if constexpr (F64) {
-      // R (accumulator layout) -> xout -> B fragments; X = inv(D) R as
-      // 4 x 4 m16n8k4 MMAs (A = inv(D) in fragment order), accumulated in
-      // the now free acc[q]; X -> xout.
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          xout[(g + 8 * (e >> 1)) * XS_LD + 8 * j + 2 * t + (e & 1)] = acc[q][j][e];
-      __syncwarp();
-      double r[4][4];
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) r[ks][j] = xout[(4 * ks + t) * XS_LD + 8 * j + g];
-      __syncwarp();
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[q][j][e] = 0.0;
-      const double2 *af = (const double2 *)dinv;
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const double2 a = af[ks * 32 + lane];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[q][j], a.x, a.y, r[ks][j]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          xout[(g + 8 * (e >> 1)) * XS_LD + 8 * j + 2 * t + (e & 1)] = acc[q][j][e];
-    } else {
-      // One lane per column: x_i = sum_{p <= i} inv(D)_ip r_p (16 independent
-      // dot products over broadcast rows of the row-major inverse).
-      float r[LB];
-#pragma unroll
-      for (int i2 = 0; i2 < 8; ++i2) {
-        r[2 * i2] = acc[q][i2].x;
-        r[2 * i2 + 1] = acc[q][i2].y;
-      }
-#pragma unroll
-      for (int i = 0; i < LB; ++i) {
-        const float4 *row = (const float4 *)(dinv + i * LB);
-        float x = 0.f;
-#pragma unroll
-        for (int v = 0; v <= i / 4; ++v) {
-          const float4 w = row[v];
-          x = fmaf(w.x, r[4 * v], x);
-          if (4 * v + 1 <= i) x = fmaf(w.y, r[4 * v + 1], x);
-          if (4 * v + 2 <= i) x = fmaf(w.z, r[4 * v + 2], x);
-          if (4 * v + 3 <= i) x = fmaf(w.w, r[4 * v + 3], x);
-        }
-        xout[i * XS_LD + lane] = x;
-      }
-    }
-    __syncwarp();
-  };
-
-  // Solved block blk (in xsrc) -> B, by all 256 threads, coalesced along the
-  // stored matrix's unit stride.
-  auto write_block = [&](int blk, const T *xsrc) {
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int idx = tid + h * THREADS;
-      const int r = rows_fast ? idx % LB : idx / NBC, c = rows_fast ? idx / LB : idx % NBC;
-      const int row = blk * LB + r;
-      const long col = col0 + c;
-      if (row < p.rows && col < p.n) p.b[row * p.rs_b + col * p.cs_b] = xsrc[r * XS_LD + c];
-    }
-  };
-
-  // acc[q] -= A_rb,d X_d for row blocks rb = warp + 8 q, q = Q0 .. 3, all in
-  // one unrolled sequence so that the blocks' independent MMA / FMA chains
-  // interleave; X_d's operand fragments (xb / xr) are loaded once per step.
-  // Row blocks past the leaf (rb >= nb) multiply a zero block instead of
-  // reading past the segment.
-  using XFrag = typename std::conditional<F64, double[4][4], float[LB]>::type;
-  auto update_from = [&](auto q0c, const T *sg, int d, const XFrag &xf) {
-    constexpr int Q0 = decltype(q0c)::value;
-    if constexpr (F64) {
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        double2 a[4];
-#pragma unroll
-        for (int q = Q0; q < 4; ++q) {
-          const int rb = warp + 8 * q;
-          a[q] = rb < nb ? ((const double2 *)(sg + (rb - d - 1) * BLK))[ks * 32 + lane]
-                         : make_double2(0.0, 0.0);
-        }
-#pragma unroll
-        for (int q = Q0; q < 4; ++q)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) dmma(acc[q][j], -a[q].x, -a[q].y, xf[ks][j]);
+            acc[q][e] = (rg + RG * q) * LB + g + 8 * (e >> 1) < p.rows ? p.alpha * acc[q][e] : T(0);
       }
     } else {
 #pragma unroll
-      for (int kk = 0; kk < LB; ++kk) {
-        const float xv = xf[kk];
+      for (int q = 0; q < NBW; ++q) {
+        T *tile = rhs + (rg + RG * q) * L::TILE;
 #pragma unroll
-        for (int q = Q0; q < 4; ++q) {
-          const int rb = warp + 8 * q;
-          if (rb >= nb) continue;
-          const float4 *col = (const float4 *)(sg + (rb - d - 1) * BLK + kk * LB);
+        for (int e = 0; e < LB; ++e) {
+          const int idx = e * 32 + lane;
+          const int r = rows_fast ? idx % LB : idx / 32, c = rows_fast ? idx / LB : idx % 32;
+          const int row = (rg + RG * q) * LB + r;
+          const long col = col0 + c;
+          tile[r * XLD + c] = row < p.rows && col < p.n ? p.b[row * p.rs_b + col * p.cs_b] : T(0);
+        }
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const float4 a = col[v];
-            acc[q][2 * v] =
-                __ffma2_rn(make_float2(a.x, a.y), make_float2(xv, xv), acc[q][2 * v]);
-            acc[q][2 * v + 1] =
-                __ffma2_rn(make_float2(a.z, a.w), make_float2(xv, xv), acc[q][2 * v + 1]);
+        for (int e = 0; e < AE; ++e) acc[q][e] = T(0);
+      }
+      __syncwarp();
+    }
+
+    // FP64: a tile x as B operand, the fragments of its four k steps, and
+    // c += blk x for one 16 x 16 block of A.
+    auto load_x = [&](double (&xf)[4], const T *x) {
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) xf[ks] = x[(4 * ks + t) * XLD + g];
+    };
+    auto mma_block = [&](double (&c)[4], const T *blk, const double (&xf)[4]) {
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks) {
+        const double2 a = ((const double2 *)blk)[ks * 32 + lane];
+        dmma(c, a.x, a.y, xf[ks]);
+      }
+    };
+    // FP32: c[i] += (MINUS: -=) the block at b[i] times the tile x, i < N.  One
+    // block alone is unrolled for its latency, several only as far as their
+    // independent chains need (the update's code stays in the instruction cache).
+    auto fma_blocks = [&](auto nc, auto minus, auto &c, const T *const *b, const T *x) {
+      constexpr int N = decltype(nc)::value, U = N == 1 ? LB : 4;
+      constexpr bool MINUS = decltype(minus)::value;
+#pragma unroll U
+      for (int k = 0; k < LB; ++k) {
+        const float4 v = *(const float4 *)&x[k * XLD + 4 * t];
+        const float xv[4] = {MINUS ? -v.x : v.x, MINUS ? -v.y : v.y, MINUS ? -v.z : v.z,
+                             MINUS ? -v.w : v.w};
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const float4 a = *(const float4 *)&b[i][k * LB + 4 * g];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            c[i][j] = fmaf(a.x, xv[j], c[i][j]);
+            c[i][4 + j] = fmaf(a.y, xv[j], c[i][4 + j]);
+            c[i][8 + j] = fmaf(a.z, xv[j], c[i][8 + j]);
+            c[i][12 + j] = fmaf(a.w, xv[j], c[i][12 + j]);
           }
         }
       }
-    }
-  };
-  // The owner's block d + 1 alone (block 0 of the segment).
-  auto update_one = [&](int q, const T *sg, const XFrag &xf) {
-    if constexpr (F64) {
-      const double2 *af = (const double2 *)sg;
-#pragma unroll
-      for (int ks = 0; ks < 4; ++ks) {
-        const double2 a = af[ks * 32 + lane];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(acc[q][j], -a.x, -a.y, xf[ks][j]);
-      }
-    } else {
-#pragma unroll
-      for (int kk = 0; kk < LB; ++kk) {
-        const float xv = xf[kk];
-        const float4 *col = (const float4 *)(sg + kk * LB);
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const float4 a = col[v];
-          acc[q][2 * v] = __ffma2_rn(make_float2(a.x, a.y), make_float2(xv, xv), acc[q][2 * v]);
-          acc[q][2 * v + 1] =
-              __ffma2_rn(make_float2(a.z, a.w), make_float2(xv, xv), acc[q][2 * v + 1]);
-        }
-      }
-    }
-  };
-
-  int d = 0;
-  bool ok = tc::mbar_wait(&bar[RING], 0, abort_flag, p.err, p.wait_ns);
-  if (__syncthreads_and(ok)) {
-    if (warp == 0) solve(0, diag0, xs);
-    for (; d + 1 < nb; ++d) {
-      ok = tc::mbar_wait(&bar[d % RING], (d / RING) & 1, abort_flag, p.err, p.wait_ns);
-      // X_d is in xs[d & 1], segment d has landed, and every warp is done
-      // with step d - 1 (so its ring slot, (d + 2) % RING, is free).
-      if (!__syncthreads_and(ok)) break;
-      if (tid == 0 && d + 2 <= nb - 2) issue(d + 2);
-      const T *sg = seg + (d % RING) * SEG_MAX;
-      const T *xd = xs + (d & 1) * LB * XS_LD;
-      XFrag xf;
+    };
+    using One = std::integral_constant<int, 1>;
+    auto store_tile = [&](T *x, const T (&c)[AE]) {
       if constexpr (F64) {
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) xf[ks][j] = xd[(4 * ks + t) * XS_LD + 8 * j + g];
+        *(double2 *)&x[g * XLD + 2 * t] = make_double2(c[0], c[1]);
+        *(double2 *)&x[(g + 8) * XLD + 2 * t] = make_double2(c[2], c[3]);
       } else {
 #pragma unroll
-        for (int kk = 0; kk < LB; ++kk) xf[kk] = -xd[kk * XS_LD + lane];
+        for (int i = 0; i < 4; ++i)
+          *(float4 *)&x[(4 * g + i) * XLD + 4 * t] =
+              make_float4(c[4 * i], c[4 * i + 1], c[4 * i + 2], c[4 * i + 3]);
       }
-      // (q runs over compile-time values so the accumulators stay in
-      // registers.)  The owner of block d + 1 goes first: its update and
-      // solve are the step's critical path.
+    };
+    int next = rg;  // the row block in acc[0]
+    // acc[0], fully updated: X = inv(D) R, published to the group's other warps
+    // and written to B; the warp's blocks move up by one.
+    auto solve = [&](const T *dinv) {
+      T *x = xtile(next);
+      if constexpr (!F64) {
+        const T *tile = rhs + next * L::TILE;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int rb = warp + 8 * q;
-        if (rb == d + 1) {
-          update_one(q, sg, xf);
-          solve(q, sg + (nb - 1 - d) * BLK, xs + ((d + 1) & 1) * LB * XS_LD);
+        for (int i = 0; i < 4; ++i) {
+          const float4 b = *(const float4 *)&tile[(4 * g + i) * XLD + 4 * t];
+          acc[0][4 * i] = fmaf(p.alpha, b.x, acc[0][4 * i]);
+          acc[0][4 * i + 1] = fmaf(p.alpha, b.y, acc[0][4 * i + 1]);
+          acc[0][4 * i + 2] = fmaf(p.alpha, b.z, acc[0][4 * i + 2]);
+          acc[0][4 * i + 3] = fmaf(p.alpha, b.w, acc[0][4 * i + 3]);
         }
       }
-      write_block(d, xd);
-      // This warp's blocks below d + 1: q >= qlo.
-      const int qlo = d + 1 - warp < 0 ? 0 : (d + 1 - warp) / 8 + 1;
-      switch (qlo) {
-        case 0: update_from(std::integral_constant<int, 0>(), sg, d, xf); break;
-        case 1: update_from(std::integral_constant<int, 1>(), sg, d, xf); break;
-        case 2: update_from(std::integral_constant<int, 2>(), sg, d, xf); break;
-        case 3: update_from(std::integral_constant<int, 3>(), sg, d, xf); break;
-        default: break;
+      store_tile(x, acc[0]);
+      __syncwarp();
+      T c[1][AE];
+#pragma unroll
+      for (int e = 0; e < AE; ++e) c[0][e] = T(0);
+      if constexpr (F64) {
+        double r[4];
+        load_x(r, x);
+        mma_block(c[0], dinv, r);
+      } else {
+        fma_blocks(One(), std::false_type(), c, &dinv, x);
       }
+      __syncwarp();
+      store_tile(x, c[0]);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&ready[(next % XSLOTS) * NCG + cg]);
+      if constexpr (F64) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int row = next * LB + g + 8 * (e >> 1);
+          const long col = col0 + 2 * t + (e & 1);
+          if (row < p.rows && col < p.n) p.b[row * p.rs_b + col * p.cs_b] = c[0][e];
+        }
+      } else if (rows_fast) {  // two columns of 16 rows to a store
+        const int r = lane % LB, row = next * LB + r;
+        const long col = col0 + lane / LB;
+        T *out = p.b + row * p.rs_b + col * p.cs_b;
+        const int left = row < p.rows ? (int)min(p.n - col, 32L) : 0;
+#pragma unroll
+        for (int e = 0; e < LB; ++e) {
+          if (2 * e < left) *out = x[r * XLD + lane / LB + 2 * e];
+          out += 2 * p.cs_b;
+        }
+      } else {  // a row to a store
+        T *out = p.b + next * LB * p.rs_b + (col0 + lane) * p.cs_b;
+        const int left = col0 + lane < p.n ? p.rows - next * LB : 0;
+#pragma unroll
+        for (int e = 0; e < LB; ++e) {
+          if (e < left) *out = x[e * XLD + lane];
+          out += p.rs_b;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q + 1 < NBW; ++q)
+#pragma unroll
+        for (int e = 0; e < AE; ++e) acc[q][e] = acc[q + 1][e];
+      next += RG;
+    };
+
+    bool ok = true;
+    if (rg == 0) {
+      ok = wait(dbar, 0);
+      if (ok) solve(diag0);
     }
-    if (d + 1 == nb) {
-      __syncthreads();  // the last block, solved in the last step
-      write_block(d, xs + (d & 1) * LB * XS_LD);
+    for (int d = 0; ok && d + 1 < nb; ++d) {
+      const int slot = d % RING;
+      ok = wait(&full[slot], d / RING);
+      if (!ok) break;
+      if (next < nb) {
+        ok = wait(&ready[(d % XSLOTS) * NCG + cg], d / XSLOTS);
+        if (!ok) break;
+        const T *sg = seg + slot * SEG_MAX;
+        if constexpr (F64) {
+          double xf[4];  // -X_d
+          load_x(xf, xtile(d));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) xf[i] = -xf[i];
+          if (next == d + 1) {
+            // The step's critical path comes first.
+            mma_block(acc[0], sg, xf);
+            solve(sg + (nb - 1 - d) * BLK);
+          }
+          // Two blocks at a time, for two chains of MMAs.  Where the second lies
+          // past the leaf its accumulators are dead; it reads the first's block.
+          const uint32_t a0 = tc::smem_u32(sg) + lane * 16;
+#pragma unroll
+          for (int q = 0; q < NBW; q += 2) {
+            const int rb = next + RG * q;
+            if (rb < nb) {
+              const uint32_t b0 = a0 + (rb - d - 1) * (BLK * 8);
+              const uint32_t b1 = b0 + (rb + RG < nb ? RG * BLK * 8 : 0);
+              double f0[4][2], f1[4][2];
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) {
+                lds128(f0[ks], b0 + ks * 512);
+                lds128(f1[ks], b1 + ks * 512);
+              }
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) {
+                dmma(acc[q], f0[ks][0], f0[ks][1], xf[ks]);
+                dmma(acc[q + 1], f1[ks][0], f1[ks][1], xf[ks]);
+              }
+            }
+          }
+        } else {
+          static_assert(F64 || NBW == 4, "four blocks a warp");
+          const T *x = xtile(d);
+          if (next == d + 1) {
+            fma_blocks(One(), std::true_type(), acc, &sg, x);
+            solve(sg + (nb - 1 - d) * BLK);
+          }
+          // Three or four blocks, or up to two; dead ones as above.
+          const T *b[4];
+          b[0] = sg + (next - d - 1) * BLK;
+#pragma unroll
+          for (int i = 1; i < 4; ++i) b[i] = next + RG * i < nb ? b[0] + RG * i * BLK : b[0];
+          if (next + 2 * RG < nb)
+            fma_blocks(std::integral_constant<int, 4>(), std::true_type(), acc, b, x);
+          else if (next < nb)
+            fma_blocks(std::integral_constant<int, 2>(), std::true_type(), acc, b, x);
+        }
+      }
+      // Reads done before the copy that refills the slot.
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&empty[slot]);
     }
-  } else {
-    d = -1;  // diagonal block 0 never arrived
   }
-  if (d + 1 < nb && tid == 0) {
-    // Gave up: wait (bounded) for this CTA's copies still in flight.
-    if (d < 0) tc::mbar_wait_drain(&bar[RING], 0);
-    for (int s = d < 0 ? 0 : d; s < issued; ++s) tc::mbar_wait_drain(&bar[s % RING], (s / RING) & 1);
+  // Every wait above is bounded, so every thread comes here; if a warp gave up,
+  // copies may still be in flight into this CTA's shared memory.
+  __syncthreads();
+  if (*abort_flag && warp == WARPS && lane == 0) {
+    tc::mbar_wait_drain(dbar, 0);
+    for (int s = issued < RING ? 0 : issued - RING; s < issued; ++s)
+      tc::mbar_wait_drain(&full[s % RING], (s / RING) & 1);
   }
 }
 
@@ -491,32 +517,49 @@ extern "C" int b200_trsm_leaf_pack(int dtype, const void *a, long rs_a, long cs_
   return B200_OK;
 }
 
-// Solves one leaf (`rows` rows) of a packed solve for n right-hand sides:
+// Solves one leaf (`rows` rows) of a packed solve for n right-hand sides, B
+// scaled by alpha first:
 // b points at the leaf's first row in lower orientation (for an upper leaf,
 // its last row, with rs_b negated).
-template <typename T>
-int leaf_solve(const void *pack, int rows, T *b, long rs_b, long cs_b, int n) {
-  if (rows <= 0 || n <= 0) return B200_OK;
-  cudaStream_t s = b200_cur_stream();
+template <typename T, int NCG>
+int leaf_launch(const LeafArgs<T> &la, cudaStream_t s) {
+  using L = Leaf<T, NCG>;
   static std::once_flag once;
   static int conf = B200_OK;
-  constexpr size_t smem = leaf_smem<T>();
   B200_TRY(b200_once(once, conf, "trsm leaf kernel: set-up failed", []() -> int {
-    B200_CUDA_TRY(cudaFuncSetAttribute(trsm_leaf_kernel<T>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    B200_CUDA_TRY(cudaFuncSetAttribute(trsm_leaf_kernel<T, NCG>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM));
     return B200_OK;
   }));
-  LeafArgs<T> la{(const T *)pack, rows, b, rs_b, cs_b, n, b200_device_error_word(), B200_WAIT_NS};
-  const long grid = b200_ceil_div(n, NBC);
+  const long grid = b200_ceil_div(la.n, L::NBC);
   if (grid > 0x7fffffffL) return b200_set_error(B200_EINVAL, "trsm: too many right-hand sides");
   B200ProfScope prof(sizeof(T) == 4 ? "trsm_leaf_s" : "trsm_leaf_d", s);
-  trsm_leaf_kernel<T><<<(unsigned)grid, THREADS, smem, s>>>(la);
+  trsm_leaf_kernel<T, NCG><<<(unsigned)grid, THREADS, L::SMEM, s>>>(la);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
 
+template <typename T>
+int leaf_solve(const void *pack, int rows, T *b, long rs_b, long cs_b, int n, double alpha) {
+  if (rows <= 0 || n <= 0) return B200_OK;
+  cudaStream_t s = b200_cur_stream();
+  const LeafArgs<T> la{(const T *)pack, rows, b, rs_b, cs_b, n, (T)alpha, b200_device_error_word(),
+                       B200_WAIT_NS};
+  if constexpr (sizeof(T) == 4) {
+    return leaf_launch<T, 1>(la, s);
+  } else {
+    // 16 columns to a CTA, or 8 where those still fit the SMs in one wave (twice
+    // the SMs on the same columns).  One leaf of 300-512 rows, us for 8 / 16 / 32
+    // columns to a CTA: n = 300 31 / 43 / 84, n = 1000 28 / 43 / 82; DTRSM calls of
+    // 1500 x 1500 304 / 280 / 397, 4096 x 4096 2680 / 2577 / 2772, 700 x 8000
+    // 329 / 307 / 326.  (Every column gets the same bits either way.)
+    if (n > 8L * b200_sm_count()) return leaf_launch<T, 2>(la, s);
+    return leaf_launch<T, 1>(la, s);
+  }
+}
+
 extern "C" int b200_trsm_leaf_solve(int dtype, const void *pack, int rows, void *b, long rs_b,
-                                    long cs_b, int n) {
-  if (dtype == B200_F32) return leaf_solve<float>(pack, rows, (float *)b, rs_b, cs_b, n);
-  return leaf_solve<double>(pack, rows, (double *)b, rs_b, cs_b, n);
+                                    long cs_b, int n, double alpha) {
+  if (dtype == B200_F32) return leaf_solve<float>(pack, rows, (float *)b, rs_b, cs_b, n, alpha);
+  return leaf_solve<double>(pack, rows, (double *)b, rs_b, cs_b, n, alpha);
 }
