@@ -1,5 +1,5 @@
 // grouped.cu -- many independent GEMMs / left TRSMs of uneven sizes in one
-// persistent launch each, plus the plan object that autotunes the tile shape
+// launch per tile shape or order class, plus the plan object that autotunes the tile shape
 // and captures the launches in a CUDA graph for replay.
 //
 // The reference has no batched interface: every call runs the full driver
@@ -7,9 +7,9 @@
 // cost is launch latency and packing passes, not flops, so the grouped path
 // (a) reads operands directly from caller memory with bounds checks (no
 // pack pass), (b) maps every output tile of every problem into one global
-// tile index space (prefix sums over per-problem tile counts) walked by a
-// persistent grid, and (c) solves each TRSM instance's column slab entirely
-// on one CTA.
+// tile index space (prefix sums over per-problem tile counts), a CTA of the
+// direct kernel (gemm_direct.cu) to a tile, and (c) solves each TRSM instance
+// in slabs of 32 right-hand sides, a CTA of trsm_small.cu to a slab.
 #include <algorithm>
 #include <cstring>
 #include <cstdio>
@@ -103,13 +103,14 @@ int build_group(std::vector<GemmEntry> &src, int variant, GemmGroup &g, cudaStre
 
 int to_entries(char dtype, const mublis_b200_gemm_problem_t *p, int count,
                std::vector<GemmEntry> (&cls)[NCLASS]) {
+  B200DevicePtrs ptrs;
   for (int q = 0; q < count; ++q) {
     const mublis_b200_gemm_problem_t &x = p[q];
     if (x.m < 0 || x.n < 0 || x.k < 0) return b200_set_error(B200_EINVAL, "grouped gemm: negative size");
     if (x.m == 0 || x.n == 0) continue;
     if (x.ldc < std::max(1, x.m)) return b200_set_error(B200_EINVAL, "grouped gemm: ldc too small");
     const bool upd = x.alpha != 0.0 && x.k > 0;
-    if (!b200_is_device_ptr(x.c) || (upd && (!b200_is_device_ptr(x.a) || !b200_is_device_ptr(x.b))))
+    if (!ptrs.device(x.c) || (upd && (!ptrs.device(x.a) || !ptrs.device(x.b))))
       return b200_set_error(B200_EINVAL, "grouped gemm: operands must be device pointers");
     GemmEntry e;
     memset(&e, 0, sizeof e);
@@ -326,13 +327,14 @@ void order_slabs(TrsmGroup &g) {
 }
 
 int to_trsm(const mublis_b200_trsm_problem_t *p, int count, TrsmGroup &g, cudaStream_t s) {
+  B200DevicePtrs ptrs;
   for (int q = 0; q < count; ++q) {
     const mublis_b200_trsm_problem_t &x = p[q];
     if (x.m < 0 || x.n < 0) return b200_set_error(B200_EINVAL, "grouped trsm: negative size");
     if (x.m == 0 || x.n == 0) continue;
     if (x.uplo != MUBLIS_LOWER && x.uplo != MUBLIS_UPPER)
       return b200_set_error(B200_EINVAL, "grouped trsm: uplo must be lower or upper");
-    if (!b200_is_device_ptr(x.b) || (x.alpha != 0.0 && !b200_is_device_ptr(x.a)))
+    if (!ptrs.device(x.b) || (x.alpha != 0.0 && !ptrs.device(x.a)))
       return b200_set_error(B200_EINVAL, "grouped trsm: operands must be device pointers");
     if (x.m > TRSM_MAX_ORDER || x.alpha == 0.0) {
       g.fallback.push_back(q);

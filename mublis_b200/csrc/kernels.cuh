@@ -366,6 +366,21 @@ int b200_group_vec(const b200_group_gemm_t &e, int elt);
 int launch_direct_group(int dtype, int tile, const b200_group_gemm_t *table, const int *tile_prob,
                         int tiles, cudaStream_t s);
 
+// b200_is_device_ptr for the many operands of one call (runtime.cu): a pointer
+// inside an allocation that an earlier one of the call lay in needs no query.
+// Lives for one call, on its thread: nothing is known of the next call's pointers.
+class B200DevicePtrs {
+ public:
+  bool device(const void *p);
+
+ private:
+  static constexpr int RANGES = 8, PROBES = 32;
+  struct Range {
+    uintptr_t base, end;
+  } range_[RANGES];
+  int count_ = 0, last_ = 0, misses_ = 0, hits_ = 0;
+};
+
 // ---- small triangular solves (trsm_small.cu)
 
 constexpr int B200_TRSM_SMALL = 256;      // largest order

@@ -562,13 +562,14 @@ int b200_tcg_create(const mublis_b200_gemm_problem_t *p, int count, b200_tcg **o
   std::vector<TcgPackTask> tasks;
   long a_bytes = 0, b_bytes = 0, nexp = 0;
   int kpad_max = TCG_BK;
+  B200DevicePtrs ptrs;
   for (int q = 0; q < count; ++q) {
     const mublis_b200_gemm_problem_t &x = p[q];
     if (x.m < 0 || x.n < 0 || x.k < 0) return b200_set_error(B200_EINVAL, "grouped gemm: negative size");
     if (x.m == 0 || x.n == 0) continue;
     if (x.ldc < std::max(1, x.m)) return b200_set_error(B200_EINVAL, "grouped gemm: ldc too small");
     const bool upd = x.alpha != 0.0 && x.k > 0;
-    if (!b200_is_device_ptr(x.c) || (upd && (!b200_is_device_ptr(x.a) || !b200_is_device_ptr(x.b))))
+    if (!ptrs.device(x.c) || (upd && (!ptrs.device(x.a) || !ptrs.device(x.b))))
       return b200_set_error(B200_EINVAL, "grouped gemm: operands must be device pointers");
     const int k = upd ? x.k : 0, kb = (int)b200_ceil_div(k, TCG_BK);
     const int mt = (int)b200_ceil_div(x.m, TCG_BM), nt128 = (int)b200_ceil_div(x.n, TCG_BM);
