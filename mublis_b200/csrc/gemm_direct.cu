@@ -629,9 +629,13 @@ int launch_direct_group(int dtype, int tile, const b200_group_gemm_t *table, con
 //   start + kb * max(alone, n * shared) + (n - 1) * next
 // -- alone / shared: a k-block of a CTA that has the SM to itself / of one
 // that shares it; next: filling and draining one more CTA.  Packed: start plus
-// the flops at the 128 x 128 kernels' rate.  Fitted to timings of both over
+// the flops at the 128 x 128 kernels' rate; an FP32 call whose tiles fill their
+// last wave does better, 27 + waves * (1.28 a k-block + 4), and is sent there
+// when that wins by 20 (operands off 16 bytes are packed for about as much):
+// 1536^3, 144 tiles on 148 SMs, 201 -> 147, 1535^3 216 -> 163, 1408 x 1536 x 900
+// 132 -> 99.  Fitted to timings of both over
 // 16^3 .. 1536^3 and ragged shapes, e.g. (FP32 packed -> direct) 64^3 40 -> 16,
-// 512^3 85 -> 25, 1024^3 121 -> 75, 1536^3 202 -> 200, 64 x 64 x 4096 139 -> 23,
+// 512^3 85 -> 25, 1024^3 121 -> 75, 64 x 64 x 4096 139 -> 23,
 // 300 x 300 x 4096 145 -> 48, 100 x 3000 x 700 84 -> 35; (FP64) 301 x 177 x 211
 // 79 -> 18, 1024^3 127 -> 98, 1536^3 243 -> 255.
 b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d) {
@@ -650,6 +654,10 @@ b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d) {
   const double tri_k = dom.jp != MUBLIS_L3_ALL || dom.pi != MUBLIS_L3_ALL ? 0.5 : 1.0;
   const double flops = 2 * m * n * k * tri_c * tri_k;
   double best = f64 ? 60.0 + 0.85e6 * flops / 34e12 : 60.0 + 1.2e6 * flops / 61e12;
+  if (!f64 && tri_c == 1.0 && tri_k == 1.0) {
+    const double waves = std::ceil(std::ceil(m / 128) * std::ceil(n / 128) / sms);
+    best = std::min(best, 47.0 + waves * (std::ceil(k / 16) * 1.28 + 4.0));
+  }
   b200_direct_choice_t ch = {0, 1};
   for (int big = 0; big < 2; ++big) {
     const Cost &c = cost[f64][big];
