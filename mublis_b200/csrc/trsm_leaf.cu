@@ -9,7 +9,7 @@
 // solves the MR x MR diagonal block A11 (packed with its diagonal already
 // inverted, packm.c:143-144) in registers.  Here a CTA owns 8 or 16 columns (FP32:
 // 32) of a leaf of 512 rows and keeps that whole block of B in registers.  A
-// column group (8 columns of FP64, 32 of FP32) has 4 or 8 of the 8 warps, and its
+// column group (8 columns of FP64, 32 of FP32) has 8 warps, and its
 // 32 row blocks of 16 go to them in turn.  For each diagonal block d of 16 rows:
 //   * the warp that owns block d + 1 first applies block d's update to it and
 //     solves it, X = inv(D) R with the inverse of its 16 x 16 diagonal block, and
@@ -25,8 +25,8 @@
 // it at 16 columns).  A CTA of 32 columns whose 8 warps each updated 16 x 32
 // blocks, with a barrier per step, took 78 us a leaf in FP64 and 82 us in FP32
 // (its FMAs took an A operand from shared memory for every two of them); now 28 us
-// (8 columns) or 43 us (16), and 52 us.  DTRSM 1000 x 1000 225 -> 123 us, 4096 x
-// 4096 2726 -> 2580; STRSM 1001 x 1500 231 -> 184.
+// (8 columns) or 37 us (16, on 16 warps), and 52 us.  DTRSM 1000 x 1000 225 -> 123
+// us, 4096 x 4096 2726 -> 2501; STRSM 1001 x 1500 231 -> 184.
 //
 // The leaf's A is packed once per solve (trsm_leaf_pack_kernel) into one contiguous
 // segment per step -- the column of 16 x 16 blocks below the diagonal block (FP64 in
@@ -55,10 +55,6 @@ constexpr int SEG_MAX = LEAF_BLOCKS * BLK; // largest segment: 31 panel blocks +
 constexpr int RING = 3;
 constexpr int XSLOTS = RING + 1;           // solved tiles kept: X_e is published once every warp is
                                            // done with step e - 1 - RING (its segment's slot)
-constexpr int WARPS = 8;                   // and a warpgroup of which one thread feeds the ring
-constexpr int THREADS = 32 * (WARPS + 4);  // 168 registers a thread at launch (65536 / 384), then
-constexpr int FEED_REGS = 56;              // 4 * 32 * 56 + 8 * 32 * 216 = 62464 of the block's
-constexpr int SOLVE_REGS = 216;            // 384 * 168 = 64512
 
 // Offset (elements) of step d's segment in a leaf of nb blocks: the leaf
 // starts with diagonal block 0, then segment d = (nb - 1 - d) panel blocks
@@ -107,7 +103,7 @@ __device__ T leaf_elem(const LeafPackArgs &a, long r0, int rows, int i, int p) {
 // leaf * LEAF_BLOCKS + s; s = 0 is diagonal block 0, s = d + 1 is step d's
 // segment, whose block x is panel block d + 1 + x or, for the last x, the
 // inverse of diagonal block d + 1.  FP64 blocks are stored in MMA
-// A-fragment order; FP32 panel blocks column-major, inverses row-major.
+// A-fragment order; FP32 blocks column-major.
 template <typename T>
 __global__ void __launch_bounds__(256) trsm_leaf_pack_kernel(const LeafPackArgs a) {
   __shared__ T tile[LB][LB + 1];
@@ -182,11 +178,16 @@ struct LeafArgs {
 };
 
 // Shape of a CTA: NCG column groups (8 columns of FP64, 32 of FP32), the rows of
-// each dealt out in blocks of 16 to its RG = 8 / NCG warps in turn.
-template <typename T, int NCG>
+// each dealt out in blocks of 16 to its RG = W / NCG warps in turn.
+template <typename T, int NCG, int W>
 struct Leaf {
   static constexpr bool F64 = sizeof(T) == 8;
-  static constexpr int RG = WARPS / NCG;
+  // W warps solve; a warpgroup, of which one thread feeds the ring, gives them its
+  // registers: 168 a thread at launch (65536 / 384), 4 * 32 * 56 + 8 * 32 * 216 =
+  // 62464 of 64512, or 96 (65536 / 640), 4 * 32 * 32 + 16 * 32 * 112 = 61440.
+  static constexpr int THREADS = 32 * (W + 4);
+  static constexpr int FEED_REGS = W == 8 ? 56 : 32, SOLVE_REGS = W == 8 ? 216 : 112;
+  static constexpr int RG = W / NCG;
   static constexpr int NBW = LEAF_BLOCKS / RG;  // row blocks of a warp
   static constexpr int CW = F64 ? 8 : 32;       // columns of a group
   static constexpr int NBC = NCG * CW;          // columns of a CTA
@@ -200,9 +201,9 @@ struct Leaf {
                                  sizeof(uint64_t) * (2 * RING + 1 + XSLOTS * NCG) + 16;
 };
 
-template <typename T, int NCG>
-__global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_constant__ LeafArgs<T> p) {
-  using L = Leaf<T, NCG>;
+template <typename T, int NCG, int W>
+__global__ void __launch_bounds__(32 * (W + 4), 1) trsm_leaf_kernel(const __grid_constant__ LeafArgs<T> p) {
+  using L = Leaf<T, NCG, W>;
   constexpr bool F64 = L::F64;
   constexpr int RG = L::RG, NBW = L::NBW, XLD = L::XLD, AE = F64 ? 4 : 16;
   extern __shared__ __align__(128) unsigned char smem[];
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
   if (tid == 0) {
     for (int i = 0; i < RING; ++i) {
       tc::mbar_init(&full[i], 1);
-      tc::mbar_init(&empty[i], WARPS);
+      tc::mbar_init(&empty[i], W);
     }
     tc::mbar_init(dbar, 1);
     for (int i = 0; i < XSLOTS * NCG; ++i) tc::mbar_init(&ready[i], 1);
@@ -231,9 +232,9 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
   __syncthreads();
 
   int issued = 0;  // segments issued (the producer's lane 0)
-  if (warp >= WARPS) {
-    tc::setmaxnreg_dec<FEED_REGS>();
-    if (warp == WARPS && lane == 0) {
+  if (warp >= W) {
+    tc::setmaxnreg_dec<L::FEED_REGS>();
+    if (warp == W && lane == 0) {
       tc::mbar_arrive_expect_tx(dbar, BLK * sizeof(T));
       tc::bulk_load_1d(diag0, p.pack, BLK * sizeof(T), dbar);
       for (int d = 0; d < nb - 1; ++d) {
@@ -248,7 +249,7 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
       }
     }
   } else {
-    tc::setmaxnreg_inc<SOLVE_REGS>();
+    tc::setmaxnreg_inc<L::SOLVE_REGS>();
     const int cg = warp % NCG, rg = warp / NCG;
     const long col0 = (long)blockIdx.x * L::NBC + cg * L::CW;
     const int g = F64 ? lane >> 2 : lane >> 3;  // FP64: rows g, g + 8; FP32: rows 4 g .. 4 g + 3
@@ -264,15 +265,20 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
     // so far; FP32: minus the updates' sum, B itself waits in shared memory, so
     // that the updates' roundings are of their (smaller) sum.
     T acc[NBW][AE];
+    // FP64: the lane's first element of B (row g of block 0, column 2 t).
+    T *const b00 = p.b + g * p.rs_b + (col0 + 2 * t) * p.cs_b;
+    const int ncol = (int)min(p.n - col0 - 2 * t, 2L);  // its columns that exist
     if constexpr (F64) {
+      const T *src = b00 + rg * LB * p.rs_b;
 #pragma unroll
-      for (int q = 0; q < NBW; ++q)
+      for (int q = 0; q < NBW; ++q) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int row = (rg + RG * q) * LB + g + 8 * (e >> 1);
-          const long col = col0 + 2 * t + (e & 1);
-          acc[q][e] = row < p.rows && col < p.n ? p.b[row * p.rs_b + col * p.cs_b] : T(0);
+          const bool in = (rg + RG * q) * LB + g + 8 * (e >> 1) < p.rows && (e & 1) < ncol;
+          acc[q][e] = in ? src[8 * (e >> 1) * p.rs_b + (e & 1) * p.cs_b] : T(0);
         }
+        src += RG * LB * p.rs_b;
+      }
       if (p.alpha != T(1)) {
 #pragma unroll
         for (int q = 0; q < NBW; ++q)
@@ -380,12 +386,11 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&ready[(next % XSLOTS) * NCG + cg]);
       if constexpr (F64) {
+        T *out = b00 + next * LB * p.rs_b;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int row = next * LB + g + 8 * (e >> 1);
-          const long col = col0 + 2 * t + (e & 1);
-          if (row < p.rows && col < p.n) p.b[row * p.rs_b + col * p.cs_b] = c[0][e];
-        }
+        for (int e = 0; e < 4; ++e)
+          if (next * LB + g + 8 * (e >> 1) < p.rows && (e & 1) < ncol)
+            out[8 * (e >> 1) * p.rs_b + (e & 1) * p.cs_b] = c[0][e];
       } else if (rows_fast) {  // two columns of 16 rows to a store
         const int r = lane % LB, row = next * LB + r;
         const long col = col0 + lane / LB;
@@ -437,6 +442,7 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
           }
           // Two blocks at a time, for two chains of MMAs.  Where the second lies
           // past the leaf its accumulators are dead; it reads the first's block.
+          constexpr int KS = W == 8 ? 4 : 2;  // k steps of fragments loaded ahead
           const uint32_t a0 = tc::smem_u32(sg) + lane * 16;
 #pragma unroll
           for (int q = 0; q < NBW; q += 2) {
@@ -444,16 +450,19 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
             if (rb < nb) {
               const uint32_t b0 = a0 + (rb - d - 1) * (BLK * 8);
               const uint32_t b1 = b0 + (rb + RG < nb ? RG * BLK * 8 : 0);
-              double f0[4][2], f1[4][2];
 #pragma unroll
-              for (int ks = 0; ks < 4; ++ks) {
-                lds128(f0[ks], b0 + ks * 512);
-                lds128(f1[ks], b1 + ks * 512);
-              }
+              for (int k0 = 0; k0 < 4; k0 += KS) {
+                double f0[KS][2], f1[KS][2];
 #pragma unroll
-              for (int ks = 0; ks < 4; ++ks) {
-                dmma(acc[q], f0[ks][0], f0[ks][1], xf[ks]);
-                dmma(acc[q + 1], f1[ks][0], f1[ks][1], xf[ks]);
+                for (int ks = 0; ks < KS; ++ks) {
+                  lds128(f0[ks], b0 + (k0 + ks) * 512);
+                  lds128(f1[ks], b1 + (k0 + ks) * 512);
+                }
+#pragma unroll
+                for (int ks = 0; ks < KS; ++ks) {
+                  dmma(acc[q], f0[ks][0], f0[ks][1], xf[k0 + ks]);
+                  dmma(acc[q + 1], f1[ks][0], f1[ks][1], xf[k0 + ks]);
+                }
               }
             }
           }
@@ -484,7 +493,7 @@ __global__ void __launch_bounds__(THREADS, 1) trsm_leaf_kernel(const __grid_cons
   // Every wait above is bounded, so every thread comes here; if a warp gave up,
   // copies may still be in flight into this CTA's shared memory.
   __syncthreads();
-  if (*abort_flag && warp == WARPS && lane == 0) {
+  if (*abort_flag && warp == W && lane == 0) {
     tc::mbar_wait_drain(dbar, 0);
     for (int s = issued < RING ? 0 : issued - RING; s < issued; ++s)
       tc::mbar_wait_drain(&full[s % RING], (s / RING) & 1);
@@ -521,20 +530,26 @@ extern "C" int b200_trsm_leaf_pack(int dtype, const void *a, long rs_a, long cs_
 // scaled by alpha first:
 // b points at the leaf's first row in lower orientation (for an upper leaf,
 // its last row, with rs_b negated).
-template <typename T, int NCG>
+template <typename T, int NCG, int W>
 int leaf_launch(const LeafArgs<T> &la, cudaStream_t s) {
-  using L = Leaf<T, NCG>;
+  using L = Leaf<T, NCG, W>;
   static std::once_flag once;
   static int conf = B200_OK;
   B200_TRY(b200_once(once, conf, "trsm leaf kernel: set-up failed", []() -> int {
-    B200_CUDA_TRY(cudaFuncSetAttribute(trsm_leaf_kernel<T, NCG>,
+    // The register split adds up only for this allocation (an increase that cannot
+    // be granted would wait for good).
+    cudaFuncAttributes fa;
+    B200_CUDA_TRY(cudaFuncGetAttributes(&fa, trsm_leaf_kernel<T, NCG, W>));
+    if (fa.numRegs * L::THREADS < 128 * L::FEED_REGS + 32 * W * L::SOLVE_REGS)
+      return b200_set_error(B200_ECUDA, "trsm leaf kernel: unexpected register allocation");
+    B200_CUDA_TRY(cudaFuncSetAttribute(trsm_leaf_kernel<T, NCG, W>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM));
     return B200_OK;
   }));
   const long grid = b200_ceil_div(la.n, L::NBC);
   if (grid > 0x7fffffffL) return b200_set_error(B200_EINVAL, "trsm: too many right-hand sides");
   B200ProfScope prof(sizeof(T) == 4 ? "trsm_leaf_s" : "trsm_leaf_d", s);
-  trsm_leaf_kernel<T, NCG><<<(unsigned)grid, THREADS, L::SMEM, s>>>(la);
+  trsm_leaf_kernel<T, NCG, W><<<(unsigned)grid, L::THREADS, L::SMEM, s>>>(la);
   B200_LAUNCH_CHECK();
   return B200_OK;
 }
@@ -546,15 +561,16 @@ int leaf_solve(const void *pack, int rows, T *b, long rs_b, long cs_b, int n, do
   const LeafArgs<T> la{(const T *)pack, rows, b, rs_b, cs_b, n, (T)alpha, b200_device_error_word(),
                        B200_WAIT_NS};
   if constexpr (sizeof(T) == 4) {
-    return leaf_launch<T, 1>(la, s);
+    return leaf_launch<T, 1, 8>(la, s);  // 16 warps: 2-4% slower
   } else {
     // 16 columns to a CTA, or 8 where those still fit the SMs in one wave (twice
-    // the SMs on the same columns).  One leaf of 300-512 rows, us for 8 / 16 / 32
-    // columns to a CTA: n = 300 31 / 43 / 84, n = 1000 28 / 43 / 82; DTRSM calls of
-    // 1500 x 1500 304 / 280 / 397, 4096 x 4096 2680 / 2577 / 2772, 700 x 8000
-    // 329 / 307 / 326.  (Every column gets the same bits either way.)
-    if (n > 8L * b200_sm_count()) return leaf_launch<T, 2>(la, s);
-    return leaf_launch<T, 1>(la, s);
+    // the SMs on the same columns).  DTRSM calls, us for 8 columns / 16 on 8 warps /
+    // 16 on 16 warps: 500 x 300 57 / 72 / 67, 1000 x 1000 130 / 159 / 149, 1500 x
+    // 1500 300 / 279 / 263, 700 x 8000 322 / 306 / 281, 4096 x 4096 2674 / 2573 /
+    // 2501; 32 columns 82 us a leaf on 8 warps and 2734 a call on 16 (registers
+    // spill).  Every column gets the same bits in each.
+    if (n > 8L * b200_sm_count()) return leaf_launch<T, 2, 16>(la, s);
+    return leaf_launch<T, 1, 8>(la, s);
   }
 }
 
