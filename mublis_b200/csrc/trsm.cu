@@ -65,8 +65,8 @@ int leaf_order(long m, long n) {
 // executes the triangle's flops only, not the 1.25 to 2x of a product with the
 // inverse).  FP32 (us, kernel / inverse): 500 x 300 92 / 153, 1001 x 1500
 // 184 / 271, 2048 x 500 321 / 341, 3000 x 1000 605 / 663, 3500 x 3500 1304 / 1557,
-// 6000 x 2500 2389 / 2453; but 4096 x 3000 1452 / 1437, 4096 x 4096 1798 / 1752,
-// 8192 x 8192 10141 / 9498, where the products are large enough for the GEMM's
+// 6000 x 2500 2389 / 2453; but 4096 x 3000 1452 / 1437, 4096 x 4096 1686 / 1612,
+// 8192 x 8192 10130 / 9494, where the products are large enough for the GEMM's
 // rate, and 3000 x 200 451 / 395, 4096 x 300 667 / 569, 8000 x 500 1737 / 1560,
 // where a leaf is latency and all of the inverses are built at once.  n is the
 // whole call's, so that every panel of a solve takes the same leaves.
