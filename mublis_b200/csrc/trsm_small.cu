@@ -149,37 +149,101 @@ __device__ __forceinline__ void update(Block<float> &b, const float *a, const fl
   }
 }
 
-// x = inv r for the inverse of a diagonal block (zero above its diagonal), into
-// shared memory.
-__device__ __forceinline__ void solve(Block<double> &b, const double *inv, double *x) {
-  constexpr int LD = Layout<double>::XLD;
+// A diagonal block in memory: element (i, q), q < i, at a[i rs + q cs]; rows from
+// `rows` on are the identity's.
+template <typename T>
+struct DiagBlock {
+  const T *a;
+  long rs, cs;
+  int rows, unit;
+};
+
+// Forward substitution of one column (x, pitch XLD) from row `first` on.
+template <typename T>
+__device__ __forceinline__ void substitute(T *x, int first, const DiagBlock<T> &d) {
+  constexpr int LD = Layout<T>::XLD;
+#pragma unroll 1
+  for (int i = first; i < min(LB, d.rows); ++i) {
+    T s = x[i * LD];
+#pragma unroll 1
+    for (int q = 0; q < i; ++q) s = fma(-d.a[i * d.rs + q * d.cs], x[q * LD], s);
+    x[i * LD] = d.unit ? s : s * (T(1) / d.a[i * (d.rs + d.cs)]);
+  }
+}
+
+__device__ __forceinline__ void multiply(double (&c)[4][4], const double *inv, const double (&f)[4][4]) {
   const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-  b.each([&](int r, int c, double v) { x[r * LD + c] = v; });
-  __syncwarp();
-  double f[4][4];
-  load_x<double>(x, f);
-  __syncwarp();
 #pragma unroll
   for (int j = 0; j < 4; ++j)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) b.c[j][e] = 0.0;
+    for (int e = 0; e < 4; ++e) c[j][e] = 0.0;
 #pragma unroll
   for (int ks = 0; ks < 4; ++ks) {
     const double a0 = inv[Layout<double>::diag(g, 4 * ks + t)];
     const double a1 = inv[Layout<double>::diag(g + 8, 4 * ks + t)];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) dmma(b.c[j], a0, a1, f[ks][j]);
+    for (int j = 0; j < 4; ++j) dmma(c[j], a0, a1, f[ks][j]);
   }
-  b.each([&](int r, int c, double v) { x[r * LD + c] = v; });
 }
-__device__ __forceinline__ void solve(Block<float> &b, const float *inv, float *x) {
+
+// x = inv r for the inverse of a diagonal block (zero above its diagonal), into
+// shared memory.  A non-finite element of r is to reach only its own row and those
+// below, as in a substitution.  The MMAs multiply the inverse's zeros by it too and
+// spoil its whole column, which shows in any one row of the product: the high words
+// of one row's elements, as floats, add up to a NaN (a sum may be one for finite
+// elements beyond 2^1016 as well).  Then the rows before a column's first such
+// element are multiplied without it and the others substituted.  The test of a row
+// after the stores costs 0-1% of a call and 3% of a group; of all of r before them
+// it cost 3-5%.
+__device__ __forceinline__ void solve(Block<double> &b, const double *inv, double *x,
+                                      const DiagBlock<double> &d) {
+  constexpr int LD = Layout<double>::XLD;
   const int lane = threadIdx.x & 31;
-  float r[LB];
+  b.each([&](int r, int c, double v) { x[r * LD + c] = v; });
+  __syncwarp();
+  double f[4][4];
+  load_x<double>(x, f);
+  __syncwarp();
+  multiply(b.c, inv, f);
+  b.each([&](int r, int c, double v) { x[r * LD + c] = v; });
+  float row = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    row += __int_as_float(__double2hiint(b.c[j][0])) + __int_as_float(__double2hiint(b.c[j][1]));
+  if (!__any_sync(0xffffffffu, isnan(row))) return;
+  __syncwarp();
+  int first = LB;  // of column `lane`
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[(4 * ks + (lane & 3)) * LD + 8 * j + (lane >> 2)] = f[ks][j];
+  __syncwarp();
+#pragma unroll 1
+  for (int i = LB - 1; i >= 0; --i)
+    if (!isfinite(x[i * LD + lane])) first = i;
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (!isfinite(f[ks][j])) f[ks][j] = 0.0;
+  multiply(b.c, inv, f);
+  __syncwarp();
+  b.each([&](int r, int c, double v) {
+    if (r < __shfl_sync(0xffffffffu, first, c)) x[r * LD + c] = v;
+  });
+  __syncwarp();
+  substitute(x + lane, first, d);
+}
+__device__ __forceinline__ void solve(Block<float> &b, const float *inv, float *x,
+                                      const DiagBlock<float> &d) {
+  constexpr int LD = Layout<float>::XLD;
+  const int lane = threadIdx.x & 31;
+  float r[LB], s;
 #pragma unroll
   for (int i = 0; i < 8; ++i) r[2 * i] = b.c[i].x, r[2 * i + 1] = b.c[i].y;
 #pragma unroll
   for (int i = 0; i < LB; ++i) {
-    float s = 0.f;
+    s = 0.f;
 #pragma unroll
     for (int q = 0; q <= i / 4; ++q) {
       const float4 w = *(const float4 *)(inv + Layout<float>::diag(i, 4 * q));
@@ -188,8 +252,17 @@ __device__ __forceinline__ void solve(Block<float> &b, const float *inv, float *
       if (4 * q + 2 <= i) s = fmaf(w.z, r[4 * q + 2], s);
       if (4 * q + 3 <= i) s = fmaf(w.w, r[4 * q + 3], s);
     }
-    x[i * Layout<float>::XLD + lane] = s;
+    x[i * LD + lane] = s;
   }
+  if (isfinite(s)) return;
+  int first = LB;
+#pragma unroll
+  for (int i = LB - 1; i >= 0; --i)
+    if (!isfinite(r[i])) first = i;
+#pragma unroll
+  for (int i = 0; i < LB; ++i)
+    if (i >= first) x[i * LD + lane] = r[i];
+  substitute(x + lane, first, d);
 }
 
 // table may be null: then `one` is the only problem.
@@ -308,7 +381,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
         for (int i = 0; i < LB / 2; ++i)
           acc.c[i] = make_float2(rhs.c[i].x - acc.c[i].x, rhs.c[i].y - acc.c[i].y);
       }
-      solve(acc, inv + d * L::BLK, xd);
+      solve(acc, inv + d * L::BLK, xd,
+            {a0 + (long)d * LB * (ars + acs), ars, acs, m - d * LB, e.unit});
     }
     cp_wait<1>();     // segment d
     __syncthreads();  // X_d and segment d are there; every warp is done with step d - 1
