@@ -374,15 +374,56 @@ __global__ void __launch_bounds__(32 * (W + 4), 1) trsm_leaf_kernel(const __grid
       T c[1][AE];
 #pragma unroll
       for (int e = 0; e < AE; ++e) c[0][e] = T(0);
+      // The product multiplies the zeros above inv(D)'s diagonal as well: a
+      // non-finite element of R spoils its whole column, which shows in any row of
+      // it (FP64: the high words of two elements, as floats, add up to a NaN).  Then
+      // the rows before that element are formed without it, and the others by
+      // inv(D)'s lower triangle alone, as a substitution leaves them.
       if constexpr (F64) {
         double r[4];
         load_x(r, x);
         mma_block(c[0], dinv, r);
+        const float row = __int_as_float(__double2hiint(c[0][0])) + __int_as_float(__double2hiint(c[0][1]));
+        if (__any_sync(0xffffffffu, isnan(row))) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) r[i] = isfinite(r[i]) ? r[i] : 0.0;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) c[0][e] = 0.0;
+          mma_block(c[0], dinv, r);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int row = g + 8 * (e >> 1);
+            bool behind = false;
+            double sum = 0.0;
+#pragma unroll 1
+            for (int q = 0; q <= row; ++q) {  // inv(D) is in MMA fragment order
+              const double v = x[q * XLD + 2 * t + (e & 1)];
+              sum = fma(dinv[((q >> 2) * 32 + 4 * g + (q & 3)) * 2 + (e >> 1)], v, sum);
+              behind |= !isfinite(v);
+            }
+            if (behind) c[0][e] = sum;
+          }
+        }
+        __syncwarp();
+        store_tile(x, c[0]);
       } else {
         fma_blocks(One(), std::false_type(), c, &dinv, x);
+        const bool spoilt = !isfinite(c[0][0]) || !isfinite(c[0][1]) || !isfinite(c[0][2]) ||
+                            !isfinite(c[0][3]);
+        const bool any = __any_sync(0xffffffffu, spoilt);
+        __syncwarp();
+        if (!any) {
+          store_tile(x, c[0]);
+        } else {
+#pragma unroll 1
+          for (int i = LB - 1; i >= 0; --i) {  // column `lane`, in place
+            float sum = 0.f;
+#pragma unroll 1
+            for (int q = 0; q <= i; ++q) sum = fmaf(dinv[q * LB + i], x[q * XLD + lane], sum);
+            x[i * XLD + lane] = sum;
+          }
+        }
       }
-      __syncwarp();
-      store_tile(x, c[0]);
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&ready[(next % XSLOTS) * NCG + cg]);
       if constexpr (F64) {

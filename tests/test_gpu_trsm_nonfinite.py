@@ -2,7 +2,8 @@
 of one column belongs to that column's rows from j on (in the order of the solve).
 The rows before it, and every other column, keep the bits they have without it; NaN
 fills the rest, and so does Inf or NaN for an Inf.  The one-launch kernel (single and
-grouped, orders up to 256) substitutes, so Inf and NaN fall as they do row by row."""
+grouped, orders up to 256) substitutes, so there Inf and NaN fall as they do row by
+row; the leaf kernel (larger orders) applies inverted 16 x 16 blocks."""
 import ctypes
 
 import numpy as np
@@ -54,7 +55,8 @@ def by_rows(a, b, lower):
 
 @pytest.mark.parametrize("p", ["s", "d"])
 @pytest.mark.parametrize("lower", [True, False], ids=["lower", "upper"])
-@pytest.mark.parametrize("order,grouped", [(48, True), (48, False), (200, True), (200, False)])
+@pytest.mark.parametrize("order,grouped", [(48, True), (48, False), (200, True), (200, False),
+                                           (600, False)])
 def test_nonfinite_rhs_reaches_only_later_rows(lib, p, lower, order, grouped):
     pytest.importorskip("torch")
     a = orc.trsm_matrix(order, DT[p], 31, 0)
