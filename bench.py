@@ -79,7 +79,7 @@ def kernel_flops(n: int) -> dict:
     triangle (they execute 2 m b n, twice the triangle's work, which is not
     credited)."""
     gemm_part = sum(flops(r, n) for r in ROUTINES)
-    return {"simt_sgemm": gemm_part, "simt_dgemm": gemm_part, "dmma_dgemm": gemm_part}
+    return {"ffma_sgemm": gemm_part, "simt_dgemm": gemm_part, "dmma_dgemm": gemm_part}
 
 
 def max_over_ranks(dist, torch, ms: float, world: int, device: str = "cuda") -> float:

@@ -380,7 +380,7 @@ int launch_ffma_gemm(FfmaGemmArgs &a, const FfmaPolicy *pol, cudaStream_t s) {
   }
   if (st == B200_OK) {
     const long units = (long)a.ntiles * a.splits;
-    B200ProfScope prof("simt_sgemm", s);
+    B200ProfScope prof("ffma_sgemm", s);
     ffma_gemm_kernel<<<(unsigned)std::min<long>(units, sms), THREADS, SMEM, s>>>(a);
     if (cudaGetLastError() != cudaSuccess) st = b200_set_error(B200_ECUDA, "gemm: launch failed");
   }

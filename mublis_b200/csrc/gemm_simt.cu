@@ -419,7 +419,7 @@ __global__ void scale_kernel(int m, int n, T beta, T *c, long rs, long cs, int j
 // Tile configurations: (BM, BN, warps along M, warps along N, cp.async
 // stages, min CTAs per SM).  Packed panels are padded to 128 in M and N, so
 // every configuration reads the same panels.  Index 0 is the default; the
-// others are kept for tuning (MUBLIS_B200_SIMT_S / MUBLIS_B200_SIMT_D).
+// others are kept for tuning (MUBLIS_B200_SIMT_D).
 // Resident CTAs per SM of a kernel at 256 threads and `smem` bytes.
 template <typename K>
 int resident_per_sm(K kern, size_t smem) {
@@ -500,20 +500,20 @@ int launch_cfg(const SimtGemmArgs<T> &a0, cudaStream_t s, const SimtPolicy *pol)
   return st;
 }
 
-int simt_variant(bool dbl) {
-  static int v[2] = {-1, -1};
-  if (v[dbl] < 0) {
-    const char *e = getenv(dbl ? "MUBLIS_B200_SIMT_D" : "MUBLIS_B200_SIMT_S");
-    v[dbl] = e ? atoi(e) : 0;
-  }
-  return v[dbl];
+// MUBLIS_B200_SIMT_D=<1..4> selects another tile (tuning).
+int simt_variant() {
+  static const int v = [] {
+    const char *e = getenv("MUBLIS_B200_SIMT_D");
+    return e ? atoi(e) : 0;
+  }();
+  return v;
 }
 
 }  // namespace
 
 template <>
 int launch_simt_gemm<double>(const SimtGemmArgs<double> &a, cudaStream_t s, const SimtPolicy *pol) {
-  switch (simt_variant(true)) {
+  switch (simt_variant()) {
   case 1: return launch_cfg<double, 128, 64, 4, 2, 4, 1>(a, s, pol);
   case 2: return launch_cfg<double, 128, 64, 4, 2, 4, 2>(a, s, pol);
   case 3: return launch_cfg<double, 64, 128, 2, 4, 4, 2>(a, s, pol);

@@ -301,8 +301,8 @@ struct SimtConfig<double> {
   static constexpr int BM = 128, BN = 128, BK = 16;  // panel padding (tiles may be smaller)
 };
 
-// pol == nullptr: one tile per CTA, no scratch (the allocation-free entry
-// point); otherwise persistent CTAs with split-K and stream-ordered scratch.
+// pol == nullptr: one tile per CTA, no scratch; otherwise persistent CTAs with
+// split-K and stream-ordered scratch.
 template <typename T>
 int launch_simt_gemm(const SimtGemmArgs<T> &a, cudaStream_t s, const SimtPolicy *pol = nullptr);
 
