@@ -111,11 +111,20 @@ bool use_dmma() {
   return on;
 }
 
-// MUBLIS_B200_DIRECT=0 keeps the pack pass for every call.
+// MUBLIS_B200_DIRECT=0 keeps the pack pass for every call and operand;
+// MUBLIS_B200_SMALL=0 sends small products (gemm_direct.cu) to the kernels of the
+// large ones, which still read operands in place.
 bool direct_on() {
   static const bool on = [] {
     const char *e = getenv("MUBLIS_B200_DIRECT");
     return !(e && !strcmp(e, "0"));
+  }();
+  return on;
+}
+bool small_on() {
+  static const bool on = [] {
+    const char *e = getenv("MUBLIS_B200_SMALL");
+    return direct_on() && !(e && !strcmp(e, "0"));
   }();
   return on;
 }
@@ -393,7 +402,7 @@ int run_simt_dgemm(const b200_l3_desc_t *d) {
 int try_direct(const b200_l3_desc_t *d, int *status) {
   // A stall armed by mublis_b200_test_stall_next waits for the FP64
   // tensor-pipe kernel of the packed path.
-  if (!direct_on() || (d->dtype == B200_F64 && (!use_dmma() || b200_test_stall_armed()))) return 0;
+  if (!small_on() || (d->dtype == B200_F64 && (!use_dmma() || b200_test_stall_armed()))) return 0;
   const mublis_l3_product_t &pr = d->product;
   if (d->npairs == 2 &&
       (pr.a.struc != MUBLIS_STRUC_GENERAL || pr.b.struc != MUBLIS_STRUC_GENERAL ||
