@@ -110,3 +110,22 @@ def test_grouped_solve(lib, p):
     assert lib.mublis_b200_trsm_grouped(p.encode(), arr, len(probs)) == 0, mb.last_error(lib)
     for (_, b), x in zip(keep, want):
         np.testing.assert_array_equal(b.cpu().numpy().T, x)
+
+
+def test_small_solve_rounds_alpha_b_minus_the_update_once(lib):
+    """FP32, A = I with a one below the first block: x[16] = alpha b[16] - x[0]."""
+    import torch
+    order, rhs, alpha = 17, 512, np.float32(0.7)
+    rng = np.random.default_rng(5)
+    a = np.eye(order, dtype=np.float32)
+    a[16, 0] = 1
+    b = rng.uniform(0.5, 1, (order, rhs)).astype(np.float32)
+    da, db = torch.from_numpy(a.T.copy()).cuda(), torch.from_numpy(b.T.copy()).cuda()
+    torch.cuda.synchronize()
+    assert lib.mublis_strsm(0, mb.M_LOWER, 0, mb.M_NON_UNIT, order, rhs, float(alpha),
+                            ctypes.c_void_p(da.data_ptr()), 1, order,
+                            ctypes.c_void_p(db.data_ptr()), 1, order) == 0, mb.last_error(lib)
+    x = db.cpu().numpy().T
+    np.testing.assert_array_equal(x[:16], alpha * b[:16])
+    once = (np.float64(alpha) * b[16] - x[0].astype(np.float64)).astype(np.float32)
+    np.testing.assert_array_equal(x[16], once)
