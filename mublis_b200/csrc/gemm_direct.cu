@@ -243,13 +243,15 @@ __device__ __forceinline__ int block_class(const DirectOperand<T> &o, long mn0, 
 
 // PLAIN: both operands general and unmasked.  (SYR2K's two pairs are plain;
 // each pair takes whole k-blocks, the last one filled up with zeros.)
-template <typename T, int TILE, bool PLAIN>
+// FOLD: after every RUN k-blocks (128 products of a thread) the sums move to totals,
+// in registers: at most three CTAs to an SM instead of four.
+template <typename T, int TILE, bool PLAIN, bool FOLD>
 __device__ __forceinline__ void direct_tile(const DirectArgs<T> &p, const int tile, const int rank,
                                             const int S) {
   using C = DirectCfg<T, TILE>;
   constexpr bool F64 = sizeof(T) == 8;
   constexpr int BM = TILE, BN = TILE, BK = C::BK, LD = C::LD, CLD = C::CLD, STAGES = C::STAGES;
-  constexpr int NT = C::NT, GROUPS = C::GROUPS, GK = BK / GROUPS;
+  constexpr int NT = C::NT, GROUPS = C::GROUPS, GK = BK / GROUPS, RUN = B200_DIRECT_RUN / GK;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *ring = reinterpret_cast<T *>(smem_raw);
 
@@ -330,59 +332,87 @@ __device__ __forceinline__ void direct_tile(const DirectArgs<T> &p, const int ti
 #pragma unroll
       for (int j = 0; j < TN / 2; ++j) facc[i][j] = make_float2(0.f, 0.f);
   }
+  // The totals, and the step that moves the sums there.
+  float2 ftot[FOLD && !F64 ? TM : 1][FOLD && !F64 ? TN / 2 : 1];
+  double dtot[FOLD && F64 ? MI : 1][FOLD && F64 ? NI : 1][4];
+  auto fold = [&](bool first) {
+    if constexpr (FOLD && F64) {
+#pragma unroll
+      for (int i = 0; i < MI; ++i)
+#pragma unroll
+        for (int j = 0; j < NI; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            dtot[i][j][e] = first ? dacc[i][j][e] : dtot[i][j][e] + dacc[i][j][e];
+            dacc[i][j][e] = 0.0;
+          }
+    } else if constexpr (FOLD) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < TN / 2; ++j) {
+          ftot[i][j] = first ? facc[i][j] : __fadd2_rn(ftot[i][j], facc[i][j]);
+          facc[i][j] = make_float2(0.f, 0.f);
+        }
+    }
+  };
+  fold(true);
 
   int stage = 0, next = STAGES - 1;
-  for (int kt = begin; kt < end; ++kt) {
-    cp_wait<STAGES - 2>();
-    __syncthreads();
-    if (kt + STAGES - 1 < end) load_stage(next, kt + STAGES - 1);
-    cp_commit();
-    const T *As = ring + stage * C::STAGE + group * GK * LD, *Bs = As + BK * LD;
-    if (++stage == STAGES) stage = 0;
-    if (++next == STAGES) next = 0;
-    if constexpr (F64) {
+  for (int kt = begin; kt < end; fold(false)) {
+    const int run_end = FOLD ? min(end, kt + RUN) : end;
+    for (; kt < run_end; ++kt) {
+      cp_wait<STAGES - 2>();
+      __syncthreads();
+      if (kt + STAGES - 1 < end) load_stage(next, kt + STAGES - 1);
+      cp_commit();
+      const T *As = ring + stage * C::STAGE + group * GK * LD, *Bs = As + BK * LD;
+      if (++stage == STAGES) stage = 0;
+      if (++next == STAGES) next = 0;
+      if constexpr (F64) {
 #pragma unroll
-      for (int ks = 0; ks < GK / 4; ++ks) {
-        const double *ar = As + (4 * ks + t) * LD + wm * (BM / 2) + g;
-        const double *br = Bs + (4 * ks + t) * LD + wn * (BN / 2) + g;
-        double a0[MI], a1[MI], b[NI];
+        for (int ks = 0; ks < GK / 4; ++ks) {
+          const double *ar = As + (4 * ks + t) * LD + wm * (BM / 2) + g;
+          const double *br = Bs + (4 * ks + t) * LD + wn * (BN / 2) + g;
+          double a0[MI], a1[MI], b[NI];
 #pragma unroll
-        for (int i = 0; i < MI; ++i) a0[i] = ar[16 * i], a1[i] = ar[16 * i + 8];
+          for (int i = 0; i < MI; ++i) a0[i] = ar[16 * i], a1[i] = ar[16 * i + 8];
 #pragma unroll
-        for (int j = 0; j < NI; ++j) b[j] = br[8 * j];
+          for (int j = 0; j < NI; ++j) b[j] = br[8 * j];
 #pragma unroll
-        for (int i = 0; i < MI; ++i)
+          for (int i = 0; i < MI; ++i)
 #pragma unroll
-          for (int j = 0; j < NI; ++j) dmma(dacc[i][j], a0[i], a1[i], b[j]);
-      }
-    } else {
-      // Fragments one k ahead of the products that use them.
-      float a[2][TM], b[2][TN];
-      auto fragments = [&](int kk, int h) {
-#pragma unroll
-        for (int u = 0; u < TM / 4; ++u) {
-          const float4 v = *reinterpret_cast<const float4 *>(As + kk * LD + 32 * u + 4 * ty);
-          a[h][4 * u] = v.x, a[h][4 * u + 1] = v.y, a[h][4 * u + 2] = v.z, a[h][4 * u + 3] = v.w;
+            for (int j = 0; j < NI; ++j) dmma(dacc[i][j], a0[i], a1[i], b[j]);
         }
-        if constexpr (TN == 4) {
-          const float4 v = *reinterpret_cast<const float4 *>(Bs + kk * LD + 4 * tx);
-          b[h][0] = v.x, b[h][1] = v.y, b[h][2] = v.z, b[h][3] = v.w;
-        } else {
-          const float2 v = *reinterpret_cast<const float2 *>(Bs + kk * LD + 2 * tx);
-          b[h][0] = v.x, b[h][1] = v.y;
+      } else {
+        // Fragments one k ahead of the products that use them.
+        float a[2][TM], b[2][TN];
+        auto fragments = [&](int kk, int h) {
+#pragma unroll
+          for (int u = 0; u < TM / 4; ++u) {
+            const float4 v = *reinterpret_cast<const float4 *>(As + kk * LD + 32 * u + 4 * ty);
+            a[h][4 * u] = v.x, a[h][4 * u + 1] = v.y, a[h][4 * u + 2] = v.z, a[h][4 * u + 3] = v.w;
+          }
+          if constexpr (TN == 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(Bs + kk * LD + 4 * tx);
+            b[h][0] = v.x, b[h][1] = v.y, b[h][2] = v.z, b[h][3] = v.w;
+          } else {
+            const float2 v = *reinterpret_cast<const float2 *>(Bs + kk * LD + 2 * tx);
+            b[h][0] = v.x, b[h][1] = v.y;
+          }
+        };
+        fragments(0, 0);
+#pragma unroll
+        for (int kk = 0; kk < GK; ++kk) {
+          if (kk + 1 < GK) fragments(kk + 1, (kk + 1) & 1);
+          const float *af = a[kk & 1], *bf = b[kk & 1];
+#pragma unroll
+          for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j)
+              facc[i][j] = __ffma2_rn(make_float2(af[i], af[i]), make_float2(bf[2 * j], bf[2 * j + 1]),
+                                      facc[i][j]);
         }
-      };
-      fragments(0, 0);
-#pragma unroll
-      for (int kk = 0; kk < GK; ++kk) {
-        if (kk + 1 < GK) fragments(kk + 1, (kk + 1) & 1);
-        const float *af = a[kk & 1], *bf = b[kk & 1];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-          for (int j = 0; j < TN / 2; ++j)
-            facc[i][j] = __ffma2_rn(make_float2(af[i], af[i]), make_float2(bf[2 * j], bf[2 * j + 1]),
-                                    facc[i][j]);
       }
     }
   }
@@ -399,15 +429,16 @@ __device__ __forceinline__ void direct_tile(const DirectArgs<T> &p, const int ti
 #pragma unroll
         for (int e = 0; e < 4; ++e)
           Cs[(wn * (BN / 2) + 8 * j + 2 * t + (e & 1)) * CLD + wm * (BM / 2) + 16 * i + g +
-             8 * (e >> 1)] = dacc[i][j][e];
+             8 * (e >> 1)] = FOLD ? dtot[FOLD ? i : 0][FOLD ? j : 0][e] : dacc[i][j][e];
   } else {
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN / 2; ++j) {
         const int r = 32 * (i / 4) + 4 * ty + i % 4;
-        Cs[(TN * tx + 2 * j) * CLD + r] = facc[i][j].x;
-        Cs[(TN * tx + 2 * j + 1) * CLD + r] = facc[i][j].y;
+        const float2 v = FOLD ? ftot[FOLD ? i : 0][FOLD ? j : 0] : facc[i][j];
+        Cs[(TN * tx + 2 * j) * CLD + r] = v.x;
+        Cs[(TN * tx + 2 * j + 1) * CLD + r] = v.y;
       }
   }
   if (S > 1) cluster_barrier();
@@ -464,10 +495,10 @@ __device__ __forceinline__ void direct_tile(const DirectArgs<T> &p, const int ti
   if (S > 1) cluster_barrier();  // no CTA leaves while another reads its sums
 }
 
-template <typename T, int TILE, bool PLAIN>
-__global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, TILE == 32 && !PLAIN ? 3 : 4)
+template <typename T, int TILE, bool PLAIN, bool FOLD>
+__global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, TILE == 32 && !PLAIN && FOLD ? 2 : (TILE == 32 && !PLAIN) || FOLD ? 3 : 4)
     direct_gemm_kernel(const __grid_constant__ DirectArgs<T> p) {
-  direct_tile<T, TILE, PLAIN>(p, blockIdx.x / p.splits, blockIdx.x % p.splits, p.splits);
+  direct_tile<T, TILE, PLAIN, FOLD>(p, blockIdx.x / p.splits, blockIdx.x % p.splits, p.splits);
 }
 
 // Many independent products: CTA b computes tile b of the group, of problem
@@ -496,13 +527,13 @@ __global__ void __launch_bounds__(DirectCfg<T, TILE>::NT, 4)
   p.alpha = (T)e.alpha;
   p.beta = (T)e.beta;
   p.jp = p.ji = p.pi = MUBLIS_L3_ALL;
-  direct_tile<T, TILE, true>(p, blockIdx.x - e.tile0, 0, 1);
+  direct_tile<T, TILE, true, false>(p, blockIdx.x - e.tile0, 0, 1);
 }
 
-template <typename T, int TILE, bool PLAIN>
+template <typename T, int TILE, bool PLAIN, bool FOLD>
 int launch_tile(DirectArgs<T> &p, cudaStream_t s) {
   using C = DirectCfg<T, TILE>;
-  auto kern = direct_gemm_kernel<T, TILE, PLAIN>;
+  auto kern = direct_gemm_kernel<T, TILE, PLAIN, FOLD>;
   static std::once_flag once;
   static int conf = B200_OK;
   B200_TRY(b200_once(once, conf, "direct gemm: set-up failed", [&]() -> int {
@@ -530,6 +561,12 @@ int launch_tile(DirectArgs<T> &p, cudaStream_t s) {
   B200ProfScope prof(sizeof(T) == 4 ? "direct_sgemm" : "direct_dgemm", s);
   B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const DirectArgs<T> &)p));
   return B200_OK;
+}
+
+template <typename T, int TILE>
+int launch_tile(DirectArgs<T> &p, bool plain, bool fold, cudaStream_t s) {
+  if (fold) return plain ? launch_tile<T, TILE, true, true>(p, s) : launch_tile<T, TILE, false, true>(p, s);
+  return plain ? launch_tile<T, TILE, true, false>(p, s) : launch_tile<T, TILE, false, false>(p, s);
 }
 
 template <typename T>
@@ -578,9 +615,7 @@ int run_direct(const b200_l3_desc_t *d, const b200_direct_choice_t &ch) {
   cudaStream_t s = b200_cur_stream();
   const bool plain = p.a.plain && p.b.plain;
   if (!plain && d->npairs != 1) return b200_set_error(B200_EINVAL, "direct gemm: structured pairs");
-  if (ch.tile == 64)
-    return plain ? launch_tile<T, 64, true>(p, s) : launch_tile<T, 64, false>(p, s);
-  return plain ? launch_tile<T, 32, true>(p, s) : launch_tile<T, 32, false>(p, s);
+  return ch.tile == 64 ? launch_tile<T, 64>(p, plain, ch.fold, s) : launch_tile<T, 32>(p, plain, ch.fold, s);
 }
 
 template <typename T, int TILE>
@@ -658,7 +693,8 @@ b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d) {
     const double waves = std::ceil(std::ceil(m / 128) * std::ceil(n / 128) / sms);
     best = std::min(best, 47.0 + waves * (std::ceil(k / 16) * 1.28 + 4.0));
   }
-  b200_direct_choice_t ch = {0, 1};
+  b200_direct_choice_t ch = {0, 1, 0};
+  long run = 0;  // products that a thread adds in a row
   for (int big = 0; big < 2; ++big) {
     const Cost &c = cost[f64][big];
     const double tile = big ? 64 : 32, bk = big ? 16 : 32;
@@ -666,19 +702,29 @@ b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d) {
     for (int S = 1; S <= 8; S *= 2) {
       const double kb = std::ceil(std::ceil(k / bk) / S);
       if (S > 1 && kb < 2) break;
-      // FP32 sums stay as short as the packed path's split-K keeps them: at
-      // most 1024 products in a row (two thread groups at tile 32), while
-      // more CTAs can be had.
-      if (!f64 && S < 8 && kb * bk > (big ? 1024 : 2048)) continue;
       const double per_sm = std::ceil(tiles * S / sms);
       const double t = c.start + kb * (tri_k < 1 && per_sm > 2 ? 0.6 : 1.0) *
                                      std::max(c.alone, per_sm * c.shared) +
                        (per_sm - 1) * (S == 1 ? c.next1 : c.next);
       if (t < best) {
         best = t;
-        ch = {big ? 64 : 32, S};
+        ch = {big ? 64 : 32, S, 0};
+        run = (long)kb * 16;  // of each k-block, 16 to a thread
       }
     }
+  }
+  // Sums are to be no longer than under the packed path's split-K when that ran on
+  // every SM's 1 (FP64) or 2 (FP32) CTAs, and in FP32 no longer than 1024: above
+  // that they are folded.  Normwise error and us of FP32 696 x 389 x 1855, k cut in
+  // 12 there, in 2 here: 2.4e-7 packed; 5.5e-7 and 65.6 in one sum, 2.1e-7 and 68.5
+  // folded; 1236 x 788 x 1005 2.9e-7; 5.7e-7 and 85.8, 2.1e-7 and 83.2; FP64 254 x
+  // 1050 x 1370 1.3e-15; 1.4e-15 and 56.3, 1.3e-15 and 54.8.  With four or more CTAs
+  // to an SM folding takes 3-9% (360 x 1411 x 2847 114 -> 126; packed 170).
+  if (ch.tile && run > B200_DIRECT_RUN) {
+    const int cut = b200_split_for((long)m, (long)n, (long)k, 128, 128, 16, {dom.jp, dom.ji, dom.pi},
+                                   f64 ? (long)sms : 2 * (long)sms, f64 ? 8.0 : 4.0);
+    const long chunk = b200_ceil_div(b200_ceil_div((long)k, 16), cut) * 16;
+    ch.fold = run > (f64 ? chunk : std::min(chunk, 1024L));
   }
   return ch;
 }

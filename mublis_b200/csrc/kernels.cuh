@@ -339,10 +339,12 @@ int b200_split_for(long m_full, long n_full, long k, int BM, int BN, int BK,
 
 // ---- small products in one launch (gemm_direct.cu)
 
-// How a product runs there: tile 64 or 32 (0: not there), and how many CTAs
-// share a tile's k range.
+// How a product runs there: tile 64 or 32 (0: not there), how many CTAs share a
+// tile's k range, and whether sums are folded into totals every B200_DIRECT_RUN
+// products.
+constexpr int B200_DIRECT_RUN = 128;
 struct b200_direct_choice_t {
-  int tile, splits;
+  int tile, splits, fold;
 };
 b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d);
 // On the calling thread's stream; C must overlap no operand.
