@@ -80,6 +80,15 @@ __device__ __forceinline__ void unit_range(const FfmaGemmArgs &p, int tm, int tn
   kt1 = min(t1, kt0 + per);
 }
 
+// How many k-blocks of a tile are added in a row.  (Formed anew at each use: held
+// through the main loop it took 1% of every call.)
+__device__ __forceinline__ int run_blocks(const FfmaGemmArgs &p, int tm, int tn) {
+  if (p.runs == 1) return p.fold;
+  int t0, t1;
+  unit_range(p, tm, tn, 0, 1, t0, t1);
+  return min(p.fold, (t1 - t0 + p.runs - 1) / p.runs);
+}
+
 __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_constant__ FfmaGemmArgs p) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *ring = (float *)smem_raw;
@@ -157,7 +166,7 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
 #pragma unroll
       for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
     for (int k0 = kt0, k1; k0 < kt1; k0 = k1) {
-      k1 = k0 + min(kt1 - k0, p.fold);
+      k1 = k0 + min(kt1 - k0, run_blocks(p, tm, tn));
       for (int kt = k0; kt < k1; ++kt) {
         const int wok = tc::mbar_wait(&full[stage], phase, abort_flag, p.err);
         if (!__all_sync(0xffffffffu, wok)) return;
@@ -193,7 +202,7 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
         if (lane == 0) tc::mbar_arrive(&empty[stage]);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
-      // Every p.fold k-blocks the sums move to a total in shared memory (a
+      // After each run of k-blocks the sums move to a total in shared memory (a
       // thread's own words).
       if (k1 < kt1) {
         const bool first = k0 == kt0;
@@ -209,7 +218,7 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
           }
       }
     }
-    if (kt1 - kt0 > p.fold) {
+    if (kt1 - kt0 > run_blocks(p, tm, tn)) {
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -355,12 +364,16 @@ int launch_ffma_gemm(FfmaGemmArgs &a, const FfmaPolicy *pol, cudaStream_t s) {
   // 6 447; 2048^3: 1 336, 2 364, 4 355.
   constexpr double SPLIT_COST = 4.0;
   a.splits = pol ? b200_split_for(pol->m_full, pol->n_full, a.k, BM, BN, BK, dom, sms, SPLIT_COST) : 1;
-  // Below 1024 tiles a sum is folded into a total every 1024 k: the split-K of
-  // smaller calls (chunks of a few hundred k) gives way to this kernel's full
-  // rate at one tile per SM, and their sums are to stay as short (1500 x 1500 x
-  // 3000: relative error 6e-7, 1e-6 without; 0.5% of the time).
+  // Sums are folded into a total where they would grow longer than the chunks into
+  // which split-K cuts k for two CTAs per SM (the two that this kernel's full rate at
+  // one tile per SM replaces; PAIR_COST: what a split unit cost them), and below
+  // 1024 tiles every 1024 k as well.  Normwise error and us, in runs of 1024 and in
+  // those chunks: 2000 x 2587 x 1300 (chunks of 336) 5.3e-7, 343; 3.3e-7, 346;
+  // 4096 x 4096 x 8192 (4096) 1.6e-6, 4272; 1.1e-6, 4321.
+  constexpr double PAIR_COST = 4.0;
   const long m_full = pol ? pol->m_full : a.m, n_full = pol ? pol->n_full : a.n;
   a.fold = b200_ceil_div(m_full, BM) * b200_ceil_div(n_full, BN) < 1024 ? 1024 / BK : 0x7fffffff;
+  a.runs = pol ? b200_split_for(m_full, n_full, a.k, BM, BN, BK, dom, 2 * sms, PAIR_COST) : 1;
   const size_t list_bytes = list.empty() || a.listed ? 0 : sizeof(int2) * list.size();
   const size_t off_arr = b200_round_up((long)list_bytes, 256);
   const size_t arr_bytes = a.splits > 1 ? sizeof(int) * a.ntiles * CONSUMERS : 0;

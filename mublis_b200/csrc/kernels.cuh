@@ -243,7 +243,8 @@ struct FfmaGemmArgs {
   // Filled by the launcher.
   int *err = nullptr;
   int tiles_m = 0, tiles_n = 0, ntiles = 0, splits = 1, listed = 0;
-  int fold = 0x7fffffff;  // k-blocks added in a row
+  int fold = 0x7fffffff;  // k-blocks added in a row, at most,
+  int runs = 1;           // and at most this share of a tile's
   const int2 *tile_list = nullptr;
   int *arrivals = nullptr;    // per (tile, warp): k-chunks finished, splits > 1
   float *partials = nullptr;  // per unit: its k-chunk's sums, splits > 1

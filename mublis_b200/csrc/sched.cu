@@ -143,6 +143,11 @@ int b200_split_for(long m_full, long n_full, long k, int BM, int BN, int BK,
         units.push_back(len + UNIT_COST + (S > 1 ? split_cost : 0.0));
       }
     }
+    // No schedule ends before its mean load: most S are out without simulating them
+    // (the FP32 kernel asks twice for every new shape).
+    double load = 0;
+    for (double c : units) load += c;
+    if (S > 1 && load / slots >= std::min(SPLIT_GAIN * t1, best_t)) continue;
     const double t = simulate(units, slots);
     if (S == 1) {
       t1 = t;

@@ -33,7 +33,10 @@ SMALL = [("s", 696, 389, 1855, 160), ("s", 1794, 151, 1863, 208), ("s", 677, 327
          ("s", 1236, 788, 1005, 256), ("d", 254, 1050, 1370, 176), ("d", 1180, 300, 1500, 304)]
 
 
-@pytest.mark.parametrize("p,m,n,k,chunk", SMALL)
+LARGE = [("s", 2000, 2587, 1300, 336), ("s", 1660, 2849, 901, 240), ("s", 197, 4081, 1805, 464)]
+
+
+@pytest.mark.parametrize("p,m,n,k,chunk", SMALL + LARGE)
 def test_sums_are_as_short_as_split_k_made_them(lib, p, m, n, k, chunk):
     torch = pytest.importorskip("torch")
     assert lib.mublis_b200_init() == 0, mb.last_error(lib)
