@@ -39,7 +39,7 @@ constexpr int WM = 4, WN = 2, CONSUMERS = WM * WN, THREADS = (CONSUMERS + 1) * 3
 constexpr int WTM = BM / WM, WTN = BN / WN, TM = WTM / 4, TN = WTN / 8;
 constexpr int STAGE = (BM + BN) * BK;  // floats
 constexpr int SUMS = TM * TN * CONSUMERS * 32;  // a tile's sums
-constexpr int SMEM = (STAGES * STAGE + SUMS) * 4 + 2 * STAGES * 8 + 16;
+constexpr int SMEM = (STAGES * STAGE + 2 * SUMS) * 4 + 2 * STAGES * 8 + 16;
 
 __device__ __forceinline__ void tile_coords(const FfmaGemmArgs &p, int idx, int &tm, int &tn) {
   if (p.listed) {
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float *ring = (float *)smem_raw;
   float4 *folded = (float4 *)(ring + STAGES * STAGE);  // [TM * TN / 4][256 threads]
-  uint64_t *full = (uint64_t *)(folded + SUMS / 4);
+  uint64_t *full = (uint64_t *)(ring + STAGES * STAGE + 2 * SUMS);  // (behind the staged sums)
   uint64_t *empty = full + STAGES;
   volatile int *abort_flag = (volatile int *)(empty + STAGES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -305,25 +305,66 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
       }
       continue;
     }
+    // Otherwise (edges, diagonals, lines off 16 bytes) through the warp's own 32 x 64
+    // floats of shared memory, so that its lanes run along C's smaller stride, 16
+    // lines' loads before their stores.  Nothing else runs on the SM meanwhile: with
+    // 4-byte accesses at the accumulators' places a tile's epilogue took about 9 us,
+    // and 512 x 20000 x 512 with odd leading dimensions 311 us (260 so), 1000 x
+    // 20000 x 200 310 (222), 967 x 2695 x 1123 207 (183).  alpha goes in here because
+    // the products' own registers must not be tied to the float4 stores: the main loop
+    // lost 1.5% to that.
+    uint32_t id;  // (threadIdx.x, but not held through the main loop)
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(id));
+    float *stage_c = ring + STAGES * STAGE + SUMS + (id >> 5) * (WTM * WTN);
+    const int l = id & 31, row4 = l >> 3, col4 = l & 7;  // ty, tx
+    const bool m_fast = labs(p.rs_c) <= labs(p.cs_c);
+    if (m_fast) {  // [column][row], a column's groups of 4 rows XORed with column / 4
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const long gi = m0 + 16 * (i >> 2) + (i & 3);
-      if (gi >= p.m) continue;
-      float cv[TN];
+      for (int q = 0; q < 2; ++q)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const long gj = n0 + 32 * (j >> 2) + (j & 3);
-        cv[j] = beta != 0.f && gj < p.n && b200_rel(p.ji, gj, gi) ? p.c[gi * p.rs_c + gj * p.cs_c] : 0.f;
+        for (int x = 0; x < 8; ++x)
+          *(float4 *)(stage_c + (32 * (x >> 2) + 4 * col4 + (x & 3)) * WTM + ((4 * q + row4) ^ col4) * 4) =
+              make_float4(alpha * sum(4 * q, x), alpha * sum(4 * q + 1, x), alpha * sum(4 * q + 2, x),
+                          alpha * sum(4 * q + 3, x));
+    } else {  // [row][column]
+#pragma unroll
+      for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+          *(float4 *)(stage_c + (16 * (i >> 2) + 4 * row4 + (i & 3)) * WTN + 32 * q + 4 * col4) =
+              make_float4(alpha * sum(i, 4 * q), alpha * sum(i, 4 * q + 1), alpha * sum(i, 4 * q + 2),
+                          alpha * sum(i, 4 * q + 3));
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int h = 0; h < 4; ++h) {
+      // Element y of a lane: row l, column 16 h + y, or row y + 16 (h & 1), column
+      // 32 (h >> 1) + l.
+      const long gi0 = (long)tm * BM + (id >> 5) % WM * WTM + (m_fast ? l : 16 * (h & 1));
+      const long gj0 = (long)tn * BN + (id >> 5) / WM * WTN + (m_fast ? 16 * h : 32 * (h >> 1) + l);
+      float *line = p.c + gi0 * p.rs_c + gj0 * p.cs_c;
+      const long step = m_fast ? p.cs_c : p.rs_c;
+      const long left = m_fast ? (gi0 < p.m ? p.n - gj0 : 0) : (gj0 < p.n ? p.m - gi0 : 0);
+      // The lane's elements y that are written: those up to (from) the diagonal.
+      int y0 = 0, y1 = (int)min(left, 16L);
+      if (p.ji != MUBLIS_L3_ALL) {
+        const long d = m_fast ? gi0 - gj0 : gj0 - gi0;
+        const bool upto = (p.ji == MUBLIS_L3_LOWER) == m_fast;
+        if (upto) y1 = (int)min((long)y1, d + 1);
+        else y0 = (int)max(0L, min(d, 16L));
       }
+      float cv[16];
 #pragma unroll
-      for (int j = 0; j < TN; ++j) {
-        const long gj = n0 + 32 * (j >> 2) + (j & 3);
-        if (gj >= p.n || !b200_rel(p.ji, gj, gi)) continue;
-        float v = alpha * sum(i, j);
-        if (beta != 0.f) v = fmaf(beta, cv[j], v);
-        p.c[gi * p.rs_c + gj * p.cs_c] = v;
+      for (int y = 0; y < 16; ++y) cv[y] = beta != 0.f && y >= y0 && y < y1 ? line[y * step] : 0.f;
+#pragma unroll
+      for (int y = 0; y < 16; ++y) {
+        float v = m_fast ? stage_c[(16 * h + y) * WTM + ((l >> 2) ^ ((4 * h + (y >> 2)) & 7)) * 4 + (l & 3)]
+                         : stage_c[(y + 16 * (h & 1)) * WTN + 32 * (h >> 1) + l];
+        if (beta != 0.f) v = fmaf(beta, cv[y], v);
+        if (y >= y0 && y < y1) line[y * step] = v;
       }
     }
+    __syncwarp();  // before the next tile's sums
   }
 }
 

@@ -104,8 +104,8 @@ __device__ __forceinline__ void bulk_load_1d(void *smem_dst, const void *gsrc, u
 }
 
 // One thread: asks for the tile of C that starts at (m0, n0) in L2, line by line
-// along C's unit stride (lines that start on 16 bytes; others are left), so
-// that the epilogue's reads of C find it there instead of in HBM.
+// along C's unit stride (the whole 16-byte pieces of each), so that the
+// epilogue's reads of C find it there instead of in HBM.
 template <typename T>
 __device__ __forceinline__ void prefetch_tile_l2(const T *c, long rs, long cs, int m, int n, int m0,
                                                  int n0, int tile) {
@@ -114,10 +114,13 @@ __device__ __forceinline__ void prefetch_tile_l2(const T *c, long rs, long cs, i
   const long ld = rows ? cs : rs;
   const T *base = c + m0 * rs + n0 * cs;
   const int len = min(tile, rows ? m - m0 : n - n0), lines = min(tile, rows ? n - n0 : m - m0);
-  const uint32_t bytes = (uint32_t)(len * sizeof(T)) & ~15u;
-  if (((uintptr_t)base & 15) != 0 || (ld * (long)sizeof(T)) % 16 != 0 || bytes == 0) return;
-  for (int i = 0; i < lines; ++i)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(base + i * ld), "r"(bytes)
+  uint64_t at = (uint64_t)(uintptr_t)base;
+  const uint64_t step = (uint64_t)(ld * (long)sizeof(T));
+  const int bytes = ((int)(len * sizeof(T)) - (((at | step) & 15) != 0 ? 15 : 0)) & ~15;
+  if (bytes <= 0) return;
+  // (Few instructions a line: the thread has loads to issue, four k-blocks ahead.)
+  for (int i = 0; i < lines; ++i, at += step)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"((at + 15) & ~(uint64_t)15), "r"(bytes)
                  : "memory");
 }
 
