@@ -14,7 +14,7 @@
 // What bounds it: latency (the call's launch and wait, 12.5 us on this host;
 // one round trip for the operands, one for C) for the smallest calls,
 // shared-memory and FMA issue for the larger ones: 64^3 SGEMM 40 -> 16 us a
-// call, 301 x 177 x 211 DGEMM 79 -> 18, 1024^3 SGEMM 121 -> 75 (28 TF/s).
+// call, 301 x 177 x 211 DGEMM 79 -> 18, 512^3 SGEMM 86 -> 29.
 //   * FP32: 8 x 4 (4 x 2) accumulators per thread as packed column pairs
 //     (__ffma2_rn, each half a correctly rounded fmaf).
 //   * FP64: m16n8k4 .f64 MMAs, a 32 x 32 (16 x 16) block per warp.  The
@@ -657,59 +657,85 @@ int launch_direct_group(int dtype, int tile, const b200_group_gemm_t *table, con
 }
 
 // Which calls run here, and how: the least of the estimates below, in us, from
-// the whole call's shape (a column panel of a larger call carries the call's m
-// and n, so every panel runs as the whole call would).
+// the whole call's shape and structure (a column panel of a larger call carries
+// the call's m and n, so every panel runs as the whole call would; strides and
+// alignment differ between a panel and its call and are left out).
 //
-// Direct: with n CTAs on the fullest SM and kb k-blocks per CTA,
+// Direct, with n CTAs on the fullest SM and kb k-blocks per CTA:
 //   start + kb * max(alone, n * shared) + (n - 1) * next
-// -- alone / shared: a k-block of a CTA that has the SM to itself / of one
-// that shares it; next: filling and draining one more CTA.  Packed: start plus
-// the flops at the 128 x 128 kernels' rate; an FP32 call whose tiles fill their
-// last wave does better, 27 + waves * (1.28 a k-block + 4), and is sent there
-// when that wins by 20 (operands off 16 bytes are packed for about as much):
-// 1536^3, 144 tiles on 148 SMs, 201 -> 147, 1535^3 216 -> 163, 1408 x 1536 x 900
-// 132 -> 99.  Fitted to timings of both over
-// 16^3 .. 1536^3 and ragged shapes, e.g. (FP32 packed -> direct) 64^3 40 -> 16,
-// 512^3 85 -> 25, 1024^3 121 -> 75, 64 x 64 x 4096 139 -> 23,
-// 300 x 300 x 4096 145 -> 48, 100 x 3000 x 700 84 -> 35; (FP64) 301 x 177 x 211
-// 79 -> 18, 1024^3 127 -> 98, 1536^3 243 -> 255.
+// -- alone / shared: a k-block of a CTA that has the SM to itself / of one that
+// shares it; next: filling and draining one more CTA; a triangle of C leaves half
+// of the CTAs without work, but evens out only where an SM gets many.  Packed:
+// start, the packs by the operands' size, and the rounds of 128 x 128 tiles, k cut
+// into the best number of chunks.
+//
+// The constants are those that choose best among packed and both tiles at S = 1, 2,
+// 4, 8, all nine timed on 566 calls (GEMM, SYMM, SYRK, SYR2K, TRMM; m, n, k 16 ..
+// 4096, widths to 80000, k to 100000): the choice costs 0.8% (FP64 1.2%) more than
+// the best of the nine on average.  Estimating the packed path by its rate alone
+// sent these the slower way (us, then -> now): STRMM 256 x 40000 325 -> 153 and
+// 512 x 10000 207 -> 112, SSYMM 256 x 20000 150 -> 104, SSYRK n = 2048, k = 512
+// 83 -> 60, SGEMM 512 x 512 x 8192 158 -> 109 and 1024^3 84 -> 73 (packed); 64 x 64
+// x 65536 FP32 351 -> 165 and FP64 622 -> 168, DGEMM 1719 x 1427 x 1060 341 -> 214
+// (direct).
 b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d) {
-  struct Cost {
+  struct Direct {
     double start, alone, shared, next1, next;  // next1: S = 1
   };
-  static const Cost cost[2][2] = {{{15.5, 0.45, 0.33, 0.4, 1.0}, {18.0, 0.57, 0.46, 0.8, 1.0}},
-                                  {{15.5, 0.53, 0.35, 0.4, 2.0}, {18.5, 0.86, 0.62, 0.8, 1.5}}};
+  struct Packed {
+    double start, packs, per_mb, structured_mb, block, tile, split;
+  };
+  // [FP64][general, symmetric, triangular or masked][tile 64]
+  static const Direct cost[2][3][2] = {{{{13.5, 0.67, 0.44, 0.75, 0.97}, {18.3, 0.79, 0.45, 2.19, 2.00}},
+                                        {{15.5, 0.97, 0.59, 1.46, 1.75}, {26.7, 1.01, 0.65, 2.00, 2.54}},
+                                        {{30.8, 0.75, 0.28, 2.76, 2.42}, {47.9, 0.75, 0.40, 6.01, 3.13}}},
+                                       {{{14.1, 0.86, 0.41, 1.01, 1.92}, {19.1, 0.98, 0.57, 2.02, 2.30}},
+                                        {{15.3, 0.90, 0.61, 0.91, 1.92}, {26.8, 1.17, 0.86, 5.21, 2.89}},
+                                        {{31.9, 0.75, 0.44, 2.27, 2.04}, {47.3, 1.29, 0.50, 8.91, 2.70}}}};
+  static const Packed packed_cost[2] = {{27.5, 7.2, 0.38, 0.35, 1.03, 4.3, 4.0},
+                                        {27.5, 12.7, 0.57, 0.25, 1.81, 4.0, 18.2}};
   const bool f64 = d->dtype == B200_F64;
-  const double m = (double)(d->policy_m > 0 ? d->policy_m : d->m);
-  const double n = (double)(d->policy_n > 0 ? d->policy_n : d->n);
-  const double k = (double)d->k * d->npairs, sms = b200_sm_count();
-  const mublis_l3_domain_t &dom = d->product.domain;
-  // Triangles halve the tiles (ji) or the k ranges (jp, pi).
-  const double tri_c = dom.ji != MUBLIS_L3_ALL ? 0.5 : 1.0;
-  const double tri_k = dom.jp != MUBLIS_L3_ALL || dom.pi != MUBLIS_L3_ALL ? 0.5 : 1.0;
-  const double flops = 2 * m * n * k * tri_c * tri_k;
-  double best = f64 ? 60.0 + 0.85e6 * flops / 34e12 : 60.0 + 1.2e6 * flops / 61e12;
-  if (!f64 && tri_c == 1.0 && tri_k == 1.0) {
-    const double waves = std::ceil(std::ceil(m / 128) * std::ceil(n / 128) / sms);
-    best = std::min(best, 47.0 + waves * (std::ceil(k / 16) * 1.28 + 4.0));
+  const long m = d->policy_m > 0 ? d->policy_m : d->m, n = d->policy_n > 0 ? d->policy_n : d->n;
+  const long k = (long)d->k * d->npairs, sms = b200_sm_count();
+  const mublis_l3_product_t &pr = d->product;
+  const mublis_l3_domain_t &dom = pr.domain;
+  const bool half_c = dom.ji != MUBLIS_L3_ALL, half_k = dom.jp != MUBLIS_L3_ALL || dom.pi != MUBLIS_L3_ALL;
+  const bool triangular = half_k || pr.a.struc == MUBLIS_STRUC_TRIANGULAR || pr.b.struc == MUBLIS_STRUC_TRIANGULAR;
+  const int kind = triangular ? 2
+                   : pr.a.struc != MUBLIS_STRUC_GENERAL || pr.b.struc != MUBLIS_STRUC_GENERAL ? 1
+                                                                                             : 0;
+  const Packed &q = packed_cost[f64];
+  const long tm = b200_ceil_div(m, 128), tn = b200_ceil_div(n, 128);
+  const double tiles = half_c ? ((double)tm * tn + std::min(tm, tn)) / 2 : (double)tm * tn;
+  const long blocks = b200_ceil_div(k, 16);
+  double best = 1e30;
+  for (int S = 1; S == 1 || (S <= 16 && blocks / S >= 8); ++S) {
+    const double kb = (double)b200_ceil_div(blocks, S), unit = q.tile + (S > 1 ? q.split : 0.0);
+    const double rounds = tiles * S / sms;
+    best = std::min(best, half_k ? std::max(kb * q.block + unit, 1.05 * rounds * (0.5 * kb * q.block + unit))
+                                 : std::ceil(rounds) * (kb * q.block + unit));
   }
+  // Operands that are certain to be packed: a structured one, or a SYR2K's four whose
+  // pairs do not meet on a k-block.
+  const double mb = (f64 ? 8e-6 : 4e-6) * k;
+  best += q.start + q.packs * (kind ? 1 : d->npairs == 2 && d->k % 16 ? 2 : 0) + q.per_mb * mb * (m + n) +
+          (kind ? q.structured_mb * mb * k : 0.0);
+
   b200_direct_choice_t ch = {0, 1, 0};
   long run = 0;  // products that a thread adds in a row
   for (int big = 0; big < 2; ++big) {
-    const Cost &c = cost[f64][big];
-    const double tile = big ? 64 : 32, bk = big ? 16 : 32;
-    const double tiles = std::ceil(m / tile) * std::ceil(n / tile) * tri_c;
+    const Direct &c = cost[f64][kind][big];
+    const long tile = big ? 64 : 32, bk = big ? 16 : 32;
+    const double ctas = (double)b200_ceil_div(m, tile) * b200_ceil_div(n, tile);
     for (int S = 1; S <= 8; S *= 2) {
-      const double kb = std::ceil(std::ceil(k / bk) / S);
+      const long kb = b200_ceil_div(b200_ceil_div(k, bk), S);
       if (S > 1 && kb < 2) break;
-      const double per_sm = std::ceil(tiles * S / sms);
-      const double t = c.start + kb * (tri_k < 1 && per_sm > 2 ? 0.6 : 1.0) *
-                                     std::max(c.alone, per_sm * c.shared) +
-                       (per_sm - 1) * (S == 1 ? c.next1 : c.next);
+      const double mean = ctas * S / sms, per_sm = std::ceil(half_c && mean > 3 ? 0.5 * mean + 1.5 : mean);
+      const double t = c.start + kb * std::max(c.alone, per_sm * c.shared) + (per_sm - 1) * (S == 1 ? c.next1 : c.next);
       if (t < best) {
         best = t;
         ch = {big ? 64 : 32, S, 0};
-        run = (long)kb * 16;  // of each k-block, 16 to a thread
+        run = kb * 16;  // of each k-block, 16 to a thread
       }
     }
   }
@@ -721,9 +747,9 @@ b200_direct_choice_t b200_direct_choice(const b200_l3_desc_t *d) {
   // 1050 x 1370 1.3e-15; 1.4e-15 and 56.3, 1.3e-15 and 54.8.  With four or more CTAs
   // to an SM folding takes 3-9% (360 x 1411 x 2847 114 -> 126; packed 170).
   if (ch.tile && run > B200_DIRECT_RUN) {
-    const int cut = b200_split_for((long)m, (long)n, (long)k, 128, 128, 16, {dom.jp, dom.ji, dom.pi},
-                                   f64 ? (long)sms : 2 * (long)sms, f64 ? 8.0 : 4.0);
-    const long chunk = b200_ceil_div(b200_ceil_div((long)k, 16), cut) * 16;
+    const int cut = b200_split_for(m, n, k, 128, 128, 16, {dom.jp, dom.ji, dom.pi}, f64 ? sms : 2 * sms,
+                                   f64 ? 8.0 : 4.0);
+    const long chunk = b200_ceil_div(blocks, cut) * 16;
     ch.fold = run > (f64 ? chunk : std::min(chunk, 1024L));
   }
   return ch;

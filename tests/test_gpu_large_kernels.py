@@ -98,13 +98,13 @@ TRANS = list(itertools.product((False, True), repeat=2))
 @pytest.mark.parametrize("ta,tb", TRANS)
 @pytest.mark.parametrize("pads", [(0, 0, 0), (1, 1, 1), (0, 1, 1), (1, 0, 0)])
 def test_gemm(lib, p, ta, tb, pads):
-    gemm(lib, p, 1601, 1447, 1333, ta, tb, pads)
+    gemm(lib, p, 3001, 2847, 1333, ta, tb, pads)
 
 
 @pytest.mark.parametrize("p", ["s", "d"])
 @pytest.mark.parametrize("order,corder,shift", [("C", "C", 0), ("F", "C", 0), ("C", "F", 0), ("F", "F", 1)])
 def test_gemm_layouts(lib, p, order, corder, shift):
-    gemm(lib, p, 1700, 1531, 1285, False, True, (0, 0, 0), order, corder, shift)
+    gemm(lib, p, 2700, 2531, 1285, False, True, (0, 0, 0), order, corder, shift)
 
 
 def rank(lib, p, routine, n, k, uplo, trans, pad, kernel=KERNEL):
@@ -130,7 +130,7 @@ def rank(lib, p, routine, n, k, uplo, trans, pad, kernel=KERNEL):
                                                  ("syr2k", 672, False, 0), ("syr2k", 672, True, 0),
                                                  ("syr2k", 667, False, 0), ("syr2k", 672, False, 1)])
 def test_triangular_outputs(lib, p, uplo, routine, k, trans, pad):
-    rank(lib, p, routine, 2601, k, uplo, trans, pad)
+    rank(lib, p, routine, 3601, k, uplo, trans, pad)
 
 
 # More than 1024 tiles of the triangle: the list is uploaded.
