@@ -68,8 +68,12 @@ int leaf_order(long m, long n) {
 // 6000 x 2500 2389 / 2453; but 4096 x 3000 1452 / 1437, 4096 x 4096 1686 / 1612,
 // 8192 x 8192 10130 / 9494, where the products are large enough for the GEMM's
 // rate, and 3000 x 200 451 / 395, 4096 x 300 667 / 569, 8000 x 500 1737 / 1560,
-// where a leaf is latency and all of the inverses are built at once.  n is the
-// whole call's, so that every panel of a solve takes the same leaves.
+// where a leaf is latency and all of the inverses are built at once.  A leaf takes
+// 52 us for each wave of 4736 columns, so in wide solves the products win again once
+// the inverses are paid for: 512 x 28000 335 / 348, 512 x 40000 485 / 453, 1024 x
+// 14000 488 / 519, 1024 x 20000 769 / 707, 1024 x 80000 2535 / 2057, 2048 x 10000
+// 1099 / 1170, 2048 x 20000 2030 / 1892, 3900 x 14000 4446 / 4288.  n is the whole
+// call's, so that every panel of a solve takes the same leaves.
 bool fused_leaves(int dtype, long m, long n) {
   static const int forced = [] {
     const char *e = getenv("MUBLIS_B200_TRSM");
@@ -79,16 +83,21 @@ bool fused_leaves(int dtype, long m, long n) {
   }();
   if (forced >= 0) return forced == 1;
   if (dtype == B200_F64) return true;
+  if (n >= 12000 && m * n >= 18000000) return false;
   return n <= 512 ? m <= 2048 : m < 4096 || n < 3000;
 }
 
 // Orders that one launch solves (trsm_small.cu); MUBLIS_B200_TRSM=fused /
-// inverse keeps the leaf methods for them too.
-bool small_solve(long m) {
+// inverse keeps the leaf methods for them too.  FP32 above order 128 has one CTA of
+// 32 columns to an SM there, and wide solves take a leaf instead (us, one launch /
+// leaf): 144 x 14000 79 / 81, 144 x 20000 113 / 92, 192 x 2500 60 / 49, 256 x 5000 92
+// / 72, 256 x 40000 325 / 217; 128 x 80000 202 / 211.
+bool small_solve(int dtype, long m, long n) {
   static const bool on = [] {
     const char *e = getenv("MUBLIS_B200_TRSM");
     return !(e && (!strcmp(e, "inverse") || !strcmp(e, "fused")));
   }();
+  if (dtype == B200_F32 && m > B200_TRSM_SMALL_HALF && n >= (m > 160 ? 2500 : 16000)) return false;
   return on && m <= B200_TRSM_SMALL;
 }
 
@@ -451,7 +460,7 @@ extern "C" int b200_trsm_prepare(const b200_trsm_desc_t *d, void **prep) {
   if (d->m <= 0) return B200_OK;
   if (d->uplo != MUBLIS_LOWER && d->uplo != MUBLIS_UPPER)
     return b200_set_error(B200_EINVAL, "trsm: uplo must be lower or upper");
-  if (small_solve(d->m)) return B200_OK;  // nothing to prepare
+  if (small_solve(d->dtype, d->m, d->policy_n > 0 ? d->policy_n : d->n)) return B200_OK;  // nothing to prepare
   TrsmPrep *p = new TrsmPrep{nullptr, 0, nullptr};
   const int st = d->dtype == B200_F32 ? build_inverse<float>(d, p) : build_inverse<double>(d, p);
   if (st != B200_OK) {
@@ -474,7 +483,7 @@ extern "C" int b200_trsm_run(const b200_trsm_desc_t *d) {
   if (d->m <= 0 || d->n <= 0) return B200_OK;
   if (d->uplo != MUBLIS_LOWER && d->uplo != MUBLIS_UPPER)
     return b200_set_error(B200_EINVAL, "trsm: uplo must be lower or upper");
-  if (small_solve(d->m)) {
+  if (small_solve(d->dtype, d->m, d->policy_n > 0 ? d->policy_n : d->n)) {
     b200_small_trsm_t e = {};
     e.a = d->a;
     e.b = d->b;

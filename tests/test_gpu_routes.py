@@ -58,3 +58,15 @@ def test_gemm(lib, p, m, n, k, kernel):
     a, b, c = zeros(p, m, k), zeros(p, k, n), zeros(p, m, n)
     assert kernel in kernels(lib, f"mublis_{p}gemm", 0, 0, m, n, k, 1.0, ptr(a), 1, m, ptr(b), 1, k, 0.0,
                              ptr(c), 1, m)
+
+
+@pytest.mark.parametrize("p,m,n,kernel", [
+    ("s", 256, 40000, "trsm_leaf_s"), ("s", 256, 80000, "trsm_inv_s"), ("s", 192, 5000, "trsm_leaf_s"),
+    ("s", 144, 5000, "small_strsm"), ("s", 128, 40000, "small_strsm"), ("s", 256, 100, "small_strsm"),
+    ("s", 1024, 5000, "trsm_leaf_s"), ("s", 1024, 40000, "trsm_inv_s"), ("s", 512, 28000, "trsm_leaf_s"),
+    ("d", 256, 40000, "small_dtrsm"), ("d", 512, 40000, "trsm_leaf_d")])
+def test_trsm(lib, p, m, n, kernel):
+    import torch
+    a, b = zeros(p, m, m), zeros(p, m, n)
+    a += torch.eye(m, dtype=a.dtype, device="cuda")
+    assert kernel in kernels(lib, f"mublis_{p}trsm", 0, mb.M_LOWER, 0, 0, m, n, 1.0, ptr(a), 1, m, ptr(b), 1, m)
