@@ -7,6 +7,7 @@
 #include <mutex>
 
 #include "b200_internal.h"
+#include "once.h"
 
 #define B200_CUDA_TRY(expr)                                                   \
   do {                                                                        \
@@ -40,13 +41,14 @@ struct B200ProfScope {
   ~B200ProfScope();
 };
 
-// Runs `setup` once per process: callers that arrive while it runs wait for
-// it, and every caller gets its status (with a last-error message of its own
-// when it failed: `what`).  For one-time kernel attribute set-up that several
+// Runs `setup` once on the current device (with a last-error message of the
+// caller's own when it failed: `what`).  For kernel attribute set-up that several
 // host threads may reach first at the same time.
 template <class F>
-int b200_once(std::once_flag &flag, int &status, const char *what, F setup) {
-  std::call_once(flag, [&] { status = setup(); });
+int b200_once(B200Once &once, const char *what, F setup) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) device = 0;
+  const int status = once.run(device, setup);
   return status == B200_OK ? B200_OK : b200_set_error(status, what);
 }
 

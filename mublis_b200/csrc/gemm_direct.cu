@@ -534,9 +534,8 @@ template <typename T, int TILE, bool PLAIN, bool FOLD>
 int launch_tile(DirectArgs<T> &p, cudaStream_t s) {
   using C = DirectCfg<T, TILE>;
   auto kern = direct_gemm_kernel<T, TILE, PLAIN, FOLD>;
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "direct gemm: set-up failed", [&]() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "direct gemm: set-up failed", [&]() -> int {
     B200_CUDA_TRY(
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
     return B200_OK;
@@ -622,9 +621,8 @@ template <typename T, int TILE>
 int launch_group_tile(const b200_group_gemm_t *table, const int *tile_prob, int tiles, cudaStream_t s) {
   using C = DirectCfg<T, TILE>;
   auto kern = direct_group_kernel<T, TILE>;
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "grouped gemm: set-up failed", [&]() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "grouped gemm: set-up failed", [&]() -> int {
     cudaFuncAttributes fa;
     B200_CUDA_TRY(
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));

@@ -397,9 +397,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 template <int LA, int LB, bool SPLIT>
 int launch_kernel(const DmmaGemmArgs &a, int grid, cudaStream_t s) {
   auto kern = dmma_gemm_kernel<LA, LB, SPLIT>;
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "dmma kernel: set-up failed", [&]() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "dmma kernel: set-up failed", [&]() -> int {
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     // An increase that the launch's registers cannot grant would wait forever.
     cudaFuncAttributes fa;

@@ -371,9 +371,8 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
 }  // namespace
 
 int launch_ffma_gemm(FfmaGemmArgs &a, const FfmaPolicy *pol, cudaStream_t s) {
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "sgemm: set-up failed", []() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "sgemm: set-up failed", []() -> int {
     B200_CUDA_TRY(cudaFuncSetAttribute(ffma_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        SMEM));
     return B200_OK;

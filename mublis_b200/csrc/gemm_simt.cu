@@ -26,6 +26,7 @@
 // chunk of a tile to finish adds them in chunk order and runs the epilogue,
 // so the result does not depend on which CTA ran what.
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
@@ -436,9 +437,9 @@ int launch_cfg(const SimtGemmArgs<T> &a0, cudaStream_t s, const SimtPolicy *pol)
   auto kern = simt_tile_kernel<T, BM, BN, BK, WM, WN, ST, MINB>;
   auto kern_split = simt_gemm_kernel<T, BM, BN, BK, WM, WN, ST, MINB, true>;
   const size_t smem = (size_t)ST * BK * (BM + BN) * sizeof(T);
-  static std::once_flag once;
-  static int conf = B200_OK, per_sm = 0;
-  B200_TRY(b200_once(once, conf, "gemm: set-up failed", [&]() -> int {
+  static B200Once once;
+  static std::atomic<int> per_sm{0};  // of every device: all are alike
+  B200_TRY(b200_once(once, "gemm: set-up failed", [&]() -> int {
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     B200_CUDA_TRY(
         cudaFuncSetAttribute(kern_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

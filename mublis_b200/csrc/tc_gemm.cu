@@ -27,6 +27,8 @@
 // The tile walk, domain pruning and k-range clipping are the same as the
 // plain kernel's (gemm_simt.cu), i.e. the reference driver's
 // (frame/l3/l3_driver.c:130-171); a tile without update writes beta * C.
+#include <algorithm>
+#include <atomic>
 #include <cudaTypedefs.h>
 
 #include <cstring>
@@ -722,8 +724,8 @@ int launch_bf16_pair(const CUtensorMap &ta, const CUtensorMap &tb, const Bf16Par
                      cudaStream_t s) {
   using C = Bf16PairCfg<TERMS, STAGES>;
   auto kern = tc_bf16_pair_kernel<TERMS, STAGES, F16>;
-  static std::once_flag once;
-  static int conf = B200_OK, max_clusters = 0;
+  static B200Once once;
+  static std::atomic<int> max_clusters{0};  // of every device: all are alike
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -735,7 +737,7 @@ int launch_bf16_pair(const CUtensorMap &ta, const CUtensorMap &tb, const Bf16Par
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  B200_TRY(b200_once(once, conf, "bf16 pair kernel: set-up failed", [&]() -> int {
+  B200_TRY(b200_once(once, "bf16 pair kernel: set-up failed", [&]() -> int {
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     cudaFuncAttributes fa;
     B200_CUDA_TRY(cudaFuncGetAttributes(&fa, kern));
@@ -743,15 +745,16 @@ int launch_bf16_pair(const CUtensorMap &ta, const CUtensorMap &tb, const Bf16Par
       return b200_set_error(B200_EINVAL, "bf16 pair kernel: register split does not fit its launch");
     cudaLaunchConfig_t q = cfg;
     q.gridDim = dim3(2 * b200_sm_count());
-    if (cudaOccupancyMaxActiveClusters(&max_clusters, (void *)kern, &q) != cudaSuccess ||
-        max_clusters < 1) {
+    int resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, (void *)kern, &q) != cudaSuccess || resident < 1) {
       cudaGetLastError();
       return b200_set_error(B200_ECUDA, "bf16 pair kernel: no CTA pair can be resident");
     }
+    max_clusters = resident;
     return B200_OK;
   }));
   const int tiles = p.w.tiles_m * p.w.tiles_n;
-  const int pairs = tiles < max_clusters ? tiles : max_clusters;
+  const int pairs = std::min<int>(tiles, max_clusters);
   cfg.gridDim = dim3(2 * pairs);
   B200ProfScope prof(F16 ? "tc_fp16x3" : (TERMS == 2 ? "tc_bf16x3" : "tc_bf16x6"), s);
   B200_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, p));
@@ -763,9 +766,8 @@ int launch_bf16(const CUtensorMap &ta, const CUtensorMap &tb, const Bf16Params &
                 cudaStream_t s) {
   using C = Bf16Cfg<TERMS, STAGES>;
   auto kern = tc_bf16_kernel<TERMS, STAGES, F16>;
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "bf16 kernel: set-up failed", [&]() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "bf16 kernel: set-up failed", [&]() -> int {
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
     // The warpgroup register split assumes this launch allocation; with
     // fewer registers per thread the epilogue's increase could never be
@@ -1720,9 +1722,9 @@ cudaLaunchConfig_t oz2_pair_config(cudaLaunchAttribute *attr, int grid, cudaStre
 // returns how many CTA pairs can be resident at once.
 template <typename T>
 int oz2_pair_clusters(int *clusters) {
-  static std::once_flag once;
-  static int conf = B200_OK, cached = 0;
-  B200_TRY(b200_once(once, conf, "ozaki2 pair kernel: set-up failed", []() -> int {
+  static B200Once once;
+  static std::atomic<int> cached{0};  // of every device: all are alike
+  B200_TRY(b200_once(once, "ozaki2 pair kernel: set-up failed", []() -> int {
     auto kern = tc_ozaki2_pair_kernel<T>;
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        OzPairCfg::SMEM));
@@ -1732,10 +1734,12 @@ int oz2_pair_clusters(int *clusters) {
       return b200_set_error(B200_EINVAL, "ozaki2 pair kernel: register split does not fit its launch");
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = oz2_pair_config<T>(attr, 2 * b200_sm_count(), nullptr);
-    if (cudaOccupancyMaxActiveClusters(&cached, (void *)kern, &cfg) != cudaSuccess || cached < 1) {
+    int resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, (void *)kern, &cfg) != cudaSuccess || resident < 1) {
       cudaGetLastError();
       return b200_set_error(B200_ECUDA, "ozaki2 pair kernel: no CTA pair can be resident");
     }
+    cached = resident;
     return B200_OK;
   }));
   *clusters = cached;
@@ -1864,10 +1868,9 @@ int run_ozaki(const b200_l3_desc_t *d, bool mod) {
     if constexpr (F64) {
       if (!mod) kern = tc_ozaki_kernel<false, double>;
     }
-    static std::once_flag once[2];
-    static int conf[2] = {B200_OK, B200_OK};
+    static B200Once once[2];
     if (st == B200_OK)
-      st = b200_once(once[mod], conf[mod], "ozaki kernel: set-up failed", [&]() -> int {
+      st = b200_once(once[mod], "ozaki kernel: set-up failed", [&]() -> int {
         B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            C::SMEM));
         // The warpgroup register split must fit the compiled allocation (an

@@ -702,9 +702,8 @@ int b200_tcg_create(const mublis_b200_gemm_problem_t *p, int count, b200_tcg **o
 // Everything the launches need beforehand (kernel attributes and code, the error
 // word's host memory): what a stream capture would not survive.
 int b200_tcg_setup() {
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "grouped fp16x3 kernels: set-up failed", []() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "grouped fp16x3 kernels: set-up failed", []() -> int {
     B200_CUDA_TRY(cudaFuncSetAttribute(tcg_pack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(sizeof(float) * TCG_PACK_NBUF * 32 * (TCG_PACK_KS + 1))));
     B200_CUDA_TRY(cudaFuncSetAttribute(tcg_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -574,9 +574,8 @@ extern "C" int b200_trsm_leaf_pack(int dtype, const void *a, long rs_a, long cs_
 template <typename T, int NCG, int W>
 int leaf_launch(const LeafArgs<T> &la, cudaStream_t s) {
   using L = Leaf<T, NCG, W>;
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "trsm leaf kernel: set-up failed", []() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "trsm leaf kernel: set-up failed", []() -> int {
     // The register split adds up only for this allocation (an increase that cannot
     // be granted would wait for good).
     cudaFuncAttributes fa;

@@ -405,9 +405,8 @@ int launch(const b200_small_trsm_t *table, const int *slab_prob, const b200_smal
            int first_slab, int slabs, int max_order, cudaStream_t s) {
   using L = Layout<T>;
   auto kern = small_trsm_kernel<T, WARPS>;
-  static std::once_flag once;
-  static int conf = B200_OK;
-  B200_TRY(b200_once(once, conf, "small trsm: set-up failed", [&]() -> int {
+  static B200Once once;
+  B200_TRY(b200_once(once, "small trsm: set-up failed", [&]() -> int {
     cudaFuncAttributes fa;
     B200_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)sizeof(T) * L::elements(WARPS)));
