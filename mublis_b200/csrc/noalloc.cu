@@ -76,9 +76,10 @@ int scratch_on_current_device(float **out) {
 }  // namespace
 
 // Called once by the library's initialisation with the device it brings up
-// current: resolves (and so claims) the scratch array there, and loads the
-// kernels the entry point launches, which the other entry points need not
-// have run before its first call.  A failure is kept and reported by the
+// current: resolves (and so claims) the scratch array there, loads the
+// kernels the entry point launches and takes the pinned word in which they
+// report a wait that ran out; the other entry points need not have run before
+// its first call.  A failure is kept and reported by the
 // entry point's first call; it does not fail the initialisation of
 // everything else.
 extern "C" void b200_noalloc_setup(void) {
@@ -87,6 +88,7 @@ extern "C" void b200_noalloc_setup(void) {
   (void)b200_ffma_preload();
   (void)b200_scale_preload();
   (void)b200_pack_preload();
+  (void)b200_device_error_word();
 }
 
 extern "C" int mublis_b200_sgemm_noalloc(mublis_trans_t trans_a, mublis_trans_t trans_b, int m,
