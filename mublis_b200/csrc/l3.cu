@@ -158,6 +158,13 @@ bool overlaps_operand(const b200_l3_desc_t *d) {
   return false;
 }
 
+// Whether a tensor map could be made; if not, the operand is packed, which is no
+// error of the call's.
+bool mapped(int status) {
+  if (status != B200_OK) b200_set_error(B200_OK, "");
+  return status == B200_OK;
+}
+
 // One operand of the FP64 tensor-pipe kernel: read in place (2-D TMA tiles)
 // when no element needs changing on the way -- a general, unmasked operand,
 // every pair with the same orientation, a SYR2K's pairs meeting on a k-block
@@ -185,10 +192,9 @@ int dmma_operand(const b200_l3_desc_t *d, bool b_side, CUtensorMap (&map)[2], in
     if (t == 0) *layout = lay;
     // k innermost: 16 k x 128 rows; m / n innermost: boxes of 16 x 16 k.
     direct = lay == *layout &&
-             (lay == B200_DMMA_K
-                  ? b200_make_tmap_f64(&map[t], x[t], d->k, len, b_side ? cs[t] : rs[t], BK, T, 1)
-                  : b200_make_tmap_f64(&map[t], x[t], len, d->k, b_side ? rs[t] : cs[t], 16, BK, 1)) ==
-                 B200_OK;
+             mapped(lay == B200_DMMA_K
+                        ? b200_make_tmap_f64(&map[t], x[t], d->k, len, b_side ? cs[t] : rs[t], BK, T, 1)
+                        : b200_make_tmap_f64(&map[t], x[t], len, d->k, b_side ? rs[t] : cs[t], 16, BK, 1));
   }
   if (direct) {
     if (d->npairs == 2) *kpair = d->k;
@@ -312,7 +318,7 @@ int ffma_operand(const b200_l3_desc_t *d, bool b_side, long len, CUtensorMap (&m
     direct = s_mn == 1 && s_k >= len && s_k % 4 == 0 && ((uintptr_t)x[t] & 15) == 0 &&
              !b200_views_overlap(d->c, d->rs_c, d->cs_c, d->m, d->n, x[t], rs[t], cs[t],
                                  b_side ? d->k : d->m, b_side ? d->n : d->k, 4) &&
-             b200_make_tmap_f32(&map[t], x[t], len, d->k, s_k, T, BK) == B200_OK;
+             mapped(b200_make_tmap_f32(&map[t], x[t], len, d->k, s_k, T, BK));
   }
   if (direct) {
     if (d->npairs == 2) *kpair = d->k;
