@@ -791,25 +791,41 @@ int launch_bf16(const CUtensorMap &ta, const CUtensorMap &tb, const Bf16Params &
 
 namespace {
 
-// Scales and packs one operand of a scaled form: the exponents of its rows
-// (columns) over the whole, concatenated k, then its planes.  amax: mn_pad
-// words of scratch.
+// One operand of a scaled form.
+struct ScaledOperand {
+  const PackView *v;  // one per pair
+  bool b_side;
+  long len, pad;  // rows of op(A) / columns of op(B), and padded
+  PackOut out;
+};
+
+// Scales and packs both operands: the exponents of A's rows and B's columns over the
+// whole, concatenated k, then the planes.  amax, exps: a.pad + b.pad words, A's first.
+// Operands without the one-pass kernel share their clearing and exponent launches.
 template <typename T>
-int scale_and_pack(const PackView (&v)[2], int npairs, bool b_side, long mn_len, long k_len,
-                   long mn_pad, long kpad, unsigned long long *amax, int *exps, const PackOut &o,
-                   cudaStream_t s) {
-  if (npairs == 1 && launch_scale_pack<T>(v[0], b_side, mn_len, k_len, mn_pad, kpad, exps, o, s)) {
-    B200_LAUNCH_CHECK();
-    return B200_OK;
+int scale_and_pack(const ScaledOperand &a, const ScaledOperand &b, int npairs, long k, long kpad,
+                   unsigned long long *amax, int *exps, cudaStream_t s) {
+  bool done[2] = {false, false};
+  const ScaledOperand *const x[2] = {&a, &b};
+  int *const e[2] = {exps, exps + a.pad};
+  unsigned long long *const am[2] = {amax, amax + a.pad};
+  for (int i = 0; i < 2 && npairs == 1; ++i) {
+    done[i] = launch_scale_pack<T>(x[i]->v[0], x[i]->b_side, x[i]->len, k, x[i]->pad, kpad, e[i], x[i]->out, s);
+    if (done[i]) B200_LAUNCH_CHECK();
   }
-  B200_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * mn_pad, s));
-  for (int t = 0; t < npairs; ++t)
-    B200_TRY(launch_absmax<T>(v[t], b_side, mn_len, k_len, amax, s));
-  B200_TRY(launch_scale_exps(amax, exps, mn_pad, s));
-  for (int t = 0; t < npairs; ++t) {
-    const long kk0 = (long)t * k_len, kk1 = t + 1 == npairs ? kpad : kk0 + k_len;
-    B200_TRY(launch_pack<T>(v[t], b_side, mn_len, k_len, mn_pad, kk0, kk1, o, s));
-  }
+  if (done[0] && done[1]) return B200_OK;
+  const int first = done[0] ? 1 : 0;
+  const long words = (done[0] ? 0 : a.pad) + (done[1] ? 0 : b.pad);
+  B200_CUDA_TRY(cudaMemsetAsync(am[first], 0, sizeof(unsigned long long) * words, s));
+  for (int i = 0; i < 2; ++i)
+    for (int t = 0; t < npairs && !done[i]; ++t)
+      B200_TRY(launch_absmax<T>(x[i]->v[t], x[i]->b_side, x[i]->len, k, am[i], s));
+  B200_TRY(launch_scale_exps(am[first], e[first], words, s));
+  for (int i = 0; i < 2; ++i)
+    for (int t = 0; t < npairs && !done[i]; ++t) {
+      const long kk0 = (long)t * k, kk1 = t + 1 == npairs ? kpad : kk0 + k;
+      B200_TRY(launch_pack<T>(x[i]->v[t], x[i]->b_side, x[i]->len, k, x[i]->pad, kk0, kk1, x[i]->out, s));
+    }
   return B200_OK;
 }
 
@@ -862,11 +878,9 @@ int tc_run_bf16(const b200_l3_desc_t *d, int form) {
   const PackOut ob{bp, kpad, npad * kpad, PACK_K_MAJOR, f16 ? PACK_FP16_SPLIT : PACK_BF16_SPLIT, terms,
                    ae ? ae + mpad : nullptr};
   if (f16) {
-    unsigned long long *am = (unsigned long long *)amax;
     if (st == B200_OK)
-      st = scale_and_pack<float>(va, d->npairs, false, d->m, d->k, mpad, kpad, am, ae, oa, s);
-    if (st == B200_OK)
-      st = scale_and_pack<float>(vb, d->npairs, true, d->n, d->k, npad, kpad, am + mpad, ae + mpad, ob, s);
+      st = scale_and_pack<float>({va, false, d->m, mpad, oa}, {vb, true, d->n, npad, ob}, d->npairs, d->k,
+                                 kpad, (unsigned long long *)amax, ae, s);
   }
   for (int t = 0; t < d->npairs && !f16 && st == B200_OK; ++t) {
     const long kk0 = (long)t * d->k, kk1 = t + 1 == d->npairs ? kpad : kk0 + d->k;
@@ -1821,10 +1835,8 @@ int run_ozaki(const b200_l3_desc_t *d, bool mod) {
     const int xform = mod ? PACK_INT8_MODULI : PACK_INT8_SLICES;
     const PackOut oa{ap, kpad, mpad * kpad, PACK_K_MAJOR, xform, slices, exps, pa, moduli};
     const PackOut ob{bp, kpad, npad * kpad, PACK_K_MAJOR, xform, slices, exps + mpad, pb, moduli};
-    unsigned long long *am = (unsigned long long *)amax;
-    st = scale_and_pack<T>(va, d->npairs, false, d->m, d->k, mpad, kpad, am, exps, oa, s);
-    if (st == B200_OK)
-      st = scale_and_pack<T>(vb, d->npairs, true, d->n, d->k, npad, kpad, am + mpad, exps + mpad, ob, s);
+    st = scale_and_pack<T>({va, false, d->m, mpad, oa}, {vb, true, d->n, npad, ob}, d->npairs, d->k, kpad,
+                           (unsigned long long *)amax, exps, s);
   }
   CUtensorMap ta, tb;
   // Boxes of one CTA's share of a tile: 256 rows, or 128 on CTA pairs.
