@@ -73,12 +73,9 @@ def family_flops(n: int) -> float:
 
 def kernel_flops(n: int) -> dict:
     """Algorithmic flops of one step attributed to the kernel that executes
-    them.  Every routine, TRSM included, runs on the packed GEMM kernel: the
-    recursive TRSM's updates do m^2 n (1 - b/m) and its leaf products (the
-    inverted b x b diagonal blocks times B) cover the remaining m b n of the
-    triangle (they execute 2 m b n, twice the triangle's work, which is not
-    credited)."""
-    gemm_part = sum(flops(r, n) for r in ROUTINES)
+    them: every routine but TRSM, whose leaves and whose smaller updates run in
+    other kernels (a larger update that this kernel runs is not credited)."""
+    gemm_part = sum(flops(r, n) for r in ROUTINES if r != "trsm")
     return {"ffma_sgemm": gemm_part, "simt_dgemm": gemm_part, "dmma_dgemm": gemm_part}
 
 

@@ -20,8 +20,8 @@
 // warps that never meet at a block barrier keep the pipe as busy as the
 // sixteen of two cp.async CTAs did, so a call with about one tile per SM runs
 // at full rate.  Whole calls, before (two cp.async CTAs of 256 threads per SM
-// over packed panels) -> now, in us: SGEMM 4096^3 NT 2325 -> 2193 (62.7 TF/s),
-// 2048^3 377 -> 337, 1500^3 202 -> 151, SSYRK n = k = 2048 (136 tiles) 254 -> 182.
+// over packed panels) -> now, in us: SGEMM 4096^3 NT 2325 -> 2155 (63.8 TF/s),
+// 2048^3 375 -> 333, 1500^3 NN 200 -> 151, SSYRK n = k = 2048 (136 tiles) 251 -> 175.
 //
 // Domain handling (ji skips and masks, jp / pi clip the k range, an empty k
 // range writes beta * C, beta == 0 never reads C) and split-K are the FP64

@@ -173,10 +173,11 @@ __device__ __forceinline__ double b200_pow2_scale(double x, int e) {
                                  : ldexp(x, e);
 }
 
-// x * 2^sh for sh within [-300, 300], as two multiplications by exact powers
+// x * 2^sh for sh within [-252, 254], as two multiplications by exact powers
 // of two: the first is the whole factor whenever 2^sh is a normal float (then
 // it is one rounding of the exact product, as ldexpf gives); for larger |sh|
-// the factor is cut in two.
+// the factor is cut in two.  (The fp16 splits' sh = 15 - e lies in [-113, 163]:
+// e is frexp's exponent of an FP32 value, -148 .. 128.)
 __device__ __forceinline__ void b200_pow2_factors(int sh, float &f1, float &f2) {
   const int s1 = sh > 127 ? 127 : (sh < -126 ? -126 : sh);
   f1 = __int_as_float((s1 + 127) << 23);
