@@ -1,6 +1,6 @@
 // trsm_small.cu -- left triangular solves of order up to 256 in one launch each,
-// or one launch for many (grouped.cu): alpha, the diagonal blocks' inverses, the
-// solve and the updates between the blocks all in one kernel.
+// or one launch for many (grouped.cu): alpha, the solve and the updates between the
+// blocks all in one kernel.
 //
 // Reference: the blocked solve of frame/l3/trsm.c:139-183 with gemmtrsm
 // micro-kernels (include/mublis_instantiate.h:95-114) over a packed A whose
@@ -9,25 +9,25 @@
 // up to order 128, 16 up to 256.  (Two blocks a warp duplicated the update and
 // solve code; a kernel whose code runs once or a few times pays for its size in
 // instruction fetches.)
-//   * Start: the 16 x 16 diagonal blocks come in by asynchronous copies and each
-//     warp inverts its own by substitution against the reciprocal diagonal.
+//   * Start: the 16 x 16 diagonal blocks come in by asynchronous copies; their
+//     diagonal becomes its reciprocal, as in the reference's packing.
 //   * Step d: X_d (solved, in shared memory) updates the blocks below,
-//     B_r -= A_rd X_d, and the warp of block d + 1 then solves it, X = inv(D) R.
+//     B_r -= A_rd X_d, and the warp of block d + 1 then solves it by substitution.
 //     One block barrier per step.
 //   * Column d of A's blocks arrives two steps ahead in a 3-deep ring of
 //     asynchronous element copies, zeros past the matrix, nothing of the
 //     unstored triangle or of a unit diagonal read.
-// FP64 updates and solves are m16n8k4 .f64 MMAs (16 x 20 blocks: a fragment
-// load's half-warp falls on 16 different 8-byte banks); FP32 ones are packed
-// FMAs with a lane per column and the blocks of A broadcast.
+// FP64 updates are m16n8k4 .f64 MMAs (16 x 20 blocks: a fragment load's half-warp
+// falls on 16 different 8-byte banks); FP32 ones and both solves are FMAs with a
+// lane per column and the blocks of A broadcast.
 // An upper triangle is the lower one with rows and columns reversed.
 //
 // What bounds it: the latency of the order / 16 dependent steps; CTAs of other
 // slabs and problems fill an SM meanwhile.  Measured (us, before -> now): groups
-// of 1024 of order 32-256, FP64 1222 -> 173 and FP32 883 -> 163 (one warp
+// of 1024 of order 32-256, FP64 1188 -> 165 and FP32 853 -> 139 (one warp
 // substituted 32 rows at a time); a call of order 256 with 4000 right-hand sides,
-// FP32 178 -> 69 (inverted blocks, a dozen launches), FP64 87 -> 67 (the leaf
-// kernel after a scale and a pack).
+// FP64 84 -> 60 (the leaf kernel after a scale and a pack); of order 128 with 1000,
+// FP32 117 -> 46 (inverted blocks, a dozen launches).
 #include <algorithm>
 #include <type_traits>
 
@@ -44,11 +44,11 @@ struct Layout {
   static constexpr int BLK = LB * PITCH;
   static constexpr int XLD = F64 ? 36 : 33;    // of a solved 16 x 32 block
   // Element (r, c) of a block below the diagonal (FP64: row-major, FP32:
-  // column-major) and of a diagonal block or its inverse (row-major).
+  // column-major) and of a diagonal block (column-major).
   __host__ __device__ static constexpr int panel(int r, int c) {
     return F64 ? r * PITCH + c : c * PITCH + r;
   }
-  __host__ __device__ static constexpr int diag(int r, int c) { return r * PITCH + c; }
+  __host__ __device__ static constexpr int diag(int r, int c) { return c * PITCH + r; }
   // Elements of shared memory for problems of up to nb blocks.
   __host__ __device__ static constexpr int elements(int nb) {
     return nb * BLK + RING * (nb > 1 ? nb - 1 : 1) * BLK + 2 * LB * XLD;
@@ -149,120 +149,57 @@ __device__ __forceinline__ void update(Block<float> &b, const float *a, const fl
   }
 }
 
-// A diagonal block in memory: element (i, q), q < i, at a[i rs + q cs]; rows from
-// `rows` on are the identity's.
-template <typename T>
-struct DiagBlock {
-  const T *a;
-  long rs, cs;
-  int rows, unit;
-};
-
-// Forward substitution of one column (x, pitch XLD) from row `first` on.
-template <typename T>
-__device__ __forceinline__ void substitute(T *x, int first, const DiagBlock<T> &d) {
-  constexpr int LD = Layout<T>::XLD;
-#pragma unroll 1
-  for (int i = first; i < min(LB, d.rows); ++i) {
-    T s = x[i * LD];
-#pragma unroll 1
-    for (int q = 0; q < i; ++q) s = fma(-d.a[i * d.rs + q * d.cs], x[q * LD], s);
-    x[i * LD] = d.unit ? s : s * (T(1) / d.a[i * (d.rs + d.cs)]);
-  }
-}
-
-__device__ __forceinline__ void multiply(double (&c)[4][4], const double *inv, const double (&f)[4][4]) {
-  const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) c[j][e] = 0.0;
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    const double a0 = inv[Layout<double>::diag(g, 4 * ks + t)];
-    const double a1 = inv[Layout<double>::diag(g + 8, 4 * ks + t)];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) dmma(c[j], a0, a1, f[ks][j]);
-  }
-}
-
-// x = inv r for the inverse of a diagonal block (zero above its diagonal), into
-// shared memory.  A non-finite element of r is to reach only its own row and those
-// below, as in a substitution.  The MMAs multiply the inverse's zeros by it too and
-// spoil its whole column, which shows in any one row of the product: the high words
-// of one row's elements, as floats, add up to a NaN (a sum may be one for finite
-// elements beyond 2^1016 as well).  Then the rows before a column's first such
-// element are multiplied without it and the others substituted.  The test of a row
-// after the stores costs 0-1% of a call and 3% of a group; of all of r before them
-// it cost 3-5%.
-__device__ __forceinline__ void solve(Block<double> &b, const double *inv, double *x,
-                                      const DiagBlock<double> &d) {
+// Solves a diagonal block D (lower triangle, reciprocal diagonal) for a warp's 32
+// columns, a column to a lane, by substitution: x[i] = r[i] / D[i][i], then r[j] -=
+// D[j][i] x[i] below.  D's columns are read as 16-byte broadcasts.  A product with
+// the block's inverse instead (on the FP64 MMAs, or as many FMAs) took as long but
+// was not backward stable -- diagonals of 0.05-1: residuals of 900 u |A||X| at order
+// 16, 2 u so -- and its zeros spread a non-finite r to rows above it.
+__device__ __forceinline__ void solve(Block<double> &b, const double *d, double *x) {
   constexpr int LD = Layout<double>::XLD;
   const int lane = threadIdx.x & 31;
   b.each([&](int r, int c, double v) { x[r * LD + c] = v; });
   __syncwarp();
-  double f[4][4];
-  load_x<double>(x, f);
-  __syncwarp();
-  multiply(b.c, inv, f);
-  b.each([&](int r, int c, double v) { x[r * LD + c] = v; });
-  float row = 0.f;
+  double r[LB];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    row += __int_as_float(__double2hiint(b.c[j][0])) + __int_as_float(__double2hiint(b.c[j][1]));
-  if (!__any_sync(0xffffffffu, isnan(row))) return;
-  __syncwarp();
-  int first = LB;  // of column `lane`
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) x[(4 * ks + (lane & 3)) * LD + 8 * j + (lane >> 2)] = f[ks][j];
-  __syncwarp();
-#pragma unroll 1
-  for (int i = LB - 1; i >= 0; --i)
-    if (!isfinite(x[i * LD + lane])) first = i;
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks)
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (!isfinite(f[ks][j])) f[ks][j] = 0.0;
-  multiply(b.c, inv, f);
-  __syncwarp();
-  b.each([&](int r, int c, double v) {
-    if (r < __shfl_sync(0xffffffffu, first, c)) x[r * LD + c] = v;
-  });
-  __syncwarp();
-  substitute(x + lane, first, d);
-}
-__device__ __forceinline__ void solve(Block<float> &b, const float *inv, float *x,
-                                      const DiagBlock<float> &d) {
-  constexpr int LD = Layout<float>::XLD;
-  const int lane = threadIdx.x & 31;
-  float r[LB], s;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) r[2 * i] = b.c[i].x, r[2 * i + 1] = b.c[i].y;
+  for (int i = 0; i < LB; ++i) r[i] = x[i * LD + lane];
 #pragma unroll
   for (int i = 0; i < LB; ++i) {
-    s = 0.f;
+    double col[LB];  // rows from i - i % 2 on
 #pragma unroll
-    for (int q = 0; q <= i / 4; ++q) {
-      const float4 w = *(const float4 *)(inv + Layout<float>::diag(i, 4 * q));
-      s = fmaf(w.x, r[4 * q], s);
-      if (4 * q + 1 <= i) s = fmaf(w.y, r[4 * q + 1], s);
-      if (4 * q + 2 <= i) s = fmaf(w.z, r[4 * q + 2], s);
-      if (4 * q + 3 <= i) s = fmaf(w.w, r[4 * q + 3], s);
+    for (int j = i / 2 * 2; j < LB; j += 2) {
+      const double2 v = *(const double2 *)(d + Layout<double>::diag(j, i));
+      col[j] = v.x, col[j + 1] = v.y;
     }
-    x[i * LD + lane] = s;
+    r[i] *= col[i];
+    x[i * LD + lane] = r[i];
+#pragma unroll
+    for (int j = i + 1; j < LB; ++j) r[j] = fma(-col[j], r[i], r[j]);
   }
-  if (isfinite(s)) return;
-  int first = LB;
+}
+// FP32: r = alpha rhs - sum, formed when its row is reached; the substitution's
+// products go to the sum.
+__device__ __forceinline__ void solve(Block<float> &sum, const Block<float> &rhs, float alpha,
+                                      const float *d, float *x) {
+  constexpr int LD = Layout<float>::XLD;
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int i = LB - 1; i >= 0; --i)
-    if (!isfinite(r[i])) first = i;
+  for (int i = 0; i < LB; ++i) {
+    float col[LB];  // rows from i - i % 4 on
 #pragma unroll
-  for (int i = 0; i < LB; ++i)
-    if (i >= first) x[i * LD + lane] = r[i];
-  substitute(x + lane, first, d);
+    for (int j = i / 4 * 4; j < LB; j += 4) {
+      const float4 v = *(const float4 *)(d + Layout<float>::diag(j, i));
+      col[j] = v.x, col[j + 1] = v.y, col[j + 2] = v.z, col[j + 3] = v.w;
+    }
+    const float r = i % 2 ? fmaf(alpha, rhs.c[i / 2].y, -sum.c[i / 2].y)
+                          : fmaf(alpha, rhs.c[i / 2].x, -sum.c[i / 2].x);
+    const float xi = r * col[i];
+    x[i * LD + lane] = xi;
+    if (i % 2 == 0) sum.c[i / 2].y = fmaf(col[i + 1], xi, sum.c[i / 2].y);
+#pragma unroll
+    for (int j = i / 2 + 1; j < LB / 2; ++j)
+      sum.c[j] = __ffma2_rn(make_float2(col[2 * j], col[2 * j + 1]), make_float2(xi, xi), sum.c[j]);
+  }
 }
 
 // table may be null: then `one` is the only problem.
@@ -276,8 +213,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
   const int slab = first_slab + blockIdx.x;
   const b200_small_trsm_t &e = table ? table[slab_prob[slab]] : one;
   const int m = e.m, nb = (m + LB - 1) / LB;
-  T *inv = (T *)smem_raw;            // [nb] diagonal blocks, then their inverses
-  T *ring = inv + nb * L::BLK;       // [RING][nb - 1] blocks
+  T *dia = (T *)smem_raw;            // [nb] diagonal blocks, reciprocal diagonal
+  T *ring = dia + nb * L::BLK;       // [RING][nb - 1] blocks
   const int seg = (nb > 1 ? nb - 1 : 1) * L::BLK;
   T *xs = ring + RING * seg;         // [2] solved blocks
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -311,7 +248,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
   };
   // The diagonal blocks: lower triangle, the identity past the matrix.
   for (int blk = eb; blk < nb; blk += STRIDE) {
-    T *dst = inv + blk * L::BLK + L::diag(er, ec);
+    T *dst = dia + blk * L::BLK + L::diag(er, ec);
     if (blk * LB + er < m && (ec < er || (ec == er && !e.unit)))
       cp_zfill<sizeof(T)>(dst, ae + (long)blk * LB * (ars + acs), true);
     else
@@ -337,29 +274,9 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 
   cp_wait<2>();  // the diagonal blocks
   __syncthreads();
-  {
-    // Warp w inverts block w, column j by lane j: L x = e_j against the
-    // reciprocal diagonal.
-    const int j = lane & 15;
-    T *d = inv + warp * L::BLK;
-    const bool mine = warp < nb && lane < LB;
-    if (mine) d[L::diag(j, j)] = T(1) / d[L::diag(j, j)];
-    __syncwarp();
-    T x[LB];
-    if (mine) {
-#pragma unroll
-      for (int i = 0; i < LB; ++i) {
-        T r = i == j ? T(1) : T(0);
-#pragma unroll
-        for (int q = 0; q < i; ++q) r = fma(-d[L::diag(i, q)], x[q], r);
-        x[i] = r * d[L::diag(i, i)];
-      }
-    }
-    __syncwarp();
-    if (mine) {
-#pragma unroll
-      for (int i = 0; i < LB; ++i) d[L::diag(i, j)] = x[i];
-    }
+  if (warp < nb && lane < LB) {  // warp w: the reciprocal diagonal of block w
+    T *d = dia + warp * L::BLK + L::diag(lane, lane);
+    *d = T(1) / *d;
   }
   __syncthreads();
 
@@ -378,14 +295,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
   for (int d = 0; d < nb; ++d) {
     T *xd = xs + (d & 1) * LB * L::XLD;
     if (warp == d) {
-      if constexpr (!L::F64) {
-#pragma unroll
-        for (int i = 0; i < LB / 2; ++i)
-          acc.c[i] = __ffma2_rn(make_float2(alpha, alpha), rhs.c[i],
-                                make_float2(-acc.c[i].x, -acc.c[i].y));
-      }
-      solve(acc, inv + d * L::BLK, xd,
-            {a0 + (long)d * LB * (ars + acs), ars, acs, m - d * LB, e.unit});
+      if constexpr (L::F64) solve(acc, dia + d * L::BLK, xd);
+      else solve(acc, rhs, alpha, dia + d * L::BLK, xd);
     }
     cp_wait<1>();     // segment d
     __syncthreads();  // X_d and segment d are there; every warp is done with step d - 1
