@@ -89,15 +89,16 @@ bool fused_leaves(int dtype, long m, long n) {
 
 // Orders that one launch solves (trsm_small.cu); MUBLIS_B200_TRSM=fused /
 // inverse keeps the leaf methods for them too.  FP32 above order 128 has one CTA of
-// 32 columns to an SM there, and wide solves take a leaf instead (us, one launch /
-// leaf): 144 x 14000 79 / 81, 144 x 20000 113 / 92, 192 x 2500 60 / 49, 256 x 5000 92
-// / 72, 256 x 40000 325 / 217; 128 x 80000 202 / 211.
+// 32 columns to an SM there, and solves wider than one such wave take a leaf instead
+// (us, one launch / leaf): 136 x 4700 50 / 56, 5000 63 / 57, 14000 67 / 70; 192 x 4700
+// 49 / 50, 10000 86 / 78, 40000 206 / 171; 256 x 4700 58 / 53, 5000 87 / 72, 40000 301
+// / 217; order 128 x 80000 202 / 211.
 bool small_solve(int dtype, long m, long n) {
   static const bool on = [] {
     const char *e = getenv("MUBLIS_B200_TRSM");
     return !(e && (!strcmp(e, "inverse") || !strcmp(e, "fused")));
   }();
-  if (dtype == B200_F32 && m > B200_TRSM_SMALL_HALF && n >= (m > 160 ? 2500 : 16000)) return false;
+  if (dtype == B200_F32 && m > B200_TRSM_SMALL_HALF && n > 32L * b200_sm_count()) return false;
   return on && m <= B200_TRSM_SMALL;
 }
 
