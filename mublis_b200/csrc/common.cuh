@@ -60,3 +60,12 @@ static inline long b200_ceil_div(long x, long m) { return (x + m - 1) / m; }
 __host__ __device__ static inline bool b200_rel(int rel, long lhs, long rhs) {
   return rel == MUBLIS_L3_LOWER ? lhs <= rhs : (rel == MUBLIS_L3_UPPER ? lhs >= rhs : true);
 }
+
+// Whether every element of tile (tm, tn) of an m x n C lies in C and is written
+// under the relation ji of j against i.  Differences, no ends: a tile's end may
+// lie past the largest int.
+__host__ __device__ static inline bool b200_whole_tile(int m, int n, int tm, int tn, int tile, int ji) {
+  const int m0 = tm * tile, n0 = tn * tile;
+  return m - m0 >= tile && n - n0 >= tile &&
+         (ji == MUBLIS_L3_ALL || (ji == MUBLIS_L3_LOWER ? m0 - n0 >= tile : n0 - m0 >= tile));
+}

@@ -340,11 +340,12 @@ __global__ void __launch_bounds__(THREADS, 1)
     // Epilogue: accumulator e of block (i, j) is MMA row g, half e >> 1, of row
     // block i and MMA column 2 t + (e & 1) of column block j / 2, half j & 1.
     const double alpha = p.alpha, beta = p.beta;
-    const bool inside = (tm + 1) * BM <= p.m && (tn + 1) * BN <= p.n &&
-                        (p.ji == MUBLIS_L3_ALL ||
-                         (p.ji == MUBLIS_L3_LOWER ? (tn + 1) * BN <= tm * BM : (tm + 1) * BM <= tn * BN));
+    const bool inside = b200_whole_tile(p.m, p.n, tm, tn, BM, p.ji);
     // This lane's first element; every other is a fixed offset from it.
-    const int i0 = tm * BM + wm * 64 + first_of<LA>(g), j0 = tn * BN + wn * 32 + first_of<LB>(2 * t);
+    // (Unsigned, and offsets compared with what is left of C: a tile's end may lie
+    // past the largest int.)
+    const unsigned i0 = tm * BM + wm * 64 + first_of<LA>(g), j0 = tn * BN + wn * 32 + first_of<LB>(2 * t);
+    const int rows = p.m - i0, cols = p.n - j0, diag = j0 - i0;
     double *c0 = p.c + i0 * p.rs_c + j0 * p.cs_c;
     if (LA != K_CONTIG && inside && ((uintptr_t)p.c & 15) == 0 && p.rs_c == 1 && p.cs_c % 2 == 0) {
       // Rows 2 g and 2 g + 1 as 16 bytes; four loads go out before their stores.
@@ -373,19 +374,19 @@ __global__ void __launch_bounds__(THREADS, 1)
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int gj = j0 + offset_of<LB>(j >> 1, j & 1, e);
-        if (gj >= p.n) continue;
-        double *col = c0 + offset_of<LB>(j >> 1, j & 1, e) * p.cs_c;
+        const int oj = offset_of<LB>(j >> 1, j & 1, e);
+        if (oj >= cols) continue;
+        double *col = c0 + oj * p.cs_c;
         double cv[8];
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
           const int o = offset_of<LA>(x >> 1, x & 1, 0);
-          cv[x] = beta != 0.0 && i0 + o < p.m && b200_rel(p.ji, gj, i0 + o) ? col[o * p.rs_c] : 0.0;
+          cv[x] = beta != 0.0 && o < rows && b200_rel(p.ji, diag + oj, o) ? col[o * p.rs_c] : 0.0;
         }
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
           const int o = offset_of<LA>(x >> 1, x & 1, 0);
-          if (i0 + o >= p.m || !b200_rel(p.ji, gj, i0 + o)) continue;
+          if (o >= rows || !b200_rel(p.ji, diag + oj, o)) continue;
           double v = alpha * acc[x >> 1][j][2 * (x & 1) + e];
           if (beta != 0.0) v = fma(beta, cv[x], v);
           col[o * p.rs_c] = v;

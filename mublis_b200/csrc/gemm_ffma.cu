@@ -275,9 +275,7 @@ __global__ void __launch_bounds__(THREADS, 1) ffma_gemm_kernel(const __grid_cons
     // move 16 bytes at a time along C's unit stride.
     const long m0 = (long)tm * BM + wm * WTM + ty * 4, n0 = (long)tn * BN + wn * WTN + tx * 4;
     const float alpha = p.alpha, beta = p.beta;
-    const bool inside = (tm + 1) * BM <= p.m && (tn + 1) * BN <= p.n &&
-                        (p.ji == MUBLIS_L3_ALL ||
-                         (p.ji == MUBLIS_L3_LOWER ? (tn + 1) * BN <= tm * BM : (tm + 1) * BM <= tn * BN));
+    const bool inside = b200_whole_tile(p.m, p.n, tm, tn, BM, p.ji);
     auto sum = [&](int i, int j) { return (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x; };
     if (vec && inside) {
       // Lines of four along m (rows 4 q + e of column j) or along n.
